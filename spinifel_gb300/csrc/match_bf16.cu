@@ -462,10 +462,35 @@ __global__ void __launch_bounds__(RR_THREADS)
   float V = 0.0f;
   int inexact = 0;
   const float *x = img + im * n_pix;
-  for (int64_t p = tid; p < n_pix; p += RR_THREADS) {
-    float xv = x[p];
-    V = fmaf(xv * xv, __ldg(m2 + p), V);
+  auto term = [&](float xv, float mv) {
+    V = fmaf(xv * xv, mv, V);
     inexact |= (__bfloat162float(__float2bfloat16_rn(xv)) != xv);
+  };
+  if ((n_pix & 3) == 0 && aligned(img, 16) && aligned(m2, 16)) {
+    // 16-byte loads, four of each row in flight: with a few frames the pass
+    // is one CTA's load latency after another
+    const float4 *x4 = reinterpret_cast<const float4 *>(x);
+    const float4 *m4 = reinterpret_cast<const float4 *>(m2);
+    const int64_t n4 = n_pix >> 2;
+    constexpr int U = 4;
+    for (int64_t p = tid; p < n4; p += RR_THREADS * U) {
+      float4 xv[U], mv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const bool in = p + u * RR_THREADS < n4;
+        xv[u] = in ? __ldg(x4 + p + u * RR_THREADS) : make_float4(0.f, 0.f, 0.f, 0.f);
+        mv[u] = in ? __ldg(m4 + p + u * RR_THREADS) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        term(xv[u].x, mv[u].x);
+        term(xv[u].y, mv[u].y);
+        term(xv[u].z, mv[u].z);
+        term(xv[u].w, mv[u].w);
+      }
+    }
+  } else {
+    for (int64_t p = tid; p < n_pix; p += RR_THREADS) term(x[p], __ldg(m2 + p));
   }
   // warp merge of the per-thread lists: 8 rounds of a lexicographic minimum
   int head = 0;
@@ -540,18 +565,6 @@ __global__ void __launch_bounds__(RR_THREADS)
   }
 }
 
-// Exact FP32 distances of the 8 candidates of each frame, computed with the
-// arithmetic of the plain kernel (k_dist_argmin_f32): acc = fma(x_p, s_p, acc)
-// for p = 0 .. n_pix-1 in order, then (x2 + s2) - 2 acc, so the re-ranked
-// values are bit-identical to the plain path's.  A CTA takes 4 frames (32
-// (frame, candidate) chains, one per lane of warp 0); all its warps stream the
-// 4 frame rows and 32 candidate rows through shared memory in 64-pixel
-// chunks, RXE_STAGES - 1 chunks in flight (cp.async groups issued by warps
-// 1-3 while warp 0 runs the chains), rows padded to 68 floats so that the
-// chains' 16-byte reads of 8 consecutive rows fall on distinct banks.  Small
-// stages keep 29 KB of shared memory per CTA, so many CTAs (and their loads)
-// are resident per SM.  Lane 0 of each group of 8 keeps the lexicographic
-// minimum and evaluates the certificate.
 // The certificate's band: a bound on |approximate - exact| distance for any
 // reference (CERT_SIGMAS sigma of the bf16 rounding, per-pixel bound, plus
 // the FP32 accumulation error of both paths).
@@ -582,6 +595,99 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
                : "memory");
 }
 
+__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem)), "l"(gmem)
+               : "memory");
+}
+
+// acc = fma(x[k], s[k], acc) for k = 0 .. N-1 in order (both rows 16-byte
+// aligned in shared memory).  Unrolled throughout, with the loads of the next
+// 16 pixels issued before the current 16 FMAs, so the chain runs at the FMA
+// latency and not at that of the loads.
+template <int N>
+__device__ __forceinline__ float fma_chain(const float *x, const float *s, float acc) {
+  static_assert(N % 16 == 0, "whole groups of 16 pixels");
+  float4 xv[2][4], sv[2][4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    xv[0][u] = reinterpret_cast<const float4 *>(x)[u];
+    sv[0][u] = reinterpret_cast<const float4 *>(s)[u];
+  }
+#pragma unroll
+  for (int g = 0; g < N / 16; ++g) {
+    if (g + 1 < N / 16) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        xv[(g + 1) & 1][u] = reinterpret_cast<const float4 *>(x)[4 * (g + 1) + u];
+        sv[(g + 1) & 1][u] = reinterpret_cast<const float4 *>(s)[4 * (g + 1) + u];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float4 a = xv[g & 1][u], b = sv[g & 1][u];
+      acc = fmaf(a.x, b.x, acc);
+      acc = fmaf(a.y, b.y, acc);
+      acc = fmaf(a.z, b.z, acc);
+      acc = fmaf(a.w, b.w, acc);
+    }
+  }
+  return acc;
+}
+
+// Distance of this lane's candidate from its chain's sum, the frame's
+// lexicographic minimum over the 8 lanes, and the certificate (lane c = 0).
+__device__ __forceinline__ void rerank_finish(
+    unsigned mask, bool live, int64_t im, int c, bool valid, int32_t j, float x2, float band,
+    float acc, const float *cand_d, const int32_t *cand_i, const float *ref_sq,
+    int64_t ref_offset, float *work, int32_t *out_idx, float *out_dist, int32_t *uncertified,
+    int32_t *out_top) {
+  float dist = valid ? __fsub_rn(__fadd_rn(x2, ref_sq[j]), __fmul_rn(2.0f, acc))
+                     : __int_as_float(0x7f800000);
+  int32_t jj = valid ? j : INT32_MAX;
+#pragma unroll
+  for (int o = 4; o >= 1; o >>= 1) {
+    float od = __shfl_xor_sync(mask, dist, o, TOPK);
+    int32_t oj = __shfl_xor_sync(mask, jj, o, TOPK);
+    if (lex_less(od, oj, dist, jj)) {
+      dist = od;
+      jj = oj;
+    }
+  }
+  if (!live) return;
+  if (out_top) out_top[im * TOPK + c] = (j == INT32_MAX) ? -1 : (int32_t)(j + ref_offset);
+  if (c != 0) return;
+  out_idx[im] = jj == INT32_MAX ? -1 : (int32_t)(jj + ref_offset);
+  if (out_dist) out_dist[im] = dist;
+  if (!uncertified) return;
+  // certificate: every reference outside the 8 has approximate distance
+  // >= d8 (+ x2), and its plain-path distance differs from that by at most
+  // the bf16 rounding error (CERT_SIGMAS sigma, per-pixel bound) plus the
+  // FP32 accumulation error of both paths; the re-ranked best must lie below
+  int32_t j7 = cand_i[(size_t)im * TOPK + TOPK - 1];
+  int cert = 1;
+  if (j7 != INT32_MAX) {
+    float d8 = cand_d[(size_t)im * TOPK + TOPK - 1] + x2;
+    cert = (d8 - band - dist) > 0.0f ? 1 : 0;
+  }
+  uncertified[im] = cert ? 0 : 1;
+  // the range that must be searched when the frame is not certified: every
+  // reference whose approximate distance (without x2) lies within the band
+  // of the re-ranked best
+  work[im] = (dist - x2) + band;
+}
+
+// Exact FP32 distances of the 8 candidates of each frame, computed with the
+// arithmetic of the plain kernel (k_dist_argmin_f32): acc = fma(x_p, s_p, acc)
+// for p = 0 .. n_pix-1 in order, then (x2 + s2) - 2 acc, so the re-ranked
+// values are bit-identical to the plain path's.  A CTA takes 4 frames (32
+// (frame, candidate) chains, one per lane of warp 0); all its warps stream the
+// 4 frame rows and 32 candidate rows through shared memory in 64-pixel
+// chunks, RXE_STAGES - 1 chunks in flight (cp.async groups issued by warps
+// 1-3 while warp 0 runs the chains), rows padded to 68 floats so that the
+// chains' 16-byte reads of 8 consecutive rows fall on distinct banks.  Small
+// stages keep 29 KB of shared memory per CTA, so many CTAs (and their loads)
+// are resident per SM.  Lane 0 of each group of 8 keeps the lexicographic
+// minimum and evaluates the certificate.
 __global__ void __launch_bounds__(RX_THREADS)
     k_rerank_exact(const float *__restrict__ cand_d, const int32_t *__restrict__ cand_i,
                    const float *__restrict__ img, const float *__restrict__ img_sq,
@@ -687,39 +793,158 @@ __global__ void __launch_bounds__(RX_THREADS)
   float x2 = live ? img_sq[imc] : 0.0f;
   const float band = live ? cert_band(work[imc], x2, ref_sq_max, n_pix) : 0.0f;
   const bool valid = live && j >= 0 && j < n_ref && !rerank_skip(cand_d, imc, c, band);
-  float dist = valid ? __fsub_rn(__fadd_rn(x2, ref_sq[j]), __fmul_rn(2.0f, acc))
-                     : __int_as_float(0x7f800000);
-  int32_t jj = valid ? j : INT32_MAX;
-#pragma unroll
-  for (int o = 4; o >= 1; o >>= 1) {
-    float od = __shfl_xor_sync(0xffffffffu, dist, o, TOPK);
-    int32_t oj = __shfl_xor_sync(0xffffffffu, jj, o, TOPK);
-    if (lex_less(od, oj, dist, jj)) {
-      dist = od;
-      jj = oj;
+  rerank_finish(0xffffffffu, live, im, c, valid, j, x2, band, acc, cand_d, cand_i, ref_sq, ref_offset,
+                work, out_idx, out_dist, uncertified, out_top);
+}
+
+// The same distances, bit for bit, with one CTA per frame, for calls of up to
+// RF_RESIDENT frames an SM: warp 1 streams the frame's row and the rows of
+// the candidates in the band through a ring (one bulk copy a row and chunk;
+// 4-byte asynchronous copies where rows are not 16-byte aligned), warp 0 runs
+// the chains, lane c that of candidate c.  A chain of n_pix dependent FMAs
+// cannot be shortened, so with few frames its latency is the time (131 us for
+// 65,536 pixels at four clocks an FMA); here the loads, the copies and the
+// barriers run beside it: 5 frames of 65,536 pixels take 175 us against
+// 496 us in k_rerank_exact.  Beyond one wave of CTAs k_rerank_exact is faster:
+// its CTAs are all resident, walk the rows in step and share them in L2
+// (957 us against 1,600 us for 4,096 frames, 50,000 references).
+constexpr int RF_THREADS = 64;
+constexpr int RF_MAX_STAGES = 16;
+constexpr int RF_RING_FEW = 11776;  // floats: five 256-pixel stages of all nine rows, 4 CTAs an SM
+constexpr int RF_RING_MANY = 4096;  // 13 CTAs an SM
+constexpr int RF_RESIDENT_FEW = 4, RF_RESIDENT = 13;
+
+template <int C>
+__device__ __forceinline__ bool rerank_chain(const float *ring, int slot, int nr, int stages,
+                                             int64_t n_pix, uint64_t *full, uint64_t *empty,
+                                             float &acc) {
+  constexpr int STRIDE = C + 4;
+  const int64_t nchunks = (n_pix + C - 1) / C;
+  int s = 0;
+  uint32_t ph = 0;
+  for (int64_t ch = 0; ch < nchunks; ++ch) {
+    if (!__all_sync(0xffffffffu, mbar_wait_for(&full[s], ph, TIMEOUT_NS))) return false;
+    const float *xb = ring + (size_t)s * nr * STRIDE;
+    const float *sb = xb + slot * STRIDE;
+    const int64_t lim = n_pix - ch * C;
+    if (lim >= C) {
+      acc = fma_chain<C>(xb, sb, acc);
+    } else {
+      for (int k = 0; k < (int)lim; ++k) acc = fmaf(xb[k], sb[k], acc);
+    }
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(&empty[s]);
+    if (++s == stages) {
+      s = 0;
+      ph ^= 1;
     }
   }
-  if (!live) return;
-  if (out_top) out_top[im * TOPK + c] = (j == INT32_MAX) ? -1 : (int32_t)(j + ref_offset);
-  if (c != 0) return;
-  out_idx[im] = jj == INT32_MAX ? -1 : (int32_t)(jj + ref_offset);
-  if (out_dist) out_dist[im] = dist;
-  if (!uncertified) return;
-  // certificate: every reference outside the 8 has approximate distance
-  // >= d8 (+ x2), and its plain-path distance differs from that by at most
-  // the bf16 rounding error (CERT_SIGMAS sigma, per-pixel bound) plus the
-  // FP32 accumulation error of both paths; the re-ranked best must lie below
-  int32_t j7 = cand_i[(size_t)im * TOPK + TOPK - 1];
-  int cert = 1;
-  if (j7 != INT32_MAX) {
-    float d8 = cand_d[(size_t)im * TOPK + TOPK - 1] + x2;
-    cert = (d8 - band - dist) > 0.0f ? 1 : 0;
+  return true;
+}
+
+__global__ void __launch_bounds__(RF_THREADS)
+    k_rerank_frame(const float *__restrict__ cand_d, const int32_t *__restrict__ cand_i,
+                   const float *__restrict__ img, const float *__restrict__ img_sq,
+                   int64_t n_img, const float *__restrict__ ref, const float *__restrict__ ref_sq,
+                   int64_t n_ref, float ref_sq_max, int64_t n_pix, int64_t ref_offset,
+                   float *__restrict__ work, int32_t *__restrict__ out_idx,
+                   float *__restrict__ out_dist, int32_t *__restrict__ uncertified,
+                   int32_t *__restrict__ out_top, unsigned int *__restrict__ err,
+                   int ring_floats) {
+  extern __shared__ __align__(16) float ring[];  // ring_floats
+  __shared__ __align__(8) uint64_t full[RF_MAX_STAGES], empty[RF_MAX_STAGES];
+  __shared__ int late;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t im = blockIdx.x;
+  if (im >= n_img) return;
+  const bool vec = (n_pix % 4) == 0 && aligned(img, 16) && aligned(ref, 16);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < RF_MAX_STAGES; ++s) {
+      mbar_init(&full[s], vec ? 1 : 32);
+      mbar_init(&empty[s], 1);
+    }
+    late = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  uncertified[im] = cert ? 0 : 1;
-  // the range that must be searched when the frame is not certified: every
-  // reference whose approximate distance (without x2) lies within the band
-  // of the re-ranked best
-  work[im] = (dist - x2) + band;
+  // candidates whose rows are read: an index outside [0, n_ref) (a candidate
+  // slot the GEMM did not write) never is
+  const int c = lane % TOPK;
+  const int32_t j = cand_i[(size_t)im * TOPK + c];
+  const float x2 = img_sq[im];
+  const float band = cert_band(work[im], x2, ref_sq_max, n_pix);
+  const bool valid = j >= 0 && j < n_ref && !rerank_skip(cand_d, im, c, band);
+  const unsigned vmask = __ballot_sync(0xffffffffu, valid) & 0xffu;
+  const int nr = 1 + __popc(vmask);  // row 0 the frame, then the candidates read
+  const int slot = valid ? 1 + __popc(vmask & ((1u << c) - 1)) : 0;
+  // the longest chunk that leaves four stages
+  const int C = 4 * nr * 260 <= ring_floats ? 256 : 4 * nr * 132 <= ring_floats ? 128 : 64;
+  const int stages = min(RF_MAX_STAGES, ring_floats / (nr * (C + 4)));
+  __syncthreads();
+  float acc = 0.0f;
+  if (warp == 1) {
+    // lane r < nr copies row r
+    const float *src = img + im * n_pix;
+    for (int q = 0; q < TOPK; ++q) {
+      const int sq = __shfl_sync(0xffffffffu, slot, q);
+      const int32_t jq = __shfl_sync(0xffffffffu, j, q);
+      if (sq > 0 && sq == lane) src = ref + (int64_t)jq * n_pix;
+    }
+    const int64_t nchunks = (n_pix + C - 1) / C;
+    int s = 0;
+    uint32_t ph = 1;  // the first round finds every stage empty
+    int64_t ch = 0;
+    for (; ch < nchunks; ++ch) {
+      if (!__all_sync(0xffffffffu, mbar_wait_for(&empty[s], ph, TIMEOUT_NS))) break;
+      const int64_t base = ch * C;
+      const int cnt = (int)(n_pix - base < C ? n_pix - base : C);
+      float *dst = ring + (size_t)s * nr * (C + 4);
+      if (vec) {
+        if (lane == 0) mbar_arrive_expect_tx(&full[s], (uint32_t)(nr * cnt * sizeof(float)));
+        __syncwarp();
+        if (lane < nr)
+          bulk_load(dst + lane * (C + 4), src + base, (uint32_t)(cnt * sizeof(float)), &full[s]);
+      } else {
+        for (int r = 0; r < nr; ++r) {
+          const float *row = reinterpret_cast<const float *>(__shfl_sync(
+              0xffffffffu, reinterpret_cast<unsigned long long>(src), r));
+          for (int q = lane; q < cnt; q += 32) cp_async4(dst + r * (C + 4) + q, row + base + q);
+        }
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(
+                         smem_u32(&full[s]))
+                     : "memory");
+      }
+      if (++s == stages) {
+        s = 0;
+        ph ^= 1;
+      }
+    }
+    if (ch < nchunks) {
+      // the chains gave up: let the copies in flight land before the CTA ends
+      late = 1;
+      for (int64_t f = ch > stages ? ch - stages : 0; f < ch; ++f)
+        mbar_wait_for(&full[f % stages], (uint32_t)((f / stages) & 1), TIMEOUT_NS);
+    }
+  } else {
+    const bool ok = C == 256   ? rerank_chain<256>(ring, slot, nr, stages, n_pix, full, empty, acc)
+                    : C == 128 ? rerank_chain<128>(ring, slot, nr, stages, n_pix, full, empty, acc)
+                               : rerank_chain<64>(ring, slot, nr, stages, n_pix, full, empty, acc);
+    if (!ok) late = 1;
+  }
+  __syncthreads();
+  if (threadIdx.x >= TOPK) return;
+  if (late) {
+    // a copy gave no sign within the bound: report it, the frame has no answer
+    if (out_top) out_top[im * TOPK + c] = -1;
+    if (c == 0) {
+      if (err) atomicExch(err, (unsigned int)(-SPF_ERR_TIMEOUT));
+      out_idx[im] = -1;
+      if (out_dist) out_dist[im] = __int_as_float(0x7fc00000);
+      if (uncertified) uncertified[im] = 0;
+    }
+    return;
+  }
+  rerank_finish(0xffu, true, im, c, valid, j, x2, band, acc, cand_d, cand_i, ref_sq, ref_offset,
+                work, out_idx, out_dist, uncertified, out_top);
 }
 
 constexpr size_t RX_SMEM = (size_t)RXE_STAGES * RX_ROWS * RXE_STRIDE * sizeof(float);
@@ -889,6 +1114,27 @@ static int rerank_smem_attr() {
                      "k_rerank_exact"));
   done[dev] = true;
   return SPF_OK;
+}
+
+// the exact re-rank of every frame's merged top 8, by the kernel its comment
+// chooses for this many frames
+static int launch_rerank(const float *cand_d, const int32_t *cand_i, const float *img,
+                         const float *img_sq, int64_t n_img, const float *ref,
+                         const float *ref_sq, int64_t n_ref, float ref_sq_max, int64_t n_pix,
+                         int64_t ref_offset, float *work, int32_t *idx, float *dist,
+                         int32_t *uncertified, int32_t *top8, unsigned int *err, cudaStream_t s) {
+  if (n_img <= (int64_t)RF_RESIDENT * sm_count()) {
+    const int ring = n_img <= (int64_t)RF_RESIDENT_FEW * sm_count() ? RF_RING_FEW : RF_RING_MANY;
+    k_rerank_frame<<<(unsigned)n_img, RF_THREADS, ring * sizeof(float), s>>>(
+        cand_d, cand_i, img, img_sq, n_img, ref, ref_sq, n_ref, ref_sq_max, n_pix, ref_offset,
+        work, idx, dist, uncertified, top8, err, ring);
+    return check_launch("k_rerank_frame");
+  }
+  SPF_TRY(rerank_smem_attr());
+  k_rerank_exact<<<(unsigned)((n_img + RX_FRAMES - 1) / RX_FRAMES), RX_THREADS, RX_SMEM, s>>>(
+      cand_d, cand_i, img, img_sq, n_img, ref, ref_sq, n_ref, ref_sq_max, n_pix, ref_offset, work,
+      idx, dist, uncertified, top8);
+  return check_launch("k_rerank_exact");
 }
 
 static int make_map(CUtensorMap *map, const void *base, int64_t rows, int64_t ld, int box_rows) {
@@ -1218,11 +1464,9 @@ static int rerank_impl(const char *name, float *d_cand_d, int32_t *d_cand_i, int
   k_merge_top8<<<(unsigned)n_img, RR_THREADS, 0, s>>>(d_cand_d, d_cand_i, n_tiles, d_img, n_img,
                                                       d_ref_m2, n_pix, d_work, d_mrg_d, d_mrg_i);
   SPF_TRY(check_launch("k_merge_top8"));
-  SPF_TRY(rerank_smem_attr());
-  k_rerank_exact<<<(unsigned)((n_img + RX_FRAMES - 1) / RX_FRAMES), RX_THREADS, RX_SMEM, s>>>(
-      d_mrg_d, d_mrg_i, d_img, d_img_sq, n_img, d_ref, d_ref_sq, n_ref, ref_sq_max, n_pix,
-      ref_offset, d_work, d_idx, d_dist, d_uncertified, d_top8);
-  return check_launch("k_rerank_exact");
+  return launch_rerank(d_mrg_d, d_mrg_i, d_img, d_img_sq, n_img, d_ref, d_ref_sq, n_ref,
+                       ref_sq_max, n_pix, ref_offset, d_work, d_idx, d_dist, d_uncertified,
+                       d_top8, device_error_word(), s);
 }
 
 int spf_rerank_fp32(float *d_cand_d, int32_t *d_cand_i, int64_t n_tiles, const float *d_img,
@@ -1440,11 +1684,9 @@ extern "C" int spf_match_bf16_static(const void *d_img_bf16, const float *d_img,
   k_merge_top8<<<(unsigned)n_img, RR_THREADS, 0, s>>>(cand_d, cand_i, tiles, d_img, n_img,
                                                       d_ref_m2, n_pix, work, cand_d, cand_i);
   SPF_TRY(check_launch("k_merge_top8 (static scratch)"));
-  SPF_TRY(rerank_smem_attr());
-  k_rerank_exact<<<(unsigned)((n_img + RX_FRAMES - 1) / RX_FRAMES), RX_THREADS, RX_SMEM, s>>>(
-      cand_d, cand_i, d_img, d_img_sq, n_img, d_ref, d_ref_sq, n_ref, ref_sq_max, n_pix, 0, work,
-      d_idx, d_dist, d_uncertified, nullptr);
-  SPF_TRY(check_launch("k_rerank_exact (static scratch)"));
+  SPF_TRY(launch_rerank(cand_d, cand_i, d_img, d_img_sq, n_img, d_ref, d_ref_sq, n_ref,
+                        ref_sq_max, n_pix, 0, work, d_idx, d_dist, d_uncertified, nullptr, err,
+                        s));
   // a GEMM that gave up a bounded wait left candidate slots unwritten: the
   // call's answers are then void, and every frame says so
   k_static_abort_mark<<<grid_for(n_img, 256, 1024), 256, 0, s>>>(err, n_img, d_idx, d_dist,

@@ -55,6 +55,16 @@ __device__ __forceinline__ bool mbar_wait_for(uint64_t *bar, uint32_t parity,
   }
 }
 
+// Untiled bulk copy; dst, src and bytes multiples of 16.
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes,
+                                          uint64_t *bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
+          "r"(smem_u32(dst)),
+      "l"(src), "r"(bytes), "r"(smem_u32(bar))
+      : "memory");
+}
+
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, uint64_t *bar,
                                             int x, int y) {
   asm volatile(
