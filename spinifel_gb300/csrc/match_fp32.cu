@@ -2,64 +2,101 @@
 // module and the FP32 distance + argmin that SNM computes with cuBLAS + CUB.
 //
 // Both operands are row-major with the pixel axis contiguous ("K-major"):
-// images [n_img][n_pix] and references [n_ref][n_pix].  A CTA computes a
-// 128 x 128 tile of (image, reference) pairs with 256 threads, each thread an
-// 8 x 8 register tile, K staged through shared memory in steps of 16 pixels
-// with register double-buffering.  The tile order is grouped (8 image tiles
-// per group) so that CTAs resident at the same time share image and
-// reference rows in L2.
+// images [n_img][n_pix] and references [n_ref][n_pix].  A CTA computes a tile
+// of (image, reference) pairs, each thread a register tile, K staged through
+// shared memory in steps of 16 pixels with register double-buffering.  The
+// tile order is grouped (8 image tiles per group) so that CTAs resident at
+// the same time share image and reference rows in L2.
 #include "common.cuh"
 
 namespace spf {
 
-constexpr int TB_M = 128;  // image rows per CTA
-constexpr int TB_N = 128;  // reference rows per CTA
 constexpr int TB_K = 16;
-constexpr int TB_THREADS = 256;
 constexpr int GROUP_M = 8;
 
 enum class Mode { DIFF, DOT };
 
-template <typename T>
+// TM x TN pairs by a CTA, RM x RN by a thread (rows in groups of four, so a
+// warp's 16-byte shared reads are free of bank conflicts).  Every pair's sum
+// is one chain over the pixels in order whatever the tile, so the tile never
+// changes a bit of the result.
+//
+// PF k-steps of both operands are on their way in registers: a 32-pair tile
+// has two warps, and with few of them on an SM nothing else hides a step's
+// loads (32 x 8,000 pairs of 16,384 pixels: 623 us with one step, 525 with
+// four).  MINB CTAs an SM are asked of the compiler for the 128-pair tile's
+// argmin (54.0 TFLOP/s against 49.3 with one).
+template <int TM_, int TN_, int RM_, int RN_, int PF_>
+struct Tile {
+  static constexpr int TM = TM_, TN = TN_, RM = RM_, RN = RN_, PF = PF_;
+  static constexpr int MINB = TM == 128 ? 2 : 1;
+  static constexpr int NTX = TN / RN, THREADS = NTX * (TM / RM);
+  static_assert((RM == 8 || RM == 4) && (RN == 8 || RN == 4) && NTX <= 32, "row groups of four");
+  __device__ static __forceinline__ int row(int ty, int i) {
+    return ty * 4 + (i & 3) + (TM / 2) * (i >> 2);
+  }
+  __device__ static __forceinline__ int col(int tx, int j) {
+    return tx * 4 + (j & 3) + (TN / 2) * (j >> 2);
+  }
+};
+using Tile128 = Tile<128, 128, 8, 8, 1>;  // 256 threads
+using Tile64 = Tile<64, 64, 8, 4, 1>;     // 128 threads
+using Tile32 = Tile<32, 32, 4, 4, 4>;     // 64 threads
+
+template <typename T, int ROWS, int THREADS, bool VEC>
 struct TileLoader {
-  // 128 rows x 16 k per tile = 2048 elements, 8 per thread as 2 x 4.
-  T v[2][4];
+  // ROWS x 16 k per tile, N groups of four per thread.  FP32 rows that are
+  // 16-byte aligned move as float4 (group g of row r); others element by
+  // element with 16 lanes along a row, so that a warp's load touches two
+  // rows' 64 bytes and not eight rows four times over (333 x 1,999 pairs of
+  // 5,550 pixels: 342 us against 455).
+  static constexpr int N = ROWS * 4 / THREADS;
+  static_assert(THREADS % 16 == 0, "whole rows of lanes");
+  T v[N][4];
   __device__ __forceinline__ void load(const T *__restrict__ base, int64_t n_rows, int64_t ld,
-                                       int64_t K, int64_t row0, int64_t k0, bool vec) {
-    int tid = threadIdx.x;
+                                       int64_t K, int64_t row0, int64_t k0) {
+    const int tid = threadIdx.x;
+    if constexpr (VEC) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      int idx = tid + i * TB_THREADS;
-      int r = idx >> 2;
-      int kq = (idx & 3) * 4;
-      int64_t row = row0 + r;
-      int64_t k = k0 + kq;
-      if (row < n_rows) {
+      for (int i = 0; i < N; ++i) {
+        const int idx = tid + i * THREADS;
+        const int64_t row = row0 + (idx >> 2);
+        const int64_t k = k0 + (idx & 3) * 4;
         const T *p = base + row * ld + k;
-        if constexpr (sizeof(T) == 4) {
-          if (vec && k + 3 < K) {
-            float4 f = __ldg(reinterpret_cast<const float4 *>(p));
-            v[i][0] = f.x; v[i][1] = f.y; v[i][2] = f.z; v[i][3] = f.w;
-            continue;
-          }
+        if (row < n_rows && k + 3 < K) {
+          const float4 f = __ldg(reinterpret_cast<const float4 *>(p));
+          v[i][0] = f.x; v[i][1] = f.y; v[i][2] = f.z; v[i][3] = f.w;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[i][j] = row < n_rows && k + j < K ? __ldg(p + j) : T(0);
         }
+      }
+    } else {
+      const int64_t k = k0 + (tid & 15);
+      const int rows = (int)(n_rows - row0 < ROWS ? n_rows - row0 : ROWS);
+      const int r0 = k < K ? tid >> 4 : ROWS;  // past K: no row
+      const T *p = base + (row0 + (tid >> 4)) * ld + k;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[i][j] = (k + j < K) ? __ldg(p + j) : T(0);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v[i][j] = T(0);
+      for (int e = 0; e < 4 * N; ++e) {
+        v[e >> 2][e & 3] = r0 + e * (THREADS / 16) < rows ? __ldg(p) : T(0);
+        p += (THREADS / 16) * ld;
       }
     }
   }
-  __device__ __forceinline__ void store(T (*s)[TB_M + 4]) {
-    int tid = threadIdx.x;
+  __device__ __forceinline__ void store(T (*s)[ROWS + 4]) {
+    const int tid = threadIdx.x;
+    if constexpr (VEC) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      int idx = tid + i * TB_THREADS;
-      int r = idx >> 2;
-      int kq = (idx & 3) * 4;
+      for (int i = 0; i < N; ++i) {
+        const int idx = tid + i * THREADS;
+        const int r = idx >> 2, kq = (idx & 3) * 4;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) s[kq + j][r] = v[i][j];
+        for (int j = 0; j < 4; ++j) s[kq + j][r] = v[i][j];
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4 * N; ++e)
+        s[tid & 15][(tid >> 4) + e * (THREADS / 16)] = v[e >> 2][e & 3];
     }
   }
 };
@@ -77,147 +114,179 @@ __device__ __forceinline__ void tile_coords(int64_t n_img_tiles, int64_t n_ref_t
   nt = in / gm;
 }
 
-// acc[i][j] accumulates for image row (ty*4 + i%4 + 64*(i/4)) and reference
-// row (tx*4 + j%4 + 64*(j/4)) of the tile.
-template <typename T, Mode MODE>
+// acc[i][j] accumulates for image row TL::row(ty, i) and reference row
+// TL::col(tx, j) of the tile.
+template <typename T, Mode MODE, class TL, bool VEC>
 __device__ __forceinline__ void tile_mainloop(const T *__restrict__ A, int64_t n_a,
                                               const T *__restrict__ B, int64_t n_b, int64_t ld,
-                                              int64_t K, int64_t a0, int64_t b0, T acc[8][8],
-                                              T (*As)[TB_K][TB_M + 4],
-                                              T (*Bs)[TB_K][TB_N + 4]) {
-  const int tx = threadIdx.x & 15;
-  const int ty = threadIdx.x >> 4;
-  const bool vec = (sizeof(T) == 4) && (ld % 4 == 0) && aligned(A, 16) && aligned(B, 16);
+                                              int64_t K, int64_t a0, int64_t b0,
+                                              T acc[TL::RM][TL::RN],
+                                              T (*As)[TB_K][TL::TM + 4],
+                                              T (*Bs)[TB_K][TL::TN + 4]) {
+  constexpr int RM = TL::RM, RN = TL::RN;
+  const int tx = threadIdx.x % TL::NTX;
+  const int ty = threadIdx.x / TL::NTX;
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < RM; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = T(0);
-  TileLoader<T> la, lb;
-  int64_t ktiles = (K + TB_K - 1) / TB_K;
+    for (int j = 0; j < RN; ++j) acc[i][j] = T(0);
+  // FP64 tiles are bound by the FP64 pipe; element loads need the registers
+  constexpr int PF = sizeof(T) == 8 ? 1 : VEC ? TL::PF : TL::PF < 2 ? TL::PF : 2;
+  TileLoader<T, TL::TM, TL::THREADS, VEC> la[PF];
+  TileLoader<T, TL::TN, TL::THREADS, VEC> lb[PF];
+  const int64_t ktiles = (K + TB_K - 1) / TB_K;
   if (ktiles == 0) return;
-  la.load(A, n_a, ld, K, a0, 0, vec);
-  lb.load(B, n_b, ld, K, b0, 0, vec);
-  la.store(As[0]);
-  lb.store(Bs[0]);
+  // k-step t travels in slot t mod PF (a step past the end loads zeros)
+#pragma unroll
+  for (int p = 0; p < PF; ++p) {
+    la[p].load(A, n_a, ld, K, a0, p * TB_K);
+    lb[p].load(B, n_b, ld, K, b0, p * TB_K);
+  }
+  la[0].store(As[0]);
+  lb[0].store(Bs[0]);
+  la[0].load(A, n_a, ld, K, a0, PF * TB_K);
+  lb[0].load(B, n_b, ld, K, b0, PF * TB_K);
+  T fa[2][RM], fb[2][RN];
+  auto frag = [&](int f, int cur, int k) {
+#pragma unroll
+    for (int i = 0; i < RM; ++i) fa[f][i] = As[cur][k][TL::row(ty, i)];
+#pragma unroll
+    for (int j = 0; j < RN; ++j) fb[f][j] = Bs[cur][k][TL::col(tx, j)];
+  };
   __syncthreads();
-  for (int64_t kt = 0; kt < ktiles; ++kt) {
-    int cur = kt & 1;
-    bool more = kt + 1 < ktiles;
-    if (more) {
-      la.load(A, n_a, ld, K, a0, (kt + 1) * TB_K, vec);
-      lb.load(B, n_b, ld, K, b0, (kt + 1) * TB_K, vec);
-    }
+  for (int64_t kt0 = 0; kt0 < ktiles; kt0 += PF) {
 #pragma unroll
-    for (int k = 0; k < TB_K; ++k) {
-      T a[8], b[8];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        a[i] = As[cur][k][ty * 4 + i];
-        a[i + 4] = As[cur][k][64 + ty * 4 + i];
-        b[i] = Bs[cur][k][tx * 4 + i];
-        b[i + 4] = Bs[cur][k][64 + tx * 4 + i];
+    for (int u = 0; u < PF; ++u) {
+      const int64_t kt = kt0 + u;
+      if (kt >= ktiles) break;
+      const int cur = kt & 1;
+      const int slot = (u + 1) % PF;  // of step kt + 1
+      if (kt + 1 < ktiles) {
+        la[slot].store(As[cur ^ 1]);
+        lb[slot].store(Bs[cur ^ 1]);
+        la[slot].load(A, n_a, ld, K, a0, (kt + 1 + PF) * TB_K);
+        lb[slot].load(B, n_b, ld, K, b0, (kt + 1 + PF) * TB_K);
       }
-      if constexpr (sizeof(T) == 4) {
-        // two outputs per instruction (packed sub / fma, each lane the same
-        // IEEE operation as below, so every output's chain is unchanged)
+      frag(0, cur, 0);
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+      for (int k = 0; k < TB_K; ++k) {
+        // the next pixel's operands are read while this one's FMAs issue
+        const int f = k & 1;
+        if (k + 1 < TB_K) frag(f ^ 1, cur, k + 1);
+        const T *a = fa[f], *b = fb[f];
+        if constexpr (sizeof(T) == 4) {
+          // two outputs per instruction (packed sub / fma, each lane the same
+          // IEEE operation as below, so every output's chain is unchanged)
 #pragma unroll
-          for (int j = 0; j < 8; j += 2) {
-            const float2 ai = make_float2(a[i], a[i]), bj = make_float2(b[j], b[j + 1]);
-            const float2 c = make_float2(acc[i][j], acc[i][j + 1]);
-            float2 r;
-            if constexpr (MODE == Mode::DIFF) {
-              const float2 d = fsub2(ai, bj);
-              r = ffma2(d, d, c);
-            } else {
-              r = ffma2(ai, bj, c);
+          for (int i = 0; i < RM; ++i)
+#pragma unroll
+            for (int j = 0; j < RN; j += 2) {
+              const float2 ai = make_float2(a[i], a[i]), bj = make_float2(b[j], b[j + 1]);
+              const float2 c = make_float2(acc[i][j], acc[i][j + 1]);
+              float2 r;
+              if constexpr (MODE == Mode::DIFF) {
+                const float2 d = fsub2(ai, bj);
+                r = ffma2(d, d, c);
+              } else {
+                r = ffma2(ai, bj, c);
+              }
+              acc[i][j] = r.x;
+              acc[i][j + 1] = r.y;
             }
-            acc[i][j] = r.x;
-            acc[i][j + 1] = r.y;
-          }
-      } else {
+        } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+          for (int i = 0; i < RM; ++i)
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            if constexpr (MODE == Mode::DIFF) {
-              T d = a[i] - b[j];
-              acc[i][j] = fma(d, d, acc[i][j]);
-            } else {
-              acc[i][j] = fma(a[i], b[j], acc[i][j]);
+            for (int j = 0; j < RN; ++j) {
+              if constexpr (MODE == Mode::DIFF) {
+                T d = a[i] - b[j];
+                acc[i][j] = fma(d, d, acc[i][j]);
+              } else {
+                acc[i][j] = fma(a[i], b[j], acc[i][j]);
+              }
             }
-          }
+        }
       }
+      __syncthreads();
     }
-    if (more) {
-      la.store(As[cur ^ 1]);
-      lb.store(Bs[cur ^ 1]);
-    }
-    __syncthreads();
   }
 }
 
+template <typename T, Mode MODE, class TL>
+__device__ __forceinline__ void tile_sums(const T *__restrict__ A, int64_t n_a,
+                                          const T *__restrict__ B, int64_t n_b, int64_t ld,
+                                          int64_t K, int64_t a0, int64_t b0,
+                                          T acc[TL::RM][TL::RN], T (*As)[TB_K][TL::TM + 4],
+                                          T (*Bs)[TB_K][TL::TN + 4]) {
+  if (sizeof(T) == 4 && ld % 4 == 0 && aligned(A, 16) && aligned(B, 16))
+    tile_mainloop<T, MODE, TL, sizeof(T) == 4>(A, n_a, B, n_b, ld, K, a0, b0, acc, As, Bs);
+  else
+    tile_mainloop<T, MODE, TL, false>(A, n_a, B, n_b, ld, K, a0, b0, acc, As, Bs);
+}
+
 // out[d][r] = sum_{p < K} (data[d][p] - ref[r][p])^2
-template <typename T>
-__global__ void __launch_bounds__(TB_THREADS) k_knn_eudist(const T *__restrict__ ref,
+template <typename T, class TL>
+__global__ void __launch_bounds__(TL::THREADS) k_knn_eudist(const T *__restrict__ ref,
                                                            const T *__restrict__ data,
                                                            int64_t n_ref, int64_t n_data,
                                                            int64_t ld, int64_t K,
                                                            T *__restrict__ out, int group_m) {
+  constexpr int TB_M = TL::TM, TB_N = TL::TN, RM = TL::RM, RN = TL::RN;
   __shared__ __align__(16) T As[2][TB_K][TB_M + 4];
   __shared__ __align__(16) T Bs[2][TB_K][TB_N + 4];
   int64_t n_img_tiles = (n_data + TB_M - 1) / TB_M;
   int64_t n_ref_tiles = (n_ref + TB_N - 1) / TB_N;
   int64_t mt, nt;
   tile_coords(n_img_tiles, n_ref_tiles, group_m, mt, nt);
-  T acc[8][8];
-  tile_mainloop<T, Mode::DIFF>(data, n_data, ref, n_ref, ld, K, mt * TB_M, nt * TB_N, acc, As,
-                               Bs);
-  const int tx = threadIdx.x & 15;
-  const int ty = threadIdx.x >> 4;
+  T acc[RM][RN];
+  tile_sums<T, Mode::DIFF, TL>(data, n_data, ref, n_ref, ld, K, mt * TB_M, nt * TB_N, acc,
+                                   As, Bs);
+  const int tx = threadIdx.x % TL::NTX;
+  const int ty = threadIdx.x / TL::NTX;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    int64_t d = mt * TB_M + ty * 4 + (i & 3) + 64 * (i >> 2);
+  for (int i = 0; i < RM; ++i) {
+    int64_t d = mt * TB_M + TL::row(ty, i);
     if (d >= n_data) continue;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      int64_t r = nt * TB_N + tx * 4 + (j & 3) + 64 * (j >> 2);
+    for (int j = 0; j < RN; ++j) {
+      int64_t r = nt * TB_N + TL::col(tx, j);
       if (r < n_ref) out[d * n_ref + r] = acc[i][j];
     }
   }
 }
 
 // Running argmin of x2 + s2 - 2 x.s, packed (order key << 32 | index).
-__global__ void __launch_bounds__(TB_THREADS) k_dist_argmin_f32(
+template <class TL>
+__global__ void __launch_bounds__(TL::THREADS, TL::MINB) k_dist_argmin_f32(
     const float *__restrict__ img, const float *__restrict__ img_sq, int64_t n_img,
     const float *__restrict__ ref, const float *__restrict__ ref_sq, int64_t n_ref, int64_t K,
     int64_t ref_offset, unsigned long long *__restrict__ best, int group_m) {
+  constexpr int TB_M = TL::TM, TB_N = TL::TN, RM = TL::RM, RN = TL::RN;
   __shared__ __align__(16) float As[2][TB_K][TB_M + 4];
   __shared__ __align__(16) float Bs[2][TB_K][TB_N + 4];
   int64_t n_img_tiles = (n_img + TB_M - 1) / TB_M;
   int64_t n_ref_tiles = (n_ref + TB_N - 1) / TB_N;
   int64_t mt, nt;
   tile_coords(n_img_tiles, n_ref_tiles, group_m, mt, nt);
-  float acc[8][8];
-  tile_mainloop<float, Mode::DOT>(img, n_img, ref, n_ref, K, K, mt * TB_M, nt * TB_N, acc, As,
-                                  Bs);
-  const int tx = threadIdx.x & 15;
-  const int ty = threadIdx.x >> 4;
-  float s2[8];
-  int64_t rr[8];
+  float acc[RM][RN];
+  tile_sums<float, Mode::DOT, TL>(img, n_img, ref, n_ref, K, K, mt * TB_M, nt * TB_N, acc,
+                                      As, Bs);
+  const int tx = threadIdx.x % TL::NTX;
+  const int ty = threadIdx.x / TL::NTX;
+  float s2[RN];
+  int64_t rr[RN];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    rr[j] = nt * TB_N + tx * 4 + (j & 3) + 64 * (j >> 2);
+  for (int j = 0; j < RN; ++j) {
+    rr[j] = nt * TB_N + TL::col(tx, j);
     s2[j] = rr[j] < n_ref ? ref_sq[rr[j]] : 0.0f;
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    int64_t d = mt * TB_M + ty * 4 + (i & 3) + 64 * (i >> 2);
+  for (int i = 0; i < RM; ++i) {
+    int64_t d = mt * TB_M + TL::row(ty, i);
     float x2 = d < n_img ? img_sq[d] : 0.0f;
     unsigned long long key = ~0ULL;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < RN; ++j) {
       if (rr[j] < n_ref) {
         float dist = __fsub_rn(__fadd_rn(x2, s2[j]), __fmul_rn(2.0f, acc[i][j]));
         unsigned long long k2 =
@@ -225,10 +294,10 @@ __global__ void __launch_bounds__(TB_THREADS) k_dist_argmin_f32(
         key = k2 < key ? k2 : key;
       }
     }
-    // the 16 threads with this ty hold the other columns of the row
+    // the NTX threads with this ty hold the other columns of the row
 #pragma unroll
-    for (int o = 8; o >= 1; o >>= 1) {
-      unsigned long long other = __shfl_xor_sync(0xffffffffu, key, o, 16);
+    for (int o = TL::NTX / 2; o >= 1; o >>= 1) {
+      unsigned long long other = __shfl_xor_sync(0xffffffffu, key, o, TL::NTX);
       key = other < key ? other : key;
     }
     if (tx == 0 && d < n_img && key != ~0ULL) atomicMin(best + d, key);
@@ -296,22 +365,76 @@ __global__ void k_best64_init(double *best_dist, int64_t *best_idx, int64_t n) {
   }
 }
 
-// sum of squares per row (FP64 accumulation, one warp per row)
-__global__ void k_row_sqnorm(const float *__restrict__ x, int64_t n_rows, int64_t n_pix,
-                             float *__restrict__ out) {
-  int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int64_t r = warp; r < n_rows; r += nwarps) {
-    const float *p = x + r * n_pix;
-    double s = 0.0;
-    for (int64_t k = lane; k < n_pix; k += 32) {
-      double v = p[k];
-      s = fma(v, v, s);
-    }
+// Sum of squares per row, rounded to FP32, by one warp a row (W = 1) or one
+// CTA of W warps.  Each thread keeps its sum as an unevaluated pair of floats
+// (error-free product and sum: Dekker 1971, Knuth TAOCP 2, 4.2.2), good to
+// about 2^-40 of it, and the pairs are added in FP64.  FP64 in the loop (a
+// conversion and an FMA an element) runs at this chip's FP64 rate: 8,000 rows
+// of 16,384 pixels took 530 us, 107 us now.  A row whose sum overflows FP32 or
+// is so small that squares are lost to underflow is summed in FP64.
+template <int W>
+__global__ void __launch_bounds__(256) k_row_sqnorm(const float *__restrict__ x, int64_t n_rows,
+                                                    int64_t n_pix, float *__restrict__ out,
+                                                    int vec) {
+  __shared__ double part[8];
+  constexpr int T = 32 * W, RPB = 8 / W;  // threads a row, rows a CTA
+  const int t = threadIdx.x % T, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto row_sum = [&](double v) {  // over the row's threads, in every one of them
 #pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) out[r] = (float)s;
+    for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (W > 1) {
+      __syncthreads();
+      if (lane == 0) part[warp] = v;
+      __syncthreads();
+      v = 0.0;
+      for (int w = 0; w < W; ++w) v += part[w];
+    }
+    return v;
+  };
+  const int64_t step = (int64_t)gridDim.x * RPB;
+  for (int64_t r = (int64_t)blockIdx.x * RPB + threadIdx.x / T; r < n_rows; r += step) {
+    const float *p = x + r * n_pix;
+    float s = 0.0f, c = 0.0f;
+    auto add = [&](float v) {
+      const float q = __fmul_rn(v, v), e = __fmaf_rn(v, v, -q);
+      const float u = __fadd_rn(s, q), z = __fsub_rn(u, s);
+      c = __fadd_rn(c, __fadd_rn(__fadd_rn(__fsub_rn(s, __fsub_rn(u, z)), __fsub_rn(q, z)), e));
+      s = u;
+    };
+    if (vec) {
+      const float4 *p4 = reinterpret_cast<const float4 *>(p);
+      const int64_t n4 = n_pix >> 2;
+      constexpr int U = 4;
+      for (int64_t k = t; k < n4; k += T * U) {
+        float4 v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          v[u] = k + u * T < n4 ? __ldg(p4 + k + u * T) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          add(v[u].x);
+          add(v[u].y);
+          add(v[u].z);
+          add(v[u].w);
+        }
+      }
+    } else {
+      constexpr int U = 8;
+      for (int64_t k = t; k < n_pix; k += T * U) {
+        float v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = k + u * T < n_pix ? __ldg(p + k + u * T) : 0.0f;
+#pragma unroll
+        for (int u = 0; u < U; ++u) add(v[u]);
+      }
+    }
+    double sum = row_sum((double)s + (double)c);
+    if (!(sum > 1e-24 && sum < 3e38)) {  // the same for all threads of the row
+      double d = 0.0;
+      for (int64_t k = t; k < n_pix; k += T) d = fma((double)p[k], (double)p[k], d);
+      sum = row_sum(d);
+    }
+    if (t == 0) out[r] = (float)sum;
   }
 }
 
@@ -559,6 +682,50 @@ __global__ void k_topk(const T *__restrict__ dist, int64_t n_rows, int64_t n_col
 
 using namespace spf;
 
+// Tile of the distance kernels for n_a x n_b pairs: the one whose tiles the
+// busiest SM finishes first, at the rates the tiles reach with a full chip
+// (128: 54, 64: 47, 32: 30 TFLOP/s).  The 128-pair tile reads shared memory
+// least per operation; with few tiles most of the chip would idle under it:
+// 333 x 1,999 x 5,550 takes 608 us there and 342 us with 32-pair tiles,
+// 500 x 2,000 x 4,096 takes 436 us and, with 64-pair tiles, 266 us (FP64:
+// 35.9 and 17.8 ms); 1,500 x 8,000 x 8,192 takes 3.65 ms there, 4.2 ms with 64.
+template <int PAIRS>
+static double tile_cost(int64_t n_a, int64_t n_b, double rate) {
+  const int64_t t = ((n_a + PAIRS - 1) / PAIRS) * ((n_b + PAIRS - 1) / PAIRS);
+  const int64_t sms = sm_count();
+  return (double)((t + sms - 1) / sms) * PAIRS * PAIRS / rate;
+}
+static int64_t tile_count(int64_t n_a, int64_t n_b, int pairs) {
+  return ((n_a + pairs - 1) / pairs) * ((n_b + pairs - 1) / pairs);
+}
+// 128, 64 or 32
+static int pick_tile(int64_t n_a, int64_t n_b, double rate64, double rate32) {
+  const double c128 = tile_cost<128>(n_a, n_b, 1.0), c64 = tile_cost<64>(n_a, n_b, rate64),
+               c32 = tile_cost<32>(n_a, n_b, rate32);
+  if (c128 <= c64 && c128 <= c32) return 128;
+  return c64 <= c32 ? 64 : 32;
+}
+
+#define SPF_TILE_DISPATCH(pairs, KERNEL_CALL)                 \
+  switch (pairs) {                                            \
+    case 128: { using TL = Tile128; KERNEL_CALL; break; }     \
+    case 64: { using TL = Tile64; KERNEL_CALL; break; }       \
+    default: { using TL = Tile32; KERNEL_CALL; break; }       \
+  }
+
+template <typename T>
+static int launch_eudist(const T *ref, const T *data, int64_t n_ref, int64_t n_data,
+                         int64_t n_pix, int64_t K, T *out, void *stream, const char *name) {
+  const int pairs = pick_tile(n_data, n_ref, 0.9, 0.6);
+  const int64_t tiles = tile_count(n_data, n_ref, pairs);
+  SPF_REQUIRE(tiles < (1LL << 31), "%s: too many tiles", name);
+  const int group_m = (int)tune_get(SPF_TUNE_FP32_GROUP_M, GROUP_M);
+  SPF_TILE_DISPATCH(pairs, (k_knn_eudist<T, TL><<<(unsigned)tiles, TL::THREADS, 0,
+                                                  as_stream(stream)>>>(
+                               ref, data, n_ref, n_data, n_pix, K, out, group_m)));
+  return check_launch(name);
+}
+
 template <typename T>
 static int knn_eudist(const T *ref, const T *data, int64_t n_ref, int64_t n_data, int64_t n_pix,
                       T *out, void *stream, const char *name) {
@@ -566,12 +733,7 @@ static int knn_eudist(const T *ref, const T *data, int64_t n_ref, int64_t n_data
   if (n_ref == 0 || n_data == 0) return SPF_OK;
   SPF_REQUIRE(ref && data && out, "%s: NULL pointer", name);
   int64_t K = (n_pix / 16) * 16;  // the reference kernel drops the ragged tail
-  int64_t tiles = ((n_data + TB_M - 1) / TB_M) * ((n_ref + TB_N - 1) / TB_N);
-  SPF_REQUIRE(tiles < (1LL << 31), "%s: too many tiles", name);
-  int group_m = (int)tune_get(SPF_TUNE_FP32_GROUP_M, GROUP_M);
-  k_knn_eudist<T><<<(unsigned)tiles, TB_THREADS, 0, as_stream(stream)>>>(ref, data, n_ref, n_data,
-                                                                          n_pix, K, out, group_m);
-  return check_launch(name);
+  return launch_eudist<T>(ref, data, n_ref, n_data, n_pix, K, out, stream, name);
 }
 
 template <typename T>
@@ -616,8 +778,15 @@ int spf_row_sqnorm_f32(const float *d_x, int64_t n_rows, int64_t n_pix, float *d
   SPF_REQUIRE(n_rows >= 0 && n_pix >= 0, "spf_row_sqnorm_f32: negative size");
   if (n_rows == 0) return SPF_OK;
   SPF_REQUIRE(d_x && d_out, "spf_row_sqnorm_f32: NULL pointer");
-  int blocks = grid_for(n_rows * 32, 256, (int64_t)sm_count() * 32);
-  k_row_sqnorm<<<blocks, 256, 0, as_stream(stream)>>>(d_x, n_rows, n_pix, d_out);
+  const int vec = n_pix % 4 == 0 && aligned(d_x, 16);
+  cudaStream_t s = as_stream(stream);
+  // a warp a row for rows too short to give a CTA's threads a few loads each
+  if (n_pix <= 2048)
+    k_row_sqnorm<1><<<grid_for(n_rows, 8, (int64_t)sm_count() * 32), 256, 0, s>>>(d_x, n_rows, n_pix,
+                                                                             d_out, vec);
+  else
+    k_row_sqnorm<8><<<grid_for(n_rows, 1, (int64_t)sm_count() * 32), 256, 0, s>>>(d_x, n_rows, n_pix,
+                                                                             d_out, vec);
   return check_launch("spf_row_sqnorm_f32");
 }
 
@@ -696,12 +865,14 @@ int spf_dist_argmin_f32(const float *d_img, const float *d_img_sq, int64_t n_img
   SPF_REQUIRE(d_img && d_img_sq && d_ref && d_ref_sq && d_best,
               "spf_dist_argmin_f32: NULL pointer");
   SPF_REQUIRE(ref_offset + n_ref < (1LL << 32), "spf_dist_argmin_f32: index exceeds 32 bits");
-  int64_t tiles = ((n_img + TB_M - 1) / TB_M) * ((n_ref + TB_N - 1) / TB_N);
+  const int pairs = pick_tile(n_img, n_ref, 0.9, 0.6);
+  const int64_t tiles = tile_count(n_img, n_ref, pairs);
   SPF_REQUIRE(tiles < (1LL << 31), "spf_dist_argmin_f32: too many tiles");
-  k_dist_argmin_f32<<<(unsigned)tiles, TB_THREADS, 0, as_stream(stream)>>>(
-      d_img, d_img_sq, n_img, d_ref, d_ref_sq, n_ref, n_pix, ref_offset,
-      reinterpret_cast<unsigned long long *>(d_best),
-      (int)tune_get(SPF_TUNE_FP32_GROUP_M, GROUP_M));
+  SPF_TILE_DISPATCH(pairs, (k_dist_argmin_f32<TL><<<(unsigned)tiles, TL::THREADS, 0,
+                                                    as_stream(stream)>>>(
+                               d_img, d_img_sq, n_img, d_ref, d_ref_sq, n_ref, n_pix, ref_offset,
+                               reinterpret_cast<unsigned long long *>(d_best),
+                               (int)tune_get(SPF_TUNE_FP32_GROUP_M, GROUP_M))));
   return check_launch("spf_dist_argmin_f32");
 }
 
@@ -730,12 +901,8 @@ int spf_dist_f64(const double *d_ref, const double *d_data, int64_t n_ref, int64
   SPF_REQUIRE(n_ref >= 0 && n_data >= 0 && n_pix >= 0, "spf_dist_f64: negative size");
   if (n_ref == 0 || n_data == 0) return SPF_OK;
   SPF_REQUIRE(d_ref && d_data && d_out, "spf_dist_f64: NULL pointer");
-  const int64_t tiles = ((n_data + TB_M - 1) / TB_M) * ((n_ref + TB_N - 1) / TB_N);
-  SPF_REQUIRE(tiles < (1LL << 31), "spf_dist_f64: too many tiles");
-  const int group_m = (int)tune_get(SPF_TUNE_FP32_GROUP_M, GROUP_M);
-  k_knn_eudist<double><<<(unsigned)tiles, TB_THREADS, 0, as_stream(stream)>>>(
-      d_ref, d_data, n_ref, n_data, n_pix, n_pix, d_out, group_m);
-  return check_launch("spf_dist_f64");
+  return launch_eudist<double>(d_ref, d_data, n_ref, n_data, n_pix, n_pix, d_out, stream,
+                               "spf_dist_f64");
 }
 
 int spf_best64_init(double *d_best_dist, int64_t *d_best_idx, int64_t n_img, void *stream) {

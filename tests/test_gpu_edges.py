@@ -52,3 +52,57 @@ def test_ingest_norms_are_exact_sums(n_pix, top):
                                   .astype(np.float32))
     np.testing.assert_allclose(fs.n4.cpu().numpy().astype(np.float64),
                                np.sqrt(np.array(s4, dtype=np.float64)), rtol=2 ** -23)
+
+
+@pytest.mark.parametrize("n_pix", [1, 3, 32, 1000, 2048, 2049, 2052, 8200, 65537])
+@pytest.mark.parametrize("scale", [1.0, 1e-12, 1e-22, 1e15, 1e20])
+def test_row_sqnorm_is_the_rounded_sum(n_pix, scale):
+    """Within one FP32 rounding of the FP64 sum (2^-24, and 2^-30 for the sum
+    itself), also where squares under- or overflow FP32; NaN and infinity stay."""
+    from spinifel_gb300 import matching
+
+    rng = np.random.default_rng(n_pix)
+    x = (rng.standard_normal((5, n_pix)) * scale).astype(np.float32)
+    x[1] = 0.0
+    x[2, : n_pix // 2] *= 1e3
+    x[3, n_pix // 2] = np.inf
+    x[4, n_pix - 1] = np.nan
+    got = matching.row_sqnorm(torch.as_tensor(x, device="cuda")).cpu().numpy()
+    with np.errstate(over="ignore"):
+        want = (x.astype(np.float64) ** 2).sum(axis=1).astype(np.float32)
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
+    np.testing.assert_allclose(got[:4], want[:4], rtol=2 ** -24 * 1.02 + 2 ** -24,
+                               atol=2 ** -149)
+
+
+@pytest.mark.parametrize("n_img,n_ref,n_pix", [(1, 1, 1), (31, 33, 17), (64, 64, 16), (65, 129, 63),
+                                               (128, 128, 64), (129, 2000, 100), (700, 1300, 37),
+                                               (1500, 1400, 48), (33, 5000, 130)])
+def test_distance_tiles(n_img, n_ref, n_pix):
+    """Every tile of the distance kernels gives each pair's sequential chain:
+    FP32 and FP64 squared differences against an FP64 reference, the fused
+    argmin against the smallest of the distances it is defined on."""
+    from spinifel_gb300 import matching
+
+    rng = np.random.default_rng(n_img + n_ref)
+    x = rng.random((n_img, n_pix)).astype(np.float32)
+    r = rng.random((n_ref, n_pix)).astype(np.float32)
+    xd, rd = torch.as_tensor(x, device="cuda"), torch.as_tensor(r, device="cuda")
+    want = torch.cdist(xd.double(), rd.double(),
+                       compute_mode="donot_use_mm_for_euclid_dist").square()
+    got = matching.dist_f64(rd.double(), xd.double())
+    torch.testing.assert_close(got, want, rtol=(n_pix + 4) * 2.0 ** -52, atol=1e-300)
+    k16 = n_pix // 16 * 16
+    if k16:
+        w16 = (xd.double()[:, None, :k16] - rd.double()[None, :64, :k16]).square().sum(-1)
+        g16 = matching.knn_eudist(rd[:64].contiguous(), xd)
+        torch.testing.assert_close(g16.double(), w16, rtol=(n_pix + 4) * 2.0 ** -23, atol=1e-30)
+    xs, rs = matching.row_sqnorm(xd), matching.row_sqnorm(rd)
+    idx, dist = matching.argmin_fp32(xd, rd, xs, rs)
+    # acc is a chain of n_pix FMAs: at most n_pix 2^-24 of the sum of |x s|
+    err = (n_pix + 4) * 2.0 ** -24 * 2 * (xs.double()[:, None] + rs.double()[None, :])
+    best = want.min(dim=1).values
+    i = idx.long()
+    rows = torch.arange(n_img, device="cuda")
+    assert bool((dist.double() - want[rows, i]).abs().le(err[rows, i]).all())
+    assert bool((want[rows, i] - best).le(2 * err.max(dim=1).values).all())
