@@ -326,6 +326,16 @@ int spf_best64_init(double *d_best_dist, int64_t *d_best_idx, int64_t n_img, voi
 int spf_argmin_rows_f64(const double *d_dist, int64_t n_img, int64_t n_ref, int64_t ref_offset,
                         double *d_best_dist, int64_t *d_best_idx, void *stream);
 
+/* The same running minimum over n_ref references without the distance block:
+ * an FP32 pass with an error bound leaves the references that can hold each
+ * image's minimum, and only those get their FP64 distance (the arithmetic of
+ * spf_dist_f64, so distances, indices and ties are the full computation's).
+ * d_work: spf_argmin_f64_work_bytes bytes of device memory. */
+int64_t spf_argmin_f64_work_bytes(int64_t n_img, int64_t n_ref, int64_t n_pix);
+int spf_argmin_f64(const double *d_img, int64_t n_img, const double *d_ref, int64_t n_ref,
+                   int64_t n_pix, int64_t ref_offset, void *d_work, int64_t work_bytes,
+                   double *d_best_dist, int64_t *d_best_idx, void *stream);
+
 /* ---- autocorrelation merge: operator and device-resident CG -----------
  * Replaces Merge.setup_linops / W_matvec / cg
  * (spinifel/sequential/autocorrelation.py:152-225):

@@ -175,6 +175,9 @@ SIGNATURES = {
     "spf_nufft64_t1_finish": [_c_void_p, _int, _c_void_p, _c_void_p, _c_void_p],
     "spf_dist_f64": [_c_void_p, _c_void_p, _i64, _i64, _i64, _c_void_p, _c_void_p],
     "spf_best64_init": [_c_void_p, _c_void_p, _i64, _c_void_p],
+    "spf_argmin_f64_work_bytes": [_i64, _i64, _i64],
+    "spf_argmin_f64": [_c_void_p, _i64, _c_void_p, _i64, _i64, _i64, _c_void_p, _i64, _c_void_p,
+                       _c_void_p, _c_void_p],
     "spf_argmin_rows_f64": [_c_void_p, _i64, _i64, _i64, _c_void_p, _c_void_p, _c_void_p],
     "spf_phase_create": [_int, ctypes.POINTER(_c_void_p)],
     "spf_phase_destroy": [_c_void_p],
@@ -194,6 +197,7 @@ _RESTYPES = {
     "spf_status_string": ctypes.c_char_p,
     "spf_last_error": ctypes.c_char_p,
     "spf_launch_count": ctypes.c_uint64,
+    "spf_argmin_f64_work_bytes": ctypes.c_int64,
     "spf_dist_topk_bf16_tiles": ctypes.c_int64,
     "spf_dist_topk_bf16_tile_refs": ctypes.c_int64,
     "spf_serve_clock": ctypes.c_double,

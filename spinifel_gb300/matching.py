@@ -82,6 +82,10 @@ def argmin_fp32(images: torch.Tensor, refs: torch.Tensor, images_sq=None, refs_s
     return t.result()
 
 
+# below this many pixels the whole FP64 block is as quick as picking minima
+MINIMA_MIN_PIXELS = 64
+
+
 class BestTracker64:
     """FP64 running (distance, index) minimum per image across reference
     batches, for matching at the reference's double precision: each batch's
@@ -104,8 +108,31 @@ class BestTracker64:
                   _lib.stream_handle())
 
     def update_fp64(self, img, ref, ref_offset: int, work: torch.Tensor | None = None):
-        """Fold the distances of img [n_img, n_pix] to ref [n_ref, n_pix]."""
+        """Fold the distances of img [n_img, n_pix] to ref [n_ref, n_pix].
+        With `work` ([n_img * n_ref] float64) the whole distance block is
+        computed and left there; without it only the distances that can be
+        an image's minimum are (spf_argmin_f64: the same indices and bits)."""
+        if work is None and self._fold_minima(img, ref, ref_offset):
+            return
         self.update_block(dist_f64(ref, img, out=work), ref_offset)
+
+    def _fold_minima(self, img, ref, ref_offset: int) -> bool:
+        _lib.require_cuda(ref, "ref", torch.float64)
+        _lib.require_cuda(img, "img", torch.float64)
+        n_img, n_ref = img.shape[0], ref.shape[0]
+        if img.dim() != 2 or ref.dim() != 2 or img.shape[1] != ref.shape[1] \
+                or n_img != self.n_img or not n_img or not n_ref \
+                or img.shape[1] < MINIMA_MIN_PIXELS or n_img * n_ref >= 1 << 31:
+            return False
+        size = int(_lib.lib().spf_argmin_f64_work_bytes(n_img, n_ref, img.shape[1]))
+        try:
+            ws = torch.empty(size, dtype=torch.uint8, device=img.device)
+        except torch.OutOfMemoryError:
+            return False
+        _lib.call("spf_argmin_f64", _lib.ptr(img), n_img, _lib.ptr(ref), n_ref, img.shape[1],
+                  int(ref_offset), _lib.ptr(ws), size, _lib.ptr(self.best_dist),
+                  _lib.ptr(self.best_idx), _lib.stream_handle())
+        return True
 
     def result(self):
         return self.best_idx, self.best_dist
@@ -132,13 +159,8 @@ def argmin_fp64(images: torch.Tensor, refs: torch.Tensor, batch: int = 4096):
     """Index (int64) and FP64 distance of the nearest reference for every
     image, references taken in batches of `batch` rows."""
     t = BestTracker64(images.shape[0], images.device)
-    work = None
     for st in range(0, refs.shape[0], batch):
-        blk = refs[st:st + batch]
-        if work is None or work.numel() != images.shape[0] * blk.shape[0]:
-            work = torch.empty(images.shape[0] * blk.shape[0], device=images.device,
-                               dtype=torch.float64)
-        t.update_fp64(images, blk, st, work)
+        t.update_fp64(images, refs[st:st + batch], st)
     return t.result()
 
 

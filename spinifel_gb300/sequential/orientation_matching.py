@@ -94,14 +94,12 @@ class SNM:
         B = self.N_batch_size
         if self.fp64:
             buf = torch.empty(B, self.N_pixels, device=self.slices_.device, dtype=torch.float64)
-            work = torch.empty(self.N_slices * B, device=self.slices_.device,
-                               dtype=torch.float64)
             best = matching.BestTracker64(self.N_slices, self.slices_.device)
             for i in range(self.N_orientations // B):
                 st = i * B
                 self.nufft.slice_real(P, st, st + B, out=buf)
                 buf *= self.slices_std / buf.std(unbiased=False)
-                best.update_fp64(self.slices_, buf, st, work)
+                best.update_fp64(self.slices_, buf, st)
             idx, _ = best.result()
             return idx
         buf = torch.empty(B, self.N_pixels, device=self.slices_.device, dtype=torch.float32)

@@ -106,3 +106,54 @@ def test_distance_tiles(n_img, n_ref, n_pix):
     rows = torch.arange(n_img, device="cuda")
     assert bool((dist.double() - want[rows, i]).abs().le(err[rows, i]).all())
     assert bool((want[rows, i] - best).le(2 * err.max(dim=1).values).all())
+
+
+def _minima_case(kind, n_img, n_ref, n_pix):
+    rng = np.random.default_rng(n_img + n_ref + n_pix)
+    r = rng.gamma(2.0, 1.0, (n_ref, n_pix))
+    x = rng.poisson(r[rng.integers(0, n_ref, n_img)]).astype(np.float64)
+    if kind == "ties":            # every reference several times over
+        r = r[rng.integers(0, max(1, n_ref // 5), n_ref)]
+    elif kind == "equal":         # no list: all references tie
+        r[:] = r[0]
+    elif kind == "exact":         # frames that are references
+        x = r[rng.integers(0, n_ref, n_img)].copy()
+    elif kind == "close":         # apart by less than FP32 resolves
+        r = r[:1] * (1 + 1e-12 * rng.standard_normal((n_ref, n_pix)))
+    elif kind == "signed":
+        x, r = rng.standard_normal((n_img, n_pix)), rng.standard_normal((n_ref, n_pix))
+    elif kind == "tiny":
+        x, r = x * 1e-25, r * 1e-25
+    elif kind == "huge":
+        r[::3] *= 1e20
+    elif kind == "overflow":
+        x, r = x * 1e200, r * 1e200
+    elif kind == "zero":
+        x[:] = 0.0
+        r[0] = 0.0
+    elif kind == "nan":
+        r[::2, n_pix // 2] = np.nan
+        x[0, 0] = np.inf
+        if n_img > 1:
+            x[1, n_pix - 1] = np.nan
+    return x, r
+
+
+@pytest.mark.parametrize("kind", ["plain", "ties", "equal", "exact", "close", "signed", "tiny",
+                                  "huge", "overflow", "zero", "nan"])
+@pytest.mark.parametrize("n_img,n_ref,n_pix", [(1, 1, 64), (33, 65, 257), (5, 700, 1025),
+                                               (130, 1100, 130), (40, 300, 5000)])
+def test_minima_equal_full_fp64_block(kind, n_img, n_ref, n_pix):
+    """Picking minima gives the indices and distances of the whole FP64 block,
+    bit for bit, in one batch and in several, whatever the values."""
+    from spinifel_gb300 import matching
+
+    x, r = _minima_case(kind, n_img, n_ref, n_pix)
+    x, r = torch.as_tensor(x, device="cuda"), torch.as_tensor(r, device="cuda")
+    for batch in (4096, (n_ref + 2) // 3):
+        full = matching.BestTracker64(n_img, x.device)
+        for st in range(0, n_ref, batch):
+            full.update_block(matching.dist_f64(r[st:st + batch], x), st)
+        idx, dist = matching.argmin_fp64(x, r, batch=batch)
+        assert torch.equal(idx, full.best_idx)
+        assert torch.equal(dist, full.best_dist)
