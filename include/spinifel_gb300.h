@@ -70,8 +70,8 @@ int spf_selftest_bounded_wait(int64_t timeout_ms, int *d_result, void *stream);
  *                           shape gives the same bits
  *   SPF_TUNE_SORT_ITEM    : points per work item of the bin-sorted passes
  *                           (read by spf_nufft_sort_orient /
- *                           spf_nufft_sort_points; default 2048,
- *                           256 .. 8192)
+ *                           spf_nufft_sort_points; default 2048, 1024
+ *                           below 2^22 points; 256 .. 8192)
  *   SPF_TUNE_STATIC_ABORT_TEST : 1 makes spf_match_bf16_static record a
  *                           given-up GEMM wait (SPF_ERR_TIMEOUT in its
  *                           error word, after the GEMM) so that tests can

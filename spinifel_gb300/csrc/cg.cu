@@ -645,6 +645,7 @@ int spf_merge_set_direct(spf_merge_s *G, spf_nufft_plan_s *plan, const float *d_
   // the points are fixed for the solve: sort them by fine-grid bin once
   G->sorted = false;
   SPF_TRY(spf_nufft_sort_orient(plan, d_quats, n_orient, d_ppr, n_pix, coord_scale, nullptr));
+  SPF_TRY(spf::check_cuda(cudaStreamSynchronize(nullptr), "spf_merge_set_direct"));
   G->sorted = true;
   return SPF_OK;
 }

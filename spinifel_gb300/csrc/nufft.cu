@@ -36,15 +36,13 @@ struct spf_nufft_plan_s {
   float *acc_pad = nullptr;
   cufftHandle fft = 0;
   bool fft_ok = false;
-  // bin-sorted orientation points (spf_nufft_sort_orient)
-  int32_t *sorted = nullptr;   // point indices o * n_pix + p, grouped by bin
-  int4 *items = nullptr;       // (bin, start, count, 0) work items
-  int64_t n_items = 0, n_sorted = 0, sorted_cap = 0, items_cap = 0;
+  // bin-sorted points (spf_nufft_sort_orient / _points)
+  float4 *sorted = nullptr;  // wrapped grid coordinates t1, t2, t3 and the point's index
+                             // (o * n_pix + p), grouped by bin
+  int4 *items = nullptr;     // (bin, start, count, 0) work items, their number in bins
+  int32_t *bins = nullptr;   // per bin: points, then next free place; the two totals
+  int64_t n_sorted = 0, max_items = 0, sorted_cap = 0, items_cap = 0;
   int nb[3] = {0, 0, 0};
-  const float *s_quats = nullptr, *s_ppr = nullptr;
-  const float *s_x = nullptr, *s_y = nullptr, *s_z = nullptr;  // explicit points instead
-  int64_t s_n_orient = 0, s_n_pix = 0;
-  double s_scale = 0;
 };
 
 namespace spf {
@@ -825,9 +823,13 @@ __global__ void k_interp_spread_orient(const float *__restrict__ re_pad,
 // ---------------------------------------------------------------------------
 constexpr int BIN = 8;
 constexpr int BIN_CHUNK = 2048;      // default points per work item (big bins are split)
+// below this many points items of half the size: too few to fill the chip's
+// 900 CTAs evenly otherwise (2.0e6 points at 41^3: 222 against 238 us; at
+// 8.2e6 736 against 680)
+constexpr int64_t BIN_CHUNK_FEW = 1 << 22;
 constexpr int BIN_CHUNK_MAX = 8192;  // largest item SPF_TUNE_SORT_ITEM may pick: the cell
-                                     // sort stages an item in 48 KB of dynamic shared memory
-constexpr size_t CELLSORT_SMEM = (size_t)BIN_CHUNK_MAX * (sizeof(int32_t) + sizeof(int16_t));
+                                     // sort stages an item in dynamic shared memory
+constexpr size_t CELLSORT_POINT = sizeof(float4) + sizeof(int16_t);
 
 // The points of the sorted passes: orientation points (point o * n_pix + p
 // is pixel p of the detector rotated by quaternion o, coordinates made in the
@@ -848,112 +850,147 @@ struct PointSrc {
   }
 };
 
-template <int W>
-__device__ __forceinline__ int point_bin(const GridGeom &g, const int *nb, float h, float k, float l,
-                                         float s1, float s2, float s3) {
-  float w[W];
-  int i0 = axis_setup<W>(h, s1, g.n1, g.off1, g.beta, g.inv_half_w, w);
-  int j0 = axis_setup<W>(k, s2, g.n2, g.off2, g.beta, g.inv_half_w, w);
-  int k0 = axis_setup<W>(l, s3, g.n3, g.off3, g.beta, g.inv_half_w, w);
-  return ((i0 / BIN) * nb[1] + (j0 / BIN)) * nb[2] + (k0 / BIN);
-}
-
 struct BinDims {
   int nb[3];
 };
 
+// Wrapped grid coordinate t of x along one axis and its padded first footprint
+// index: the index arithmetic of axis_setup without the weights (the same
+// explicitly rounded operations, so every kernel agrees on the cell).
 template <int W>
-__global__ void k_bin_count(GridGeom g, BinDims bd, PointSrc src, int64_t n, float s1, float s2,
-                            float s3, int32_t *__restrict__ bin_of, int32_t *__restrict__ counts) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    float h, k, l;
-    src.coords(i, h, k, l);
-    int b = point_bin<W>(g, bd.nb, h, k, l, s1, s2, s3);
-    bin_of[i] = b;
-    atomicAdd(counts + b, 1);
-  }
-}
-
-// exclusive prefix sum of n ints, one block of 1024 threads
-__global__ void __launch_bounds__(1024) k_scan(const int32_t *__restrict__ in, int64_t n,
-                                               int32_t *__restrict__ out) {
-  __shared__ int32_t part[1024];
-  const int t = threadIdx.x;
-  const int64_t per = (n + 1023) / 1024;
-  const int64_t lo = t * per, hi = lo + per < n ? lo + per : n;
-  int32_t s = 0;
-  for (int64_t i = lo; i < hi; ++i) s += in[i];
-  part[t] = s;
-  __syncthreads();
-  for (int off = 1; off < 1024; off <<= 1) {
-    int32_t v = t >= off ? part[t - off] : 0;
-    __syncthreads();
-    part[t] += v;
-    __syncthreads();
-  }
-  int32_t run = t > 0 ? part[t - 1] : 0;
-  for (int64_t i = lo; i < hi; ++i) {
-    out[i] = run;
-    run += in[i];
-  }
-}
-
-__global__ void k_bin_scatter(const int32_t *__restrict__ bin_of, int64_t n,
-                              const int32_t *__restrict__ offsets, int32_t *__restrict__ cursor,
-                              int32_t *__restrict__ sorted) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    int b = bin_of[i];
-    int pos = atomicAdd(cursor + b, 1);
-    sorted[offsets[b] + pos] = (int32_t)i;
-  }
-}
-
-// Padded first footprint index of a point along one axis: the index
-// arithmetic of axis_setup without the weights (same explicitly rounded
-// operations, so the cell agrees with the one the kernels use).
-template <int W>
-__device__ __forceinline__ int axis_cell(float x, float s, int n, int off) {
-  float fn = (float)n;
-  float t = __fmul_rn(x, s);
+__device__ __forceinline__ int axis_cell(float x, float s, int n, int off, float &t) {
+  const float fn = (float)n;
+  t = __fmul_rn(x, s);
   t = __fsub_rn(t, __fmul_rn(fn, floorf(__fadd_rn(__fdiv_rn(t, fn), 0.5f))));
   return (int)ceilf(__fsub_rn(t, 0.5f * W)) + off;
+}
+
+// The sort, all on the device (sizes stay there, nothing is read back): count
+// the points of each bin; give each bin a range of the sorted array and work
+// items for it (bins in any order: the ranges come from one counter); move
+// every point, as its three grid coordinates and its index, to its bin's
+// range; order each item by footprint cell.  Later passes then read 16
+// contiguous bytes a point instead of gathering three coordinates and
+// recomputing the cell.  Neighbouring points are often in one bin, so a
+// warp's points of a bin take one atomic.  With a scan in one block, items
+// made on the host and temporaries allocated on every call the sort's kernels
+// took 620 us for 1.3e7 points on the 320^3 grid and 465 us for 2.0e6 on 90^3,
+// where most points fall in few bins, and the host added some 300 us; the
+// kernels take 305 and 115 us now and the host adds nothing.
+
+// bin of point i; its coordinates in t
+template <int W>
+__device__ __forceinline__ int point_bin(const GridGeom &g, const BinDims &bd, const PointSrc &src,
+                                         int64_t i, float s1, float s2, float s3, float3 &t) {
+  float h, k, l;
+  src.coords(i, h, k, l);
+  const int i0 = axis_cell<W>(h, s1, g.n1, g.off1, t.x);
+  const int j0 = axis_cell<W>(k, s2, g.n2, g.off2, t.y);
+  const int k0 = axis_cell<W>(l, s3, g.n3, g.off3, t.z);
+  // clamped: a coordinate too large to wrap in FP32 has no cell, and the
+  // passes leave its point out
+  const int b1 = min(max(i0 / BIN, 0), bd.nb[0] - 1), b2 = min(max(j0 / BIN, 0), bd.nb[1] - 1),
+            b3 = min(max(k0 / BIN, 0), bd.nb[2] - 1);
+  return (b1 * bd.nb[1] + b2) * bd.nb[2] + b3;
+}
+
+template <int W>
+__global__ void __launch_bounds__(256)
+    k_bin_count(GridGeom g, BinDims bd, PointSrc src, int64_t n, float s1, float s2, float s3,
+                int32_t *__restrict__ counts) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x; i0 < n;
+       i0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = i0 + threadIdx.x;
+    float3 t;
+    const int b = i < n ? point_bin<W>(g, bd, src, i, s1, s2, s3, t) : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, b);
+    if (b >= 0 && lane == __ffs(same) - 1) atomicAdd(counts + b, __popc(same));
+  }
+}
+
+// next[b] = first place of bin b in the sorted array, and its work items of
+// at most chunk points; totals[0] / [1] count the places and items taken
+__global__ void __launch_bounds__(256)
+    k_bin_items(const int32_t *__restrict__ counts, int n_bins, int chunk,
+                int32_t *__restrict__ next, int32_t *__restrict__ totals,
+                int4 *__restrict__ items) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  const int c = b < n_bins ? counts[b] : 0;
+  const int ni = (c + chunk - 1) / chunk;
+  int pc = c, pi = ni;  // inclusive sums over the warp
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int vc = __shfl_up_sync(0xffffffffu, pc, o), vi = __shfl_up_sync(0xffffffffu, pi, o);
+    if (lane >= o) {
+      pc += vc;
+      pi += vi;
+    }
+  }
+  int bc = 0, bi = 0;
+  if (lane == 31 && pi > 0) {
+    bc = atomicAdd(totals, pc);
+    bi = atomicAdd(totals + 1, pi);
+  }
+  bc = __shfl_sync(0xffffffffu, bc, 31) + pc - c;
+  bi = __shfl_sync(0xffffffffu, bi, 31) + pi - ni;
+  if (b < n_bins) next[b] = bc;
+  for (int q = 0; q < ni; ++q)
+    items[bi + q] = make_int4(b, bc + q * chunk, min(chunk, c - q * chunk), 0);
+}
+
+template <int W>
+__global__ void __launch_bounds__(256)
+    k_bin_scatter(GridGeom g, BinDims bd, PointSrc src, int64_t n, float s1, float s2, float s3,
+                  int32_t *__restrict__ next, float4 *__restrict__ sorted) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x; i0 < n;
+       i0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = i0 + threadIdx.x;
+    float3 t;
+    const int b = i < n ? point_bin<W>(g, bd, src, i, s1, s2, s3, t) : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, b);
+    const int leader = __ffs(same) - 1;
+    int at = 0;
+    if (b >= 0 && lane == leader) at = atomicAdd(next + b, __popc(same));
+    at = __shfl_sync(0xffffffffu, at, leader) + __popc(same & ((1u << lane) - 1));
+    if (b >= 0) sorted[at] = make_float4(t.x, t.y, t.z, __int_as_float((int)i));
+  }
+}
+
+// first footprint cell of a sorted point, relative to its bin
+template <int W>
+__device__ __forceinline__ int cell_in_bin(float t, int off, int b0) {
+  return (int)ceilf(__fsub_rn(t, 0.5f * W)) + off - b0;
 }
 
 // Orders the points of each work item by their first footprint cell within
 // the bin (a counting sort over the 8^3 cells in shared memory), so that
 // points sharing a footprint are consecutive.  The point set of every item is
-// unchanged; only its order within the item is.
+// unchanged; only its order within the item is.  Dynamic shared memory: the
+// item's points and keys, chunk * 18 bytes.
 template <int W>
 __global__ void __launch_bounds__(256)
     k_item_cellsort(GridGeom g, BinDims bd, const int4 *__restrict__ items,
-                    int32_t *__restrict__ sorted, PointSrc src, float s1, float s2, float s3,
-                    unsigned int *__restrict__ err) {
+                    const int32_t *__restrict__ n_items, float4 *__restrict__ sorted, int chunk) {
   constexpr int NC = BIN * BIN * BIN;
-  extern __shared__ __align__(16) unsigned char cs_smem[];  // CELLSORT_SMEM bytes
-  int32_t *idx = reinterpret_cast<int32_t *>(cs_smem);              // BIN_CHUNK_MAX
-  int16_t *key = reinterpret_cast<int16_t *>(idx + BIN_CHUNK_MAX);  // BIN_CHUNK_MAX
+  extern __shared__ __align__(16) unsigned char cs_smem[];
+  float4 *pt = reinterpret_cast<float4 *>(cs_smem);
+  int16_t *key = reinterpret_cast<int16_t *>(pt + chunk);
   __shared__ int32_t cnt[NC];
+  if ((int)blockIdx.x >= *n_items) return;
   const int4 it = items[blockIdx.x];
-  if (it.z > BIN_CHUNK_MAX) {  // an item larger than the staging arrays is never read
-    if (threadIdx.x == 0 && err) atomicExch(err, (unsigned int)(-SPF_ERR_ARG));
-    return;
-  }
   const int b = it.x;
   const int bi = b / (bd.nb[1] * bd.nb[2]), bj = (b / bd.nb[2]) % bd.nb[1], bk = b % bd.nb[2];
-  const int i0b = bi * BIN, j0b = bj * BIN, k0b = bk * BIN;
   for (int t = threadIdx.x; t < NC; t += blockDim.x) cnt[t] = 0;
   __syncthreads();
   for (int q = threadIdx.x; q < it.z; q += blockDim.x) {
-    const int32_t pi = sorted[it.y + q];
-    float h, k, l;
-    src.coords(pi, h, k, l);
-    const int ci = min(max(axis_cell<W>(h, s1, g.n1, g.off1) - i0b, 0), BIN - 1);
-    const int cj = min(max(axis_cell<W>(k, s2, g.n2, g.off2) - j0b, 0), BIN - 1);
-    const int ck = min(max(axis_cell<W>(l, s3, g.n3, g.off3) - k0b, 0), BIN - 1);
+    const float4 v = sorted[it.y + q];
+    const int ci = min(max(cell_in_bin<W>(v.x, g.off1, bi * BIN), 0), BIN - 1);
+    const int cj = min(max(cell_in_bin<W>(v.y, g.off2, bj * BIN), 0), BIN - 1);
+    const int ck = min(max(cell_in_bin<W>(v.z, g.off3, bk * BIN), 0), BIN - 1);
     const int kk = (ci * BIN + cj) * BIN + ck;
-    idx[q] = pi;
+    pt[q] = v;
     key[q] = (int16_t)kk;
     atomicAdd(&cnt[kk], 1);
   }
@@ -979,10 +1016,8 @@ __global__ void __launch_bounds__(256)
     }
   }
   __syncthreads();
-  for (int q = threadIdx.x; q < it.z; q += blockDim.x) {
-    const int pos = atomicAdd(&cnt[key[q]], 1);
-    sorted[it.y + pos] = idx[q];
-  }
+  for (int q = threadIdx.x; q < it.z; q += blockDim.x)
+    sorted[it.y + atomicAdd(&cnt[key[q]], 1)] = pt[q];
 }
 
 // Fused type 2 -> weight -> type 1 over bin-sorted points.  A CTA takes one
@@ -998,8 +1033,8 @@ __global__ void __launch_bounds__(256)
 // spread box (shared atomics), only when the cell changes.  The separable
 // weights are shuffled in once per point (w1 for the plane, w2 * w3 for the
 // lane's two rows).  With a row stride of 24 floats the 32 lanes of either
-// row set fall on 32 distinct banks.  Each point's coordinates are computed
-// once by one lane and broadcast; lanes 0-7 / 8-15 / 16-23 evaluate the
+// row set fall on 32 distinct banks.  Each point's slot is
+// prepared once by one lane; lanes 0-7 / 8-15 / 16-23 evaluate the
 // kernel on axes 1 / 2 / 3.
 constexpr int SORTED_ROW_STRIDE = 24;
 constexpr int SORTED_THREADS = 256;
@@ -1008,8 +1043,8 @@ template <int W>
 __global__ void __launch_bounds__(SORTED_THREADS, 4)
     k_interp_spread_sorted(const float *__restrict__ re_pad, float *__restrict__ acc_pad,
                            GridGeom g, BinDims bd, const int4 *__restrict__ items,
-                           const int32_t *__restrict__ sorted, PointSrc src, float s1, float s2,
-                           float s3, const float *__restrict__ weights,
+                           const int32_t *__restrict__ n_items,
+                           const float4 *__restrict__ sorted, const float *__restrict__ weights,
                            const __grid_constant__ CUtensorMap tmap, int use_tma,
                            unsigned int *__restrict__ err) {
   static_assert(W <= 8, "eight lanes per footprint row, two rows per lane");
@@ -1022,6 +1057,7 @@ __global__ void __launch_bounds__(SORTED_THREADS, 4)
   __shared__ float abox[D * SP];
   __shared__ float4 pt_tw[SORTED_THREADS];  // per warp: 32 prepared points
   __shared__ int pt_key[SORTED_THREADS];
+  if ((int)blockIdx.x >= *n_items) return;
   const int4 it = items[blockIdx.x];
   const int b = it.x;
   const int bi = b / (bd.nb[1] * bd.nb[2]), bj = (b / bd.nb[2]) % bd.nb[1], bk = b % bd.nb[2];
@@ -1082,26 +1118,20 @@ __global__ void __launch_bounds__(SORTED_THREADS, 4)
   const int ax_shift = 10 - 5 * ax;
   const int ax_base = ax == 0 ? i0b - g.off1 : (ax == 1 ? j0b - g.off2 : k0b - g.off3);
   const float beta_log2e = g.beta * 1.4426950408889634f;
-  const float fn1 = (float)g.n1, fn2 = (float)g.n2, fn3 = (float)g.n3;
   float4 *my_tw = pt_tw + warp * 32;
   int *my_key = pt_key + warp * 32;
   for (int q0 = warp * 32; q0 < it.z; q0 += nwarps * 32) {
     const int cnt = min(32, it.z - q0);
-    // lane L prepares point q0 + L (same arithmetic as axis_setup / the bin sort)
+    // lane L prepares point q0 + L
     // into the warp's slots: (t1, t2, t3, weight) and the packed first cell
     // in the box, or -1 for a point outside the box
     if (lane < cnt) {
-      const int32_t pi = sorted[it.y + q0 + lane];
-      const float pw = weights ? weights[pi] : 1.0f;
-      float h, k, l;
-      src.coords(pi, h, k, l);
-      float t1 = __fmul_rn(h, s1), t2 = __fmul_rn(k, s2), t3 = __fmul_rn(l, s3);
-      t1 = __fsub_rn(t1, __fmul_rn(fn1, floorf(__fadd_rn(__fdiv_rn(t1, fn1), 0.5f))));
-      t2 = __fsub_rn(t2, __fmul_rn(fn2, floorf(__fadd_rn(__fdiv_rn(t2, fn2), 0.5f))));
-      t3 = __fsub_rn(t3, __fmul_rn(fn3, floorf(__fadd_rn(__fdiv_rn(t3, fn3), 0.5f))));
-      const int li = (int)ceilf(__fsub_rn(t1, 0.5f * W)) + g.off1 - i0b;
-      const int lj = (int)ceilf(__fsub_rn(t2, 0.5f * W)) + g.off2 - j0b;
-      const int lk = (int)ceilf(__fsub_rn(t3, 0.5f * W)) + g.off3 - k0b;
+      const float4 v = sorted[it.y + q0 + lane];
+      const float t1 = v.x, t2 = v.y, t3 = v.z;
+      const float pw = weights ? weights[__float_as_int(v.w)] : 1.0f;
+      const int li = cell_in_bin<W>(t1, g.off1, i0b);
+      const int lj = cell_in_bin<W>(t2, g.off2, j0b);
+      const int lk = cell_in_bin<W>(t3, g.off3, k0b);
       const bool inside =
           li >= 0 && lj >= 0 && lk >= 0 && li + W <= di && lj + W <= dj && lk + W <= dk;
       if (!inside && err)  // cannot happen for a correctly binned point; never read outside
@@ -1171,7 +1201,7 @@ __global__ void __launch_bounds__(SORTED_THREADS, 4)
 // Adding each run of equal cells (14 shared float atomics, 0.30 a clock and
 // SM, at about every point when points are sparse) took 2,887 us for 1.3e7
 // points on the 320^3 grid (0.8 a cell) and 9,368 us for 6.6e7; this takes
-// 1,547 and 5,658.  Four warps an item: sparse bins hold some 400 points.
+// 1,530 and 5,470.  Four warps an item: sparse bins hold some 400 points.
 // Lane j of a warp evaluates the 3 W kernel values of the j-th of 32 points.
 constexpr int PEN_WORDS = 28;  // a point's slot: w1 c[8], w2[8], w3[8], cell, 3 unused;
                                // seven 16-byte quads, so 8 lanes' quads share no bank
@@ -1181,8 +1211,8 @@ constexpr int PEN_THREADS = 128;
 template <int W>
 __global__ void __launch_bounds__(PEN_THREADS, 6)
     k_spread_sorted(float *__restrict__ acc_pad, GridGeom g, BinDims bd,
-                    const int4 *__restrict__ items, const int32_t *__restrict__ sorted,
-                    PointSrc src, float s1, float s2, float s3, const float *__restrict__ values,
+                    const int4 *__restrict__ items, const int32_t *__restrict__ n_items,
+                    const float4 *__restrict__ sorted, const float *__restrict__ values,
                     unsigned int *__restrict__ err) {
   static_assert(W <= 8, "four planes a half-warp, eight rows a plane");
   constexpr int D = BIN + W - 1;
@@ -1191,6 +1221,7 @@ __global__ void __launch_bounds__(PEN_THREADS, 6)
   constexpr int SP = D * PEN_ROW + 4;
   __shared__ float abox[D * SP];
   __shared__ __align__(16) float slots[PEN_THREADS / 32][32 * PEN_WORDS];
+  if ((int)blockIdx.x >= *n_items) return;
   const int4 it = items[blockIdx.x];
   const int b = it.x;
   const int bi = b / (bd.nb[1] * bd.nb[2]), bj = (b / bd.nb[2]) % bd.nb[1], bk = b % bd.nb[2];
@@ -1202,7 +1233,6 @@ __global__ void __launch_bounds__(PEN_THREADS, 6)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int h = lane >> 4, k = lane & 15;
   const float beta_log2e = g.beta * 1.4426950408889634f;
-  const float fn1 = (float)g.n1, fn2 = (float)g.n2, fn3 = (float)g.n3;
   float *my = slots[warp];
   float acc[4][W];
 #pragma unroll
@@ -1225,14 +1255,9 @@ __global__ void __launch_bounds__(PEN_THREADS, 6)
   for (int q0 = lo; q0 < hi; q0 += 32) {
     const int cnt = min(32, hi - q0);
     if (lane < cnt) {
-      const int32_t pi = sorted[it.y + q0 + lane];
-      const float c = values ? values[pi] : 1.0f;
-      float x, y, z;
-      src.coords(pi, x, y, z);
-      float t1 = __fmul_rn(x, s1), t2 = __fmul_rn(y, s2), t3 = __fmul_rn(z, s3);
-      t1 = __fsub_rn(t1, __fmul_rn(fn1, floorf(__fadd_rn(__fdiv_rn(t1, fn1), 0.5f))));
-      t2 = __fsub_rn(t2, __fmul_rn(fn2, floorf(__fadd_rn(__fdiv_rn(t2, fn2), 0.5f))));
-      t3 = __fsub_rn(t3, __fmul_rn(fn3, floorf(__fadd_rn(__fdiv_rn(t3, fn3), 0.5f))));
+      const float4 v = sorted[it.y + q0 + lane];
+      const float t1 = v.x, t2 = v.y, t3 = v.z;
+      const float c = values ? values[__float_as_int(v.w)] : 1.0f;
       const float l1 = ceilf(__fsub_rn(t1, 0.5f * W)), l2 = ceilf(__fsub_rn(t2, 0.5f * W)),
                   l3 = ceilf(__fsub_rn(t3, 0.5f * W));
       const int li = (int)l1 + g.off1 - i0b, lj = (int)l2 + g.off2 - j0b,
@@ -1479,6 +1504,7 @@ int spf_nufft_plan_destroy(spf_nufft_plan P) {
   cudaFree(P->acc_pad);
   cudaFree(P->sorted);
   cudaFree(P->items);
+  cudaFree(P->bins);
   if (P->fft_ok) cufftDestroy(P->fft);
   if (prev != P->dev && prev >= 0) cudaSetDevice(prev);
   delete P;
@@ -1700,83 +1726,51 @@ static int sort_points(spf_nufft_plan P, PointSrc src, int64_t n, double scale, 
   float s1 = (float)(scale * P->n[0] / (2.0 * M_PI));
   float s2 = (float)(scale * P->n[1] / (2.0 * M_PI));
   float s3 = (float)(scale * P->n[2] / (2.0 * M_PI));
-  // temporaries
-  int32_t *bin_of = nullptr, *counts = nullptr, *offsets = nullptr, *cursor = nullptr;
-  int st = check_cuda(cudaMalloc(&bin_of, (n > 0 ? n : 1) * sizeof(int32_t)), "sort_orient");
-  if (st == SPF_OK) st = check_cuda(cudaMalloc(&counts, n_bins * 3 * sizeof(int32_t)), "sort_orient");
-  if (st == SPF_OK && n > P->sorted_cap) {
+  int32_t chunk = (int32_t)tune_get(SPF_TUNE_SORT_ITEM, 0);
+  if (chunk < 1 || chunk > BIN_CHUNK_MAX)  // (the cell sort stages <= the max)
+    chunk = n < BIN_CHUNK_FEW ? BIN_CHUNK / 2 : BIN_CHUNK;
+  // items: one per non-empty bin and one more per full chunk at most
+  const int64_t max_items = (n < n_bins ? n : n_bins) + n / chunk;
+  P->n_sorted = 0;
+  if (!P->bins)
+    SPF_TRY(check_cuda(cudaMalloc(&P->bins, (2 * n_bins + 2) * sizeof(int32_t)), "spf_nufft_sort"));
+  if (n > P->sorted_cap) {
     cudaFree(P->sorted);
     P->sorted = nullptr;
-    st = check_cuda(cudaMalloc(&P->sorted, n * sizeof(int32_t)), "sort_orient");
-    if (st == SPF_OK) P->sorted_cap = n;
+    P->sorted_cap = 0;
+    SPF_TRY(check_cuda(cudaMalloc(&P->sorted, n * sizeof(float4)), "spf_nufft_sort"));
+    P->sorted_cap = n;
   }
-  if (st == SPF_OK) {
-    offsets = counts + n_bins;
-    cursor = counts + 2 * n_bins;
-    cudaMemsetAsync(counts, 0, n_bins * 3 * sizeof(int32_t), s);
-    int grid = grid_for(n, 256, (int64_t)sm_count() * 16);
-    SPF_W_DISPATCH(P->w, (k_bin_count<W><<<grid, 256, 0, s>>>(g, bd, src, n, s1, s2, s3, bin_of,
-                                                                 counts)));
-    st = check_launch("k_bin_count");
-  }
-  if (st == SPF_OK) {
-    k_scan<<<1, 1024, 0, s>>>(counts, n_bins, offsets);
-    st = check_launch("k_scan");
-  }
-  if (st == SPF_OK) {
-    k_bin_scatter<<<grid_for(n, 256, (int64_t)sm_count() * 16), 256, 0, s>>>(bin_of, n, offsets,
-                                                                            cursor, P->sorted);
-    st = check_launch("k_bin_scatter");
-  }
-  // work items: every non-empty bin, big bins split into BIN_CHUNK points
-  std::vector<int32_t> h_counts, h_offsets;
-  if (st == SPF_OK) {
-    h_counts.resize(n_bins);
-    h_offsets.resize(n_bins);
-    st = check_cuda(cudaMemcpyAsync(h_counts.data(), counts, n_bins * sizeof(int32_t),
-                                    cudaMemcpyDeviceToHost, s), "sort_orient");
-    if (st == SPF_OK)
-      st = check_cuda(cudaMemcpyAsync(h_offsets.data(), offsets, n_bins * sizeof(int32_t),
-                                      cudaMemcpyDeviceToHost, s), "sort_orient");
-    if (st == SPF_OK) st = check_cuda(cudaStreamSynchronize(s), "sort_orient");
-  }
-  cudaFree(bin_of);
-  cudaFree(counts);
-  if (st != SPF_OK) return st;
-  std::vector<int4> h_items;
-  int32_t chunk = (int32_t)tune_get(SPF_TUNE_SORT_ITEM, BIN_CHUNK);
-  if (chunk < 1 || chunk > BIN_CHUNK_MAX) chunk = BIN_CHUNK;  // the cell sort stages <= the max
-  for (int64_t b = 0; b < n_bins; ++b)
-    for (int32_t c = 0; c < h_counts[b]; c += chunk)
-      h_items.push_back(make_int4((int)b, h_offsets[b] + c,
-                                  h_counts[b] - c < chunk ? h_counts[b] - c : chunk, 0));
-  if ((int64_t)h_items.size() > P->items_cap) {
+  if (max_items > P->items_cap) {
     cudaFree(P->items);
     P->items = nullptr;
-    SPF_TRY(check_cuda(cudaMalloc(&P->items, (h_items.size() + 1) * sizeof(int4)), "sort_orient"));
-    P->items_cap = (int64_t)h_items.size();
+    P->items_cap = 0;
+    SPF_TRY(check_cuda(cudaMalloc(&P->items, max_items * sizeof(int4)), "spf_nufft_sort"));
+    P->items_cap = max_items;
   }
-  if (!h_items.empty())
-    SPF_TRY(check_cuda(cudaMemcpy(P->items, h_items.data(), h_items.size() * sizeof(int4),
-                                  cudaMemcpyHostToDevice), "sort_orient"));
-  P->n_items = (int64_t)h_items.size();
+  P->max_items = max_items;
+  if (n == 0) return SPF_OK;
+  int32_t *next = P->bins + n_bins, *totals = P->bins + 2 * n_bins;
+  SPF_TRY(check_cuda(cudaMemsetAsync(P->bins, 0, (2 * n_bins + 2) * sizeof(int32_t), s),
+                     "spf_nufft_sort"));
+  const int grid = grid_for(n, 256, (int64_t)sm_count() * 16);
+  SPF_W_DISPATCH(P->w, (k_bin_count<W><<<grid, 256, 0, s>>>(g, bd, src, n, s1, s2, s3, P->bins)));
+  SPF_TRY(check_launch("k_bin_count"));
+  k_bin_items<<<grid_for(n_bins, 256), 256, 0, s>>>(P->bins, (int)n_bins, chunk, next, totals,
+                                                    P->items);
+  SPF_TRY(check_launch("k_bin_items"));
+  SPF_W_DISPATCH(P->w, (k_bin_scatter<W><<<grid, 256, 0, s>>>(g, bd, src, n, s1, s2, s3, next,
+                                                              P->sorted)));
+  SPF_TRY(check_launch("k_bin_scatter"));
+  // points sharing a footprint cell become consecutive
+  const int smem = (int)(CELLSORT_POINT * chunk);
+  SPF_W_DISPATCH(P->w, (cudaFuncSetAttribute(k_item_cellsort<W>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(CELLSORT_POINT * BIN_CHUNK_MAX)),
+                        k_item_cellsort<W><<<(unsigned)max_items, 256, smem, s>>>(
+                            g, bd, P->items, totals + 1, P->sorted, chunk)));
+  SPF_TRY(check_launch("k_item_cellsort"));
   P->n_sorted = n;
-  if (P->n_items > 0) {  // points sharing a footprint cell become consecutive
-    SPF_W_DISPATCH(P->w, (cudaFuncSetAttribute(k_item_cellsort<W>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)CELLSORT_SMEM),
-                          k_item_cellsort<W><<<(unsigned)P->n_items, 256, CELLSORT_SMEM, s>>>(
-                             g, bd, P->items, P->sorted, src, s1, s2, s3,
-                             device_error_word())));
-    SPF_TRY(check_launch("k_item_cellsort"));
-  }
-  P->s_quats = src.quats;
-  P->s_ppr = src.ppr;
-  P->s_n_pix = src.n_pix;
-  P->s_x = src.x;
-  P->s_y = src.y;
-  P->s_z = src.z;
-  P->s_scale = scale;
   return SPF_OK;
 }
 
@@ -1786,10 +1780,9 @@ int spf_nufft_sort_orient(spf_nufft_plan P, const float *d_quats, int64_t n_orie
   SPF_REQUIRE(n_orient >= 0 && n_pix >= 0, "spf_nufft_sort_orient: negative size");
   SPF_REQUIRE(d_quats && d_ppr, "spf_nufft_sort_orient: NULL pointer");
   SPF_REQUIRE(n_pix > 0 || n_orient == 0, "spf_nufft_sort_orient: n_pix = 0");
-  SPF_TRY(sort_points(P, PointSrc{d_quats, d_ppr, n_pix > 0 ? n_pix : 1, nullptr, nullptr, nullptr},
-                      n_orient * n_pix, scale, stream));
-  P->s_n_orient = n_orient;
-  return SPF_OK;
+  return sort_points(P,
+                     PointSrc{d_quats, d_ppr, n_pix > 0 ? n_pix : 1, nullptr, nullptr, nullptr},
+                     n_orient * n_pix, scale, stream);
 }
 
 int spf_nufft_sort_points(spf_nufft_plan P, const float *d_x, const float *d_y,
@@ -1797,26 +1790,19 @@ int spf_nufft_sort_points(spf_nufft_plan P, const float *d_x, const float *d_y,
   SPF_TRY(check_plan(P, "spf_nufft_sort_points"));
   SPF_REQUIRE(n >= 0, "spf_nufft_sort_points: negative size");
   SPF_REQUIRE(n == 0 || (d_x && d_y && d_z), "spf_nufft_sort_points: NULL pointer");
-  SPF_TRY(sort_points(P, PointSrc{nullptr, nullptr, 1, d_x, d_y, d_z}, n, 1.0, stream));
-  P->s_n_orient = 0;
-  return SPF_OK;
+  return sort_points(P, PointSrc{nullptr, nullptr, 1, d_x, d_y, d_z}, n, 1.0, stream);
 }
 
 static int sorted_pass(spf_nufft_plan P, const float *d_weights, bool interp, const char *what,
                        void *stream) {
   SPF_TRY(check_plan(P, what));
-  SPF_REQUIRE(P->sorted != nullptr && P->n_sorted > 0 || P->n_items == 0,
-              "%s: call spf_nufft_sort_orient first", what);
-  if (P->n_items == 0) return SPF_OK;
+  if (P->n_sorted == 0) return SPF_OK;
   cudaStream_t s = as_stream(stream);
   GridGeom g = geom_of(P);
   BinDims bd;
   for (int d = 0; d < 3; ++d) bd.nb[d] = P->nb[d];
-  float s1 = (float)(P->s_scale * P->n[0] / (2.0 * M_PI));
-  float s2 = (float)(P->s_scale * P->n[1] / (2.0 * M_PI));
-  float s3 = (float)(P->s_scale * P->n[2] / (2.0 * M_PI));
-  SPF_REQUIRE(P->n_items < (1LL << 31), "%s: too many items", what);
-  const PointSrc src{P->s_quats, P->s_ppr, P->s_n_pix, P->s_x, P->s_y, P->s_z};
+  SPF_REQUIRE(P->max_items < (1LL << 31), "%s: too many items", what);
+  const int32_t *n_items = P->bins + 2 * ((int64_t)bd.nb[0] * bd.nb[1] * bd.nb[2]) + 1;
   // TMA map of the padded grid for the bins' boxes (rows are 16-byte aligned)
   CUtensorMap tmap;
   memset(&tmap, 0, sizeof(tmap));
@@ -1836,12 +1822,12 @@ static int sorted_pass(spf_nufft_plan P, const float *d_weights, bool interp, co
   }
   if (interp) {
     SPF_W_DISPATCH(P->w, (k_interp_spread_sorted<W>
-                          <<<(unsigned)P->n_items, SORTED_THREADS, 0, s>>>(
-                              P->re_pad, P->acc_pad, g, bd, P->items, P->sorted, src, s1, s2,
-                              s3, d_weights, tmap, use_tma, device_error_word())));
+                          <<<(unsigned)P->max_items, SORTED_THREADS, 0, s>>>(
+                              P->re_pad, P->acc_pad, g, bd, P->items, n_items, P->sorted,
+                              d_weights, tmap, use_tma, device_error_word())));
   } else {
-    SPF_W_DISPATCH(P->w, (k_spread_sorted<W><<<(unsigned)P->n_items, PEN_THREADS, 0, s>>>(
-                             P->acc_pad, g, bd, P->items, P->sorted, src, s1, s2, s3, d_weights,
+    SPF_W_DISPATCH(P->w, (k_spread_sorted<W><<<(unsigned)P->max_items, PEN_THREADS, 0, s>>>(
+                             P->acc_pad, g, bd, P->items, n_items, P->sorted, d_weights,
                              device_error_word())));
   }
   return check_launch(what);

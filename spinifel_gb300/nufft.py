@@ -135,9 +135,10 @@ class NufftPlan:
                   _lib.ptr(c), x.numel(), _lib.stream_handle())
 
     # from this many points on, spread_orient bin-sorts the points and uses
-    # the sorted spreading (points sharing a footprint cell summed in
-    # registers); below it, the patch or thread-per-point kernels
-    SORTED_MIN_POINTS = 1 << 21
+    # the sorted spreading (a pencil's cells summed in registers); below it,
+    # the patch kernel (2.1e9 points/s; the sort and its pass take as long at
+    # about 1.5e5 points) or the thread-per-point kernel
+    SORTED_MIN_POINTS = 1 << 18
 
     def spread_orient(self, quats, ppr, scale, c, det_shape: tuple | None = None,
                       sort: bool | None = None):

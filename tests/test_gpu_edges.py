@@ -157,3 +157,34 @@ def test_minima_equal_full_fp64_block(kind, n_img, n_ref, n_pix):
         idx, dist = matching.argmin_fp64(x, r, batch=batch)
         assert torch.equal(idx, full.best_idx)
         assert torch.equal(dist, full.best_dist)
+
+
+@pytest.mark.parametrize("w,eps", [(3, 1e-2), (5, 1e-4), (7, 1e-6), (8, 1e-7)])
+@pytest.mark.parametrize("n,spread", [(1, 3.0), (33, 3.0), (1025, 0.02), (5000, 3.0), (20000, 0.3),
+                                      (70001, 3.1)])
+def test_sorted_spread_equals_per_point_spread(w, eps, n, spread):
+    """Bin sort and pencil spreading against one thread per point: the same
+    sums to FP32 rounding (each cell adds at most n terms of one sign here),
+    for one point, points of one cell, dense clusters and whole grids."""
+    from spinifel_gb300.nufft import NufftPlan
+
+    rng = np.random.default_rng(n + w)
+    P = NufftPlan((19, 24, 31), eps)
+    assert P.width == w
+    x, y, z = (torch.as_tensor(rng.uniform(-spread, spread, n).astype(np.float32), device="cuda")
+               for _ in range(3))
+    c = torch.as_tensor(rng.random(n).astype(np.float32), device="cuda")
+    P.spread_zero()
+    P.spread(x, y, z, c)
+    want = P.finish(+1, want_imag=True)
+    for values in (c, c):  # a second pass over one sort
+        P.sort_points(x, y, z)
+        P.spread_zero()
+        P.spread_sorted(values)
+        got = P.finish(+1, want_imag=True)
+        # of the complex sums: near the origin the imaginary part alone cancels
+        a, b = (torch.complex(re.double(), im.double()) for re, im in (got, want))
+        assert float((a - b).norm() / b.norm()) < 1e-5
+    from spinifel_gb300 import matching
+
+    matching.check_device_error()
