@@ -2,7 +2,7 @@
 // FP32 on the device, for the Spinifel slicing and merge operators.
 //
 // Layout in HBM (per plan):
-//   fine   : n1*n2*n3 complex64, the upsampled grid the FFT works on;
+//   fine   : n1*n2*n3 float, the upsampled grid, and half, its half spectrum;
 //   re_pad : (n1+2p)(n2+2p)(n3+2p) float, Re of the type-2 fine grid with a
 //            periodic halo of p = ceil(w/2)+1 cells on every side, so that a
 //            kernel footprint never wraps (no modulo in the inner loop);
@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "tma.cuh"
 #include "es_params.cuh"
+#include "fine_grid.cuh"
 
 struct spf_nufft_plan_s {
   int dev = 0;
@@ -30,7 +31,8 @@ struct spf_nufft_plan_s {
   int w = 0;
   double beta = 0, sigma = 2.0, eps = 1e-6;
   float *inv_p[3] = {nullptr, nullptr, nullptr};  // 1 / kernel FT per mode
-  float2 *fine = nullptr;
+  float *fine = nullptr;       // n1*n2*n3
+  float2 *half = nullptr;      // n1*n2*(n3/2+1)
   float *re_pad = nullptr;
   float *im_pad = nullptr;
   float *acc_pad = nullptr;
@@ -205,45 +207,6 @@ __device__ __forceinline__ void rotate_inv(const float *__restrict__ quat, float
 // ---------------------------------------------------------------------------
 // kernels
 // ---------------------------------------------------------------------------
-
-// b[k mod n] = f_k * support_k / (p1 p2 p3), complex fine grid pre-zeroed.
-__global__ void k_t2_scatter_modes(const float *__restrict__ f, const float *__restrict__ sup,
-                                   int m1, int m2, int m3, int n1, int n2, int n3,
-                                   const float *__restrict__ ip1, const float *__restrict__ ip2,
-                                   const float *__restrict__ ip3, float2 *__restrict__ fine) {
-  int64_t total = (int64_t)m1 * m2 * m3;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    int c = (int)(idx % m3);
-    int b = (int)((idx / m3) % m2);
-    int a = (int)(idx / ((int64_t)m2 * m3));
-    float v = f[idx];
-    if (sup) v *= sup[idx];
-    v *= ip1[a] * ip2[b] * ip3[c];
-    int fa = ((a - m1 / 2) % n1 + n1) % n1;
-    int fb = ((b - m2 / 2) % n2 + n2) % n2;
-    int fc = ((c - m3 / 2) % n3 + n3) % n3;
-    fine[((int64_t)fa * n2 + fb) * n3 + fc] = make_float2(v, 0.0f);
-  }
-}
-
-// re_pad[i] = Re fine[(i - off) mod n] (and Im), for every padded cell.
-__global__ void k_t2_fill_padded(const float2 *__restrict__ fine, GridGeom g, float im_sign,
-                                 float *__restrict__ re_pad, float *__restrict__ im_pad) {
-  int64_t total = (int64_t)g.p1 * g.p2 * g.p3;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    int k = (int)(idx % g.p3);
-    int j = (int)((idx / g.p3) % g.p2);
-    int i = (int)(idx / ((int64_t)g.p2 * g.p3));
-    int a = ((i - g.off1) % g.n1 + g.n1) % g.n1;
-    int b = ((j - g.off2) % g.n2 + g.n2) % g.n2;
-    int c = ((k - g.off3) % g.n3 + g.n3) % g.n3;
-    float2 v = fine[((int64_t)a * g.n2 + b) * g.n3 + c];
-    re_pad[idx] = v.x;
-    if (im_pad) im_pad[idx] = im_sign * v.y;
-  }
-}
 
 template <int W>
 __global__ void k_t2_interp(const float *__restrict__ re_pad, const float *__restrict__ im_pad,
@@ -1334,56 +1297,6 @@ __global__ void __launch_bounds__(PEN_THREADS, 6)
   box_flush(abox, acc_pad, g, shape);
 }
 
-// fine[l] = sum of acc_pad[i] over padded i == l + off (mod n)  (Im = 0).
-__global__ void k_t1_fold(const float *__restrict__ acc_pad, GridGeom g,
-                          float2 *__restrict__ fine) {
-  int64_t total = (int64_t)g.n1 * g.n2 * g.n3;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    int c = (int)(idx % g.n3);
-    int b = (int)((idx / g.n3) % g.n2);
-    int a = (int)(idx / ((int64_t)g.n2 * g.n3));
-    int ia[2], ib[2], ic[2];
-    int na = 0, nb = 0, nc = 0;
-    int i0 = (a + g.off1) % g.n1;
-    ia[na++] = i0;
-    if (i0 + g.n1 < g.p1) ia[na++] = i0 + g.n1;
-    int j0 = (b + g.off2) % g.n2;
-    ib[nb++] = j0;
-    if (j0 + g.n2 < g.p2) ib[nb++] = j0 + g.n2;
-    int k0 = (c + g.off3) % g.n3;
-    ic[nc++] = k0;
-    if (k0 + g.n3 < g.p3) ic[nc++] = k0 + g.n3;
-    float s = 0.0f;
-    for (int u = 0; u < na; ++u)
-      for (int v = 0; v < nb; ++v)
-        for (int q = 0; q < nc; ++q)
-          s += acc_pad[((int64_t)ia[u] * g.p2 + ib[v]) * g.p3 + ic[q]];
-    fine[idx] = make_float2(s, 0.0f);
-  }
-}
-
-// modes[k] = fine[k mod n] / (p1 p2 p3)
-__global__ void k_t1_extract(const float2 *__restrict__ fine, int m1, int m2, int m3, int n1,
-                             int n2, int n3, const float *__restrict__ ip1,
-                             const float *__restrict__ ip2, const float *__restrict__ ip3,
-                             float *__restrict__ out_re, float *__restrict__ out_im) {
-  int64_t total = (int64_t)m1 * m2 * m3;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    int c = (int)(idx % m3);
-    int b = (int)((idx / m3) % m2);
-    int a = (int)(idx / ((int64_t)m2 * m3));
-    int fa = ((a - m1 / 2) % n1 + n1) % n1;
-    int fb = ((b - m2 / 2) % n2 + n2) % n2;
-    int fc = ((c - m3 / 2) % n3 + n3) % n3;
-    float2 v = fine[((int64_t)fa * n2 + fb) * n3 + fc];
-    float s = ip1[a] * ip2[b] * ip3[c];
-    out_re[idx] = v.x * s;
-    if (out_im) out_im[idx] = v.y * s;
-  }
-}
-
 // ---------------------------------------------------------------------------
 // dispatch on the kernel width
 // ---------------------------------------------------------------------------
@@ -1413,16 +1326,21 @@ static int check_plan(spf_nufft_plan P, const char *what) {
   return SPF_OK;
 }
 
-static int fft_exec(spf_nufft_plan P, int isign, cudaStream_t s, const char *what) {
+static GridDims grid_dims(const spf_nufft_plan_s *P) {
+  const GridGeom g = geom_of(P);
+  return GridDims{g.n1, g.n2, g.n3, g.p1, g.p2, g.p3, g.off1, g.off2, g.off3};
+}
+
+// half spectrum (sign -1) of the fine grid
+static int fft_exec(spf_nufft_plan P, cudaStream_t s, const char *what) {
   if (cufftSetStream(P->fft, s) != CUFFT_SUCCESS) {
     set_error("%s: cufftSetStream failed", what);
     return SPF_ERR_CUDA;
   }
-  cufftResult r = cufftExecC2C(P->fft, reinterpret_cast<cufftComplex *>(P->fine),
-                               reinterpret_cast<cufftComplex *>(P->fine),
-                               isign < 0 ? CUFFT_FORWARD : CUFFT_INVERSE);
+  cufftResult r = cufftExecR2C(P->fft, reinterpret_cast<cufftReal *>(P->fine),
+                               reinterpret_cast<cufftComplex *>(P->half));
   if (r != CUFFT_SUCCESS) {
-    set_error("%s: cufftExecC2C failed (%d)", what, (int)r);
+    set_error("%s: cufftExecR2C failed (%d)", what, (int)r);
     return SPF_ERR_CUDA;
   }
   count_launch();
@@ -1472,11 +1390,15 @@ int spf_nufft_plan_create(int m1, int m2, int m3, double eps, double upsampfac,
       st = check_cuda(cudaMemcpy(P->inv_p[d], v.data(), v.size() * sizeof(float),
                                  cudaMemcpyHostToDevice), "plan_create");
   }
-  if (st == SPF_OK) st = check_cuda(cudaMalloc(&P->fine, nfine * sizeof(float2)), "plan_create");
+  // one allocation: the real grid (an even number of values), then its half spectrum
+  if (st == SPF_OK)
+    st = check_cuda(cudaMalloc(&P->fine, nfine * sizeof(float) + (size_t)P->n[0] * P->n[1] *
+                                             (P->n[2] / 2 + 1) * sizeof(float2)), "plan_create");
+  if (st == SPF_OK) P->half = reinterpret_cast<float2 *>(P->fine + nfine);
   if (st == SPF_OK) st = check_cuda(cudaMalloc(&P->re_pad, npad * sizeof(float)), "plan_create");
   if (st == SPF_OK) st = check_cuda(cudaMalloc(&P->acc_pad, npad * sizeof(float)), "plan_create");
   if (st == SPF_OK) {
-    cufftResult r = cufftPlan3d(&P->fft, P->n[0], P->n[1], P->n[2], CUFFT_C2C);
+    cufftResult r = cufftPlan3d(&P->fft, P->n[0], P->n[1], P->n[2], CUFFT_R2C);
     if (r != CUFFT_SUCCESS) {
       set_error("plan_create: cufftPlan3d(%d,%d,%d) failed (%d)", P->n[0], P->n[1], P->n[2], (int)r);
       st = r == CUFFT_ALLOC_FAILED ? SPF_ERR_OOM : SPF_ERR_CUDA;
@@ -1528,21 +1450,18 @@ int spf_nufft_t2_set_modes(spf_nufft_plan P, const float *d_modes, const float *
   SPF_REQUIRE(d_modes != nullptr, "spf_nufft_t2_set_modes: modes is NULL");
   SPF_REQUIRE(isign == 1 || isign == -1, "spf_nufft_t2_set_modes: isign must be +-1");
   cudaStream_t s = as_stream(stream);
-  size_t nfine = (size_t)P->n[0] * P->n[1] * P->n[2];
-  size_t npad = (size_t)P->np[0] * P->np[1] * P->np[2];
+  const size_t npad = (size_t)P->np[0] * P->np[1] * P->np[2];
   if (want_imag && !P->im_pad)
     SPF_TRY(check_cuda(cudaMalloc(&P->im_pad, npad * sizeof(float)), "spf_nufft_t2_set_modes"));
-  SPF_TRY(check_cuda(cudaMemsetAsync(P->fine, 0, nfine * sizeof(float2), s), "t2_set_modes"));
-  int64_t nm = (int64_t)P->m[0] * P->m[1] * P->m[2];
-  k_t2_scatter_modes<<<grid_for(nm, 256, 8 * 1024), 256, 0, s>>>(
-      d_modes, d_support, P->m[0], P->m[1], P->m[2], P->n[0], P->n[1], P->n[2], P->inv_p[0],
-      P->inv_p[1], P->inv_p[2], P->fine);
-  SPF_TRY(check_launch("k_t2_scatter_modes"));
-  SPF_TRY(fft_exec(P, isign, s, "spf_nufft_t2_set_modes"));
-  GridGeom g = geom_of(P);
-  k_t2_fill_padded<<<grid_for((int64_t)npad, 256, 16 * 1024), 256, 0, s>>>(
-      P->fine, g, 1.0f, P->re_pad, want_imag ? P->im_pad : nullptr);
-  return check_launch("k_t2_fill_padded");
+  const GridDims g = grid_dims(P);
+  k_modes_to_grid<float><<<row_grid((int64_t)g.n1 * g.n2), row_block(), 0, s>>>(
+      d_modes, d_support, P->m[0], P->m[1], P->m[2], g, P->inv_p[0], P->inv_p[1], P->inv_p[2],
+      P->fine);
+  SPF_TRY(check_launch("k_modes_to_grid"));
+  SPF_TRY(fft_exec(P, s, "spf_nufft_t2_set_modes"));
+  k_spectrum_to_padded<float><<<row_grid((int64_t)g.p1 * g.p2), row_block(), 0, s>>>(
+      P->half, g, isign < 0 ? float(1) : float(-1), P->re_pad, want_imag ? P->im_pad : nullptr);
+  return check_launch("k_spectrum_to_padded");
 }
 
 int spf_nufft_t2_interp(spf_nufft_plan P, const float *d_x, const float *d_y, const float *d_z,
@@ -1847,16 +1766,14 @@ int spf_nufft_t1_finish(spf_nufft_plan P, int isign, float *d_out_re, float *d_o
   SPF_REQUIRE(isign == 1 || isign == -1, "spf_nufft_t1_finish: isign must be +-1");
   SPF_REQUIRE(d_out_re != nullptr, "spf_nufft_t1_finish: out_re is NULL");
   cudaStream_t s = as_stream(stream);
-  GridGeom g = geom_of(P);
-  int64_t nfine = (int64_t)P->n[0] * P->n[1] * P->n[2];
-  k_t1_fold<<<grid_for(nfine, 256, 16 * 1024), 256, 0, s>>>(P->acc_pad, g, P->fine);
-  SPF_TRY(check_launch("k_t1_fold"));
-  SPF_TRY(fft_exec(P, isign, s, "spf_nufft_t1_finish"));
-  int64_t nm = (int64_t)P->m[0] * P->m[1] * P->m[2];
-  k_t1_extract<<<grid_for(nm, 256, 16 * 1024), 256, 0, s>>>(
-      P->fine, P->m[0], P->m[1], P->m[2], P->n[0], P->n[1], P->n[2], P->inv_p[0], P->inv_p[1],
-      P->inv_p[2], d_out_re, d_out_im);
-  return check_launch("k_t1_extract");
+  const GridDims g = grid_dims(P);
+  k_fold_padded<float><<<row_grid((int64_t)g.n1 * g.n2), row_block(), 0, s>>>(P->acc_pad, g, P->fine);
+  SPF_TRY(check_launch("k_fold_padded"));
+  SPF_TRY(fft_exec(P, s, "spf_nufft_t1_finish"));
+  k_spectrum_to_modes<float><<<row_grid((int64_t)P->m[0] * P->m[1]), row_block(), 0, s>>>(
+      P->half, P->m[0], P->m[1], P->m[2], g, P->inv_p[0], P->inv_p[1], P->inv_p[2],
+      isign < 0 ? float(1) : float(-1), d_out_re, d_out_im);
+  return check_launch("k_spectrum_to_modes");
 }
 
 int spf_spread_t1(spf_nufft_plan P, const float *d_x, const float *d_y, const float *d_z,

@@ -4,7 +4,7 @@
 // cannot reach (its floor is about 1e-7).  Kernel widths 2..16.
 //
 // Same layout and conventions as the FP32 plan of nufft.cu, in double:
-//   fine   : n1*n2*n3 complex128, the upsampled grid (cuFFT Z2Z);
+//   fine   : n1*n2*n3, the upsampled grid, and half, its half spectrum (D2Z);
 //   re_pad : Re of the type-2 fine grid with a periodic halo of
 //            p = ceil(w/2)+1 cells per side (no modulo in the inner loops);
 //   im_pad : Im (only when requested);
@@ -22,6 +22,7 @@
 
 #include "common.cuh"
 #include "es_params.cuh"
+#include "fine_grid.cuh"
 
 struct spf_nufft64_plan_s {
   int dev = 0;
@@ -32,7 +33,8 @@ struct spf_nufft64_plan_s {
   int w = 0;
   double beta = 0, sigma = 2.0, eps = 1e-12;
   double *inv_p[3] = {nullptr, nullptr, nullptr};
-  double2 *fine = nullptr;
+  double *fine = nullptr;       // n1*n2*n3
+  double2 *half = nullptr;      // n1*n2*(n3/2+1)
   double *re_pad = nullptr;
   double *im_pad = nullptr;
   double *acc_pad = nullptr;
@@ -125,45 +127,6 @@ __device__ __forceinline__ void rotate_inv(const double *__restrict__ quat, doub
   l = r02 * qx + r12 * qy + r22 * qz;
 }
 
-// b[k mod n] = f_k * support_k / (p1 p2 p3), complex fine grid pre-zeroed.
-__global__ void k_scatter_modes(const double *__restrict__ f, const double *__restrict__ sup,
-                                int m1, int m2, int m3, int n1, int n2, int n3,
-                                const double *__restrict__ ip1, const double *__restrict__ ip2,
-                                const double *__restrict__ ip3, double2 *__restrict__ fine) {
-  const int64_t total = (int64_t)m1 * m2 * m3;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(idx % m3);
-    const int b = (int)((idx / m3) % m2);
-    const int a = (int)(idx / ((int64_t)m2 * m3));
-    double v = f[idx];
-    if (sup) v *= sup[idx];
-    v *= ip1[a] * ip2[b] * ip3[c];
-    const int fa = ((a - m1 / 2) % n1 + n1) % n1;
-    const int fb = ((b - m2 / 2) % n2 + n2) % n2;
-    const int fc = ((c - m3 / 2) % n3 + n3) % n3;
-    fine[((int64_t)fa * n2 + fb) * n3 + fc] = make_double2(v, 0.0);
-  }
-}
-
-// re_pad[i] = Re fine[(i - off) mod n] (and Im), every padded cell.
-__global__ void k_fill_padded(const double2 *__restrict__ fine, Geom g,
-                              double *__restrict__ re_pad, double *__restrict__ im_pad) {
-  const int64_t total = (int64_t)g.p1 * g.p2 * g.p3;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int k = (int)(idx % g.p3);
-    const int j = (int)((idx / g.p3) % g.p2);
-    const int i = (int)(idx / ((int64_t)g.p2 * g.p3));
-    const int a = ((i - g.off1) % g.n1 + g.n1) % g.n1;
-    const int b = ((j - g.off2) % g.n2 + g.n2) % g.n2;
-    const int c = ((k - g.off3) % g.n3 + g.n3) % g.n3;
-    const double2 v = fine[((int64_t)a * g.n2 + b) * g.n3 + c];
-    re_pad[idx] = v.x;
-    if (im_pad) im_pad[idx] = v.y;
-  }
-}
-
 template <int W>
 __global__ void __launch_bounds__(128)
     k_interp(const double *__restrict__ re_pad, const double *__restrict__ im_pad, Geom g,
@@ -220,45 +183,6 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// fine[l] = sum of acc_pad[i] over padded i == l + off (mod n), Im = 0.
-__global__ void k_fold(const double *__restrict__ acc_pad, Geom g, double2 *__restrict__ fine) {
-  const int64_t total = (int64_t)g.n1 * g.n2 * g.n3;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(idx % g.n3);
-    const int b = (int)((idx / g.n3) % g.n2);
-    const int a = (int)(idx / ((int64_t)g.n2 * g.n3));
-    // padded indices i = l + off - n*s for the s that keep i in [0, p)
-    double v = 0.0;
-    for (int i = (a + g.off1) % g.n1; i < g.p1; i += g.n1)
-      for (int j = (b + g.off2) % g.n2; j < g.p2; j += g.n2)
-        for (int k = (c + g.off3) % g.n3; k < g.p3; k += g.n3)
-          v += acc_pad[((int64_t)i * g.p2 + j) * g.p3 + k];
-    fine[idx] = make_double2(v, 0.0);
-  }
-}
-
-// modes[k] = fine[k mod n] / (p1 p2 p3)
-__global__ void k_extract(const double2 *__restrict__ fine, int m1, int m2, int m3, int n1,
-                          int n2, int n3, const double *__restrict__ ip1,
-                          const double *__restrict__ ip2, const double *__restrict__ ip3,
-                          double *__restrict__ out_re, double *__restrict__ out_im) {
-  const int64_t total = (int64_t)m1 * m2 * m3;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(idx % m3);
-    const int b = (int)((idx / m3) % m2);
-    const int a = (int)(idx / ((int64_t)m2 * m3));
-    const int fa = ((a - m1 / 2) % n1 + n1) % n1;
-    const int fb = ((b - m2 / 2) % n2 + n2) % n2;
-    const int fc = ((c - m3 / 2) % n3 + n3) % n3;
-    const double2 v = fine[((int64_t)fa * n2 + fb) * n3 + fc];
-    const double s = ip1[a] * ip2[b] * ip3[c];
-    out_re[idx] = v.x * s;
-    if (out_im) out_im[idx] = v.y * s;
-  }
-}
-
 #define SPF_W64_DISPATCH(w, KERNEL_CALL)                           \
   switch (w) {                                                     \
     case 2: { constexpr int W = 2; KERNEL_CALL; break; }           \
@@ -293,16 +217,21 @@ static int check_plan(spf_nufft64_plan P, const char *what) {
   return SPF_OK;
 }
 
-static int fft_exec(spf_nufft64_plan P, int isign, cudaStream_t s, const char *what) {
+static GridDims grid_dims(const spf_nufft64_plan_s *P) {
+  const Geom g = geom_of(P);
+  return GridDims{g.n1, g.n2, g.n3, g.p1, g.p2, g.p3, g.off1, g.off2, g.off3};
+}
+
+// half spectrum (sign -1) of the fine grid
+static int fft_exec(spf_nufft64_plan P, cudaStream_t s, const char *what) {
   if (cufftSetStream(P->fft, s) != CUFFT_SUCCESS) {
     set_error("%s: cufftSetStream failed", what);
     return SPF_ERR_CUDA;
   }
-  cufftResult r = cufftExecZ2Z(P->fft, reinterpret_cast<cufftDoubleComplex *>(P->fine),
-                               reinterpret_cast<cufftDoubleComplex *>(P->fine),
-                               isign < 0 ? CUFFT_FORWARD : CUFFT_INVERSE);
+  cufftResult r = cufftExecD2Z(P->fft, reinterpret_cast<cufftDoubleReal *>(P->fine),
+                               reinterpret_cast<cufftDoubleComplex *>(P->half));
   if (r != CUFFT_SUCCESS) {
-    set_error("%s: cufftExecZ2Z failed (%d)", what, (int)r);
+    set_error("%s: cufftExecD2Z failed (%d)", what, (int)r);
     return SPF_ERR_CUDA;
   }
   count_launch();
@@ -356,10 +285,14 @@ int spf_nufft64_plan_create(int m1, int m2, int m3, double eps, double upsampfac
       st = check_cuda(cudaMemcpy(P->inv_p[d], v.data(), v.size() * sizeof(double),
                                  cudaMemcpyHostToDevice), "plan64_create");
   }
-  if (st == SPF_OK) st = check_cuda(cudaMalloc(&P->fine, nfine * sizeof(double2)), "plan64_create");
+  // one allocation: the real grid (an even number of values), then its half spectrum
+  if (st == SPF_OK)
+    st = check_cuda(cudaMalloc(&P->fine, nfine * sizeof(double) + (size_t)P->n[0] * P->n[1] *
+                                             (P->n[2] / 2 + 1) * sizeof(double2)), "plan64_create");
+  if (st == SPF_OK) P->half = reinterpret_cast<double2 *>(P->fine + nfine);
   if (st == SPF_OK) st = check_cuda(cudaMalloc(&P->re_pad, npad * sizeof(double)), "plan64_create");
   if (st == SPF_OK) {
-    cufftResult r = cufftPlan3d(&P->fft, P->n[0], P->n[1], P->n[2], CUFFT_Z2Z);
+    cufftResult r = cufftPlan3d(&P->fft, P->n[0], P->n[1], P->n[2], CUFFT_D2Z);
     if (r != CUFFT_SUCCESS) {
       set_error("plan64_create: cufftPlan3d(%d,%d,%d) failed (%d)", P->n[0], P->n[1], P->n[2],
                 (int)r);
@@ -410,22 +343,18 @@ int spf_nufft64_t2_set_modes(spf_nufft64_plan P, const double *d_modes, const do
   SPF_REQUIRE(d_modes != nullptr, "spf_nufft64_t2_set_modes: modes is NULL");
   SPF_REQUIRE(isign == 1 || isign == -1, "spf_nufft64_t2_set_modes: isign must be +-1");
   cudaStream_t s = as_stream(stream);
-  const size_t nfine = (size_t)P->n[0] * P->n[1] * P->n[2];
   const size_t npad = (size_t)P->np[0] * P->np[1] * P->np[2];
   if (want_imag && !P->im_pad)
     SPF_TRY(check_cuda(cudaMalloc(&P->im_pad, npad * sizeof(double)), "spf_nufft64_t2_set_modes"));
-  SPF_TRY(check_cuda(cudaMemsetAsync(P->fine, 0, nfine * sizeof(double2), s),
-                     "spf_nufft64_t2_set_modes"));
-  const int64_t nm = (int64_t)P->m[0] * P->m[1] * P->m[2];
-  k_scatter_modes<<<grid_for(nm, 256, 8 * 1024), 256, 0, s>>>(
-      d_modes, d_support, P->m[0], P->m[1], P->m[2], P->n[0], P->n[1], P->n[2], P->inv_p[0],
-      P->inv_p[1], P->inv_p[2], P->fine);
-  SPF_TRY(check_launch("k_scatter_modes (f64)"));
-  SPF_TRY(fft_exec(P, isign, s, "spf_nufft64_t2_set_modes"));
-  const Geom g = geom_of(P);
-  k_fill_padded<<<grid_for((int64_t)npad, 256, 16 * 1024), 256, 0, s>>>(
-      P->fine, g, P->re_pad, want_imag ? P->im_pad : nullptr);
-  return check_launch("k_fill_padded (f64)");
+  const GridDims g = grid_dims(P);
+  k_modes_to_grid<double><<<row_grid((int64_t)g.n1 * g.n2), row_block(), 0, s>>>(
+      d_modes, d_support, P->m[0], P->m[1], P->m[2], g, P->inv_p[0], P->inv_p[1], P->inv_p[2],
+      P->fine);
+  SPF_TRY(check_launch("k_modes_to_grid"));
+  SPF_TRY(fft_exec(P, s, "spf_nufft64_t2_set_modes"));
+  k_spectrum_to_padded<double><<<row_grid((int64_t)g.p1 * g.p2), row_block(), 0, s>>>(
+      P->half, g, isign < 0 ? double(1) : double(-1), P->re_pad, want_imag ? P->im_pad : nullptr);
+  return check_launch("k_spectrum_to_padded");
 }
 
 int spf_nufft64_t2_interp(spf_nufft64_plan P, const double *d_x, const double *d_y,
@@ -494,16 +423,14 @@ int spf_nufft64_t1_finish(spf_nufft64_plan P, int isign, double *d_out_re, doubl
   SPF_REQUIRE(isign == 1 || isign == -1, "spf_nufft64_t1_finish: isign must be +-1");
   SPF_REQUIRE(d_out_re != nullptr, "spf_nufft64_t1_finish: out_re is NULL");
   cudaStream_t s = as_stream(stream);
-  const Geom g = geom_of(P);
-  const int64_t nfine = (int64_t)P->n[0] * P->n[1] * P->n[2];
-  k_fold<<<grid_for(nfine, 256, 16 * 1024), 256, 0, s>>>(P->acc_pad, g, P->fine);
-  SPF_TRY(check_launch("k_fold (f64)"));
-  SPF_TRY(fft_exec(P, isign, s, "spf_nufft64_t1_finish"));
-  const int64_t nm = (int64_t)P->m[0] * P->m[1] * P->m[2];
-  k_extract<<<grid_for(nm, 256, 16 * 1024), 256, 0, s>>>(
-      P->fine, P->m[0], P->m[1], P->m[2], P->n[0], P->n[1], P->n[2], P->inv_p[0], P->inv_p[1],
-      P->inv_p[2], d_out_re, d_out_im);
-  return check_launch("k_extract (f64)");
+  const GridDims g = grid_dims(P);
+  k_fold_padded<double><<<row_grid((int64_t)g.n1 * g.n2), row_block(), 0, s>>>(P->acc_pad, g, P->fine);
+  SPF_TRY(check_launch("k_fold_padded"));
+  SPF_TRY(fft_exec(P, s, "spf_nufft64_t1_finish"));
+  k_spectrum_to_modes<double><<<row_grid((int64_t)P->m[0] * P->m[1]), row_block(), 0, s>>>(
+      P->half, P->m[0], P->m[1], P->m[2], g, P->inv_p[0], P->inv_p[1], P->inv_p[2],
+      isign < 0 ? double(1) : double(-1), d_out_re, d_out_im);
+  return check_launch("k_spectrum_to_modes");
 }
 
 }  // extern "C"

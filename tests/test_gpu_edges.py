@@ -188,3 +188,35 @@ def test_sorted_spread_equals_per_point_spread(w, eps, n, spread):
     from spinifel_gb300 import matching
 
     matching.check_device_error()
+
+
+@pytest.mark.parametrize("m", [(9, 8, 7), (5, 12, 21), (16, 3, 2)])
+@pytest.mark.parametrize("isign", [1, -1])
+@pytest.mark.parametrize("eps", [1e-6, 1e-12])
+def test_real_transforms_against_direct_sums(m, isign, eps):
+    """Both halves of the spectrum, both signs, odd and even mode counts: type
+    2 and type 1 against the direct sums at the plan's tolerance (20 eps, and
+    1e-5 for what FP32 resolves)."""
+    from oracle import nufft as onufft
+    from spinifel_gb300.nufft import make_plan
+
+    rng = np.random.default_rng(sum(m) + isign)
+    P = make_plan(m, eps)
+    dt = np.float32 if eps > 1e-7 else np.float64
+    tol = 1e-5 if eps > 1e-7 else 20 * eps
+    x, y, z = rng.uniform(-np.pi, np.pi, (3, 300)).astype(dt)
+    f, c = rng.standard_normal(m).astype(dt), rng.standard_normal(300).astype(dt)
+    t = [torch.as_tensor(v, device="cuda") for v in (x, y, z, c, f)]
+    P.set_modes(t[4], isign=isign, want_imag=True)
+    re, im = P.interp(*t[:3], want_imag=True)
+    got = re.cpu().numpy() + 1j * im.cpu().numpy()
+    want = onufft.nudft3d2(x.astype(float), y.astype(float), z.astype(float), f.astype(float),
+                           isign)
+    assert np.linalg.norm(got - want) < tol * np.linalg.norm(want)
+    P.spread_zero()
+    P.spread(*t[:4])
+    re, im = P.finish(isign, want_imag=True)
+    got = re.cpu().numpy() + 1j * im.cpu().numpy()
+    want = onufft.nudft3d1(x.astype(float), y.astype(float), z.astype(float), c.astype(float), m,
+                           isign)
+    assert np.linalg.norm(got - want) < tol * np.linalg.norm(want)
