@@ -15,6 +15,7 @@
 #include <cufft.h>
 #include <math.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -373,8 +374,8 @@ __device__ __forceinline__ void box_flush(const float *box, float *__restrict__ 
   });
 }
 
-// Slicing on a multi-panel detector [n_panels][nx][ny]: a CTA of 256 threads
-// takes a 16 x 16 pixel patch of one panel at one orientation, so its points
+// Slicing on a multi-panel detector [n_panels][nx][ny]: a CTA takes a 16 x 16
+// or 8 x 16 pixel patch of one panel at one orientation, so its points
 // are neighbours on the Ewald sphere.  It finds the bounding box of their
 // kernel footprints in the padded fine grid, stages that box in shared memory
 // (coalesced along the fastest axis) and interpolates from there; a box too
@@ -390,7 +391,7 @@ __device__ __forceinline__ int patch_dx(int t) { return ((t >> 5) >> 1) * 4 + ((
 __device__ __forceinline__ int patch_dy(int t) { return ((t >> 5) & 1) * 8 + (t & 7); }
 constexpr int SLICE_SMEM_FLOATS = 11264;  // 44 KB
 
-// Tile shapes of the slicing kernel (256 threads, one pixel each): the patch
+// Tile shapes of the slicing kernel (a thread a pixel): the patch
 // is px x py pixels of a panel and each warp takes a wx x wy block of it.
 // The shape decides how many distinct box rows a warp's loads touch (bank
 // conflicts) and the box's size; which is fastest depends on the detector's
@@ -404,10 +405,11 @@ constexpr int SLICE_SMEM_FLOATS = 11264;  // 44 KB
 // + 0..3, sk = dk + 0..3) by the number of distinct banks its warps'
 // footprint starts hit (one warp-wide OR of bank bits per candidate) and
 // keeps the best one that fits in shared memory.
+constexpr int SLICE_SHAPE_8X16 = 8;  // 128 threads, picked by default_shape
 struct PatchShape {
   int px, py, wx, wy, search;
 };
-constexpr int N_SLICE_SHAPES = 8;
+constexpr int N_SLICE_SHAPES = 8;  // that SPF_TUNE_SLICE_SHAPE may pick
 constexpr int SLICE_SEARCH = 4;  // candidates per stride
 __host__ __device__ inline PatchShape slice_shape(int code) {
   switch (code) {
@@ -416,9 +418,10 @@ __host__ __device__ inline PatchShape slice_shape(int code) {
     case 3: return PatchShape{8, 32, 4, 8, 0};
     case 4: return PatchShape{32, 8, 8, 4, 0};
     case 5: return PatchShape{32, 8, 16, 2, 0};
-    case 6: return PatchShape{16, 16, 4, 8, 1};
     case 7: return PatchShape{16, 16, 8, 4, 1};
-    default: return PatchShape{16, 16, 4, 8, 0};
+    case SLICE_SHAPE_8X16: return PatchShape{8, 16, 4, 8, 0};
+    case SLICE_SHAPE_8X16 + 1: return PatchShape{8, 16, 4, 8, 1};
+    default: return PatchShape{16, 16, 4, 8, 1};  // 6
   }
 }
 
@@ -427,8 +430,8 @@ __global__ void __launch_bounds__(256)
     k_slice_t2_det(const float *__restrict__ re_pad, GridGeom g, const float *__restrict__ quats,
                    const float *__restrict__ ppr, int n_panels, int nx, int ny, float scale1,
                    float scale2, float scale3, float *__restrict__ out,
-                   __nv_bfloat16 *__restrict__ out_bf16, PatchShape ps) {
-  __shared__ float box[SLICE_SMEM_FLOATS];
+                   __nv_bfloat16 *__restrict__ out_bf16, PatchShape ps, int box_floats) {
+  extern __shared__ float box[];  // box_floats
   constexpr int NCAND = SLICE_SEARCH * SLICE_SEARCH;
   __shared__ int bb[7];
   __shared__ int score[8][NCAND];
@@ -499,7 +502,7 @@ __global__ void __launch_bounds__(256)
       int tot = 0;
       if (lane < NCAND)
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tot += score[w][lane];
-      const bool fits = lane < NCAND && (int64_t)di * sjc * skc <= SLICE_SMEM_FLOATS;
+      const bool fits = lane < NCAND && (int64_t)di * sjc * skc <= box_floats;
       // most distinct banks; ties go to the lower candidate (the smaller box)
       const int key = fits ? (tot << 5) | (31 - lane) : -1;
       const int best = __reduce_max_sync(0xffffffffu, key);
@@ -513,7 +516,7 @@ __global__ void __launch_bounds__(256)
   }
   const int64_t svol = (int64_t)di * sj * sk;
   float acc = 0.0f;
-  if (bb[3] >= imin && svol <= SLICE_SMEM_FLOATS) {
+  if (bb[3] >= imin && svol <= box_floats) {
     const BoxShape shape{imin, jmin, kmin, di, dj, dk, sj * sk, sk};
     if ((g.p3 & 3) == 0)
       box_load_q(box, re_pad, g, shape);
@@ -1499,6 +1502,27 @@ int spf_slice_t2(spf_nufft_plan P, const float *d_quats, int64_t n_orient, const
   return check_launch("k_slice_t2");
 }
 
+// Patch shape where none was tuned, by the spacing of the pixels in grid
+// cells (n / sqrt(n_pix) for a detector that spans the grid, as the panels of
+// a flat detector do).  The patch decides whether its box fits in shared
+// memory; the stride search (16 reductions a warp) pays unless the footprints
+// of a warp all but coincide.  Times in us with 16 x 16 patches, 16 x 16 with
+// the search, 8 x 16 without and with it (grid, detector, orientations):
+//   0.35 cells  90^3,  4 x 128 x 128,  100:   384   420   378   417
+//   0.63 cells 162^3,  4 x 128 x 128,  500:  2474  2061  2119  2050
+//   1.25 cells 320^3,  4 x 128 x 128,  200:  1622  1474  1469  1349
+//   1.41 cells  90^3,  4 x 32 x 32,   2000:  1308  1187   989   911
+//   1.72 cells 128^3,  3 x 50 x 37,    500:   362   315   313   294
+//   2.53 cells 162^3,  4 x 32 x 32,   1000:  1639  1629  3793  1779
+// (A detector with more 8 x 16 patches than a launch takes keeps 16 x 16.)
+static int default_shape(const spf_nufft_plan_s *P, int n_panels, int nx, int ny) {
+  const int64_t n_pix = (int64_t)n_panels * nx * ny;
+  if ((int64_t)n_panels * ((nx + 7) / 8) * ((ny + 15) / 16) > 65535) return 6;
+  const int n = std::max(P->n[0], std::max(P->n[1], P->n[2]));
+  const double cells = n / sqrt((double)n_pix);
+  return cells < 0.5 ? SLICE_SHAPE_8X16 : cells < 2.2 ? SLICE_SHAPE_8X16 + 1 : 6;
+}
+
 int spf_slice_t2_det(spf_nufft_plan P, const float *d_quats, int64_t n_orient, const float *d_ppr,
                      int n_panels, int nx, int ny, double scale, float *d_out, void *d_out_bf16,
                      void *stream) {
@@ -1507,8 +1531,9 @@ int spf_slice_t2_det(spf_nufft_plan P, const float *d_quats, int64_t n_orient, c
               "spf_slice_t2_det: negative size");
   if (n_orient == 0 || n_panels == 0 || nx == 0 || ny == 0) return SPF_OK;
   SPF_REQUIRE(d_quats && d_ppr && d_out, "spf_slice_t2_det: NULL pointer");
-  const int code = (int)tune_get(SPF_TUNE_SLICE_SHAPE, 0);
-  const PatchShape ps = slice_shape(code >= 0 && code < N_SLICE_SHAPES ? code : 0);
+  const int tuned = (int)tune_get(SPF_TUNE_SLICE_SHAPE, 0);
+  const PatchShape ps = slice_shape(
+      tuned > 0 && tuned < N_SLICE_SHAPES ? tuned : default_shape(P, n_panels, nx, ny));
   int64_t patches = (int64_t)n_panels * ((nx + ps.px - 1) / ps.px) * ((ny + ps.py - 1) / ps.py);
   SPF_REQUIRE(n_orient < (1LL << 31) && patches <= 65535, "spf_slice_t2_det: size too large");
   cudaStream_t s = as_stream(stream);
@@ -1518,14 +1543,18 @@ int spf_slice_t2_det(spf_nufft_plan P, const float *d_quats, int64_t n_orient, c
   float s3 = (float)(scale * P->n[2] / (2.0 * M_PI));
   dim3 grid((unsigned)n_orient, (unsigned)patches);
   auto *bf = reinterpret_cast<__nv_bfloat16 *>(d_out_bf16);
+  const int threads = ps.px * ps.py;
+  // five CTAs an SM of 256 threads, six of 128
+  const int floats = threads == 256 ? SLICE_SMEM_FLOATS : SLICE_SMEM_FLOATS * 5 / 6;
+  const size_t smem = floats * sizeof(float);
   if (ps.search) {
-    SPF_W_DISPATCH(P->w, (k_slice_t2_det<W, true><<<grid, 256, 0, s>>>(
+    SPF_W_DISPATCH(P->w, (k_slice_t2_det<W, true><<<grid, threads, smem, s>>>(
                              P->re_pad, g, d_quats, d_ppr, n_panels, nx, ny, s1, s2, s3, d_out,
-                             bf, ps)));
+                             bf, ps, floats)));
   } else {
-    SPF_W_DISPATCH(P->w, (k_slice_t2_det<W, false><<<grid, 256, 0, s>>>(
+    SPF_W_DISPATCH(P->w, (k_slice_t2_det<W, false><<<grid, threads, smem, s>>>(
                              P->re_pad, g, d_quats, d_ppr, n_panels, nx, ny, s1, s2, s3, d_out,
-                             bf, ps)));
+                             bf, ps, floats)));
   }
   return check_launch("k_slice_t2_det");
 }

@@ -190,6 +190,30 @@ def test_sorted_spread_equals_per_point_spread(w, eps, n, spread):
     matching.check_device_error()
 
 
+@pytest.mark.parametrize("M,det,n", [(41, (4, 32, 32), 30), (41, (4, 128, 128), 3),
+                                     (41, (4, 16, 16), 9), (31, (3, 50, 37), 20),
+                                     (61, (1, 7, 33), 40), (21, (2, 8, 16), 50),
+                                     (25, (1, 9, 17), 12), (81, (1, 1, 1), 5)])
+def test_default_patch_shape_gives_per_point_bits(M, det, n):
+    """The patch shape picked by the pixels' spacing slices with the bits of
+    the per-point kernel, bf16 copy included, whole and ragged patches alike."""
+    from spinifel_gb300 import geom
+    from spinifel_gb300.nufft import NufftPlan
+
+    rng = np.random.default_rng(M + n)
+    ppr, pdr = geom.flat_detector(*det)
+    q = torch.as_tensor(geom.uniform_quaternions(n, rng).astype(np.float32), device="cuda")
+    p = torch.as_tensor(ppr.reshape(3, -1).astype(np.float32), device="cuda")
+    P = NufftPlan(M, 1e-6)
+    P.set_modes(torch.as_tensor(rng.random((M, M, M)).astype(np.float32), device="cuda"))
+    mult = np.pi / pdr.max()
+    bf = [torch.empty(n, p.shape[1], dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    a = P.slice(q, p, mult, out_bf16=bf[0])
+    b = P.slice(q, p, mult, out_bf16=bf[1], det_shape=det)
+    assert torch.equal(a, b)
+    assert torch.equal(bf[0], bf[1])
+
+
 @pytest.mark.parametrize("m", [(9, 8, 7), (5, 12, 21), (16, 3, 2)])
 @pytest.mark.parametrize("isign", [1, -1])
 @pytest.mark.parametrize("eps", [1e-6, 1e-12])
