@@ -59,7 +59,8 @@ struct spf_merge_s {
   float *modes = nullptr;      // M^3 (direct form input / output)
   float *t1_out = nullptr;     // M^3
   double *r = nullptr, *p = nullptr, *q = nullptr;
-  double *partial = nullptr;   // reduction scratch
+  double *partial = nullptr;   // reduction scratch: p.q, b.b
+  double *rr_partial = nullptr;  // r.r
   double *scal = nullptr;      // device scalars
   int *flags = nullptr;        // [0] done, [1] iterations
   cufftHandle r2c_L = 0, c2r_L = 0, r2c_M = 0, c2r_M = 0;
@@ -84,6 +85,8 @@ struct spf_merge_s {
   int det[3] = {0, 0, 0};
   bool sorted = false;
   double coord_scale = 0;
+  cudaStream_t side = nullptr;       // the Toeplitz product's stream
+  cudaEvent_t fork = nullptr, join = nullptr;
   struct Sweep *sweep = nullptr;  // batched buffers of spf_merge_cg_sweep
 };
 
@@ -164,43 +167,43 @@ __global__ void k_cg_init(const double *partial, double rtol, double *scal, int 
   }
 }
 
-// stage 1: rho = r.r, convergence test, beta
-__global__ void k_cg_stage1(const double *partial, int it, double *scal, int *flags,
-                            double *hist) {
-  double rho = sum_partials(partial);
+// rho = r.r from its partials, convergence test, beta = rho / last rho; then
+// p = r + beta p and the operator inputs (S . p in FP32) for both forms.
+// Every CTA adds up the partials itself (in the one order, so with the same
+// bits), which costs less than kernels between the vector passes: an iteration at
+// M = 41 takes 228 us and took 237.  One thread
+// takes the root and the quotient (an FP64 instruction costs a warp 64 clocks;
+// in all threads of 8 CTAs an SM they took 12 us).  CTA 0 keeps rho and the
+// done flag; the others may read the flag before or after it is set, with the
+// same outcome: they make the same test.
+__global__ void __launch_bounds__(RED_THREADS)
+    k_cg_update_p(double *__restrict__ p, const double *__restrict__ r,
+                  const double *__restrict__ rr_partial, int it, double *__restrict__ scal,
+                  volatile int *flags, double *__restrict__ hist, const float *__restrict__ S,
+                  int M, int L, float *__restrict__ conv_in, double *__restrict__ conv_in64,
+                  double *__restrict__ reg_in, float *__restrict__ modes) {
+  __shared__ double beta_s;
+  __shared__ bool done_s;
+  const double rho = sum_partials(rr_partial);
   if (threadIdx.x == 0) {
-    if (hist) hist[it] = sqrt(rho);
-    if (!flags[0]) {
-      if (sqrt(rho) < scal[S_ATOL]) {
+    const double norm = sqrt(rho);
+    const bool stop = flags[0] != 0 || norm < scal[S_ATOL];
+    done_s = stop;
+    beta_s = it > 0 ? rho / scal[S_RHO_PREV] : 0.0;
+    if (blockIdx.x == 0) {
+      if (hist) hist[it] = norm;
+      if (stop)
         flags[0] = 1;
-      } else {
+      else
         scal[S_RHO] = rho;
-        scal[S_BETA] = it > 0 ? rho / scal[S_RHO_PREV] : 0.0;
-      }
     }
   }
-}
-
-// stage 2: alpha = rho / p.q
-__global__ void k_cg_stage2(const double *partial, double *scal, const int *flags) {
-  double pq = sum_partials(partial);
-  if (threadIdx.x == 0 && !flags[0]) {
-    scal[S_PQ] = pq;
-    scal[S_ALPHA] = scal[S_RHO] / pq;
-    scal[S_RHO_PREV] = scal[S_RHO];
-  }
-}
-
-// p = r + beta p; operator inputs (S . p in FP32) for both forms
-__global__ void k_cg_update_p(double *__restrict__ p, const double *__restrict__ r,
-                              const double *__restrict__ scal, const int *__restrict__ flags,
-                              const float *__restrict__ S, int M, int L, float *__restrict__ conv_in,
-                              double *__restrict__ conv_in64, double *__restrict__ reg_in,
-                              float *__restrict__ modes) {
-  const bool done = flags[0] != 0;
-  const double beta = scal[S_BETA];
+  __syncthreads();
+  const bool done = done_s;
+  const double beta = beta_s;
   const int64_t n = (int64_t)M * M * M;
   const int h = M / 2;
+#pragma unroll 4
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     double pv = p[i];
@@ -272,6 +275,7 @@ __global__ void __launch_bounds__(RED_THREADS)
   const int h = M / 2;
   const double reg_scale = 1.0 / ((double)M * M * M);
   double s = 0.0;
+#pragma unroll 4
   for (int64_t i = blockIdx.x * (int64_t)RED_THREADS + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * RED_THREADS) {
     const unsigned iu = (unsigned)i;  // M^3 < 2^31 (M <= 1024)
@@ -291,18 +295,37 @@ __global__ void __launch_bounds__(RED_THREADS)
   if (partial && threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 
-__global__ void k_cg_update_xr(double *__restrict__ x, double *__restrict__ r,
-                               const double *__restrict__ p, const double *__restrict__ q,
-                               const double *__restrict__ scal, int *__restrict__ flags,
-                               int64_t n) {
-  if (flags[0]) return;
-  const double alpha = scal[S_ALPHA];
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
+// alpha = rho / p.q from its partials; x += alpha p, r -= alpha q, and the
+// partials of the new r.r (the grid, and so the order, of k_dot_partial)
+__global__ void __launch_bounds__(RED_THREADS)
+    k_cg_update_xr(double *__restrict__ x, double *__restrict__ r, const double *__restrict__ p,
+                   const double *__restrict__ q, const double *__restrict__ pq_partial,
+                   double *__restrict__ scal, int *__restrict__ flags, int64_t n,
+                   double *__restrict__ rr_partial) {
+  if (flags[0]) return;  // r and its partials stay
+  __shared__ double alpha_s;
+  const double rho = scal[S_RHO];
+  const double pq = sum_partials(pq_partial);
+  if (threadIdx.x == 0) alpha_s = rho / pq;
+  __syncthreads();
+  const double alpha = alpha_s;
+  double s = 0.0;
+#pragma unroll 4
+  for (int64_t i = blockIdx.x * (int64_t)RED_THREADS + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * RED_THREADS) {
     x[i] = fma(alpha, p[i], x[i]);
-    r[i] = fma(-alpha, q[i], r[i]);
+    const double v = fma(-alpha, q[i], r[i]);
+    r[i] = v;
+    s = fma(v, v, s);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) flags[1] += 1;
+  s = block_sum(s);
+  if (threadIdx.x == 0) {
+    rr_partial[blockIdx.x] = s;
+    if (blockIdx.x == 0) {
+      scal[S_RHO_PREV] = rho;
+      flags[1] += 1;
+    }
+  }
 }
 
 // r = b - q (q = W x0), or r = b when x0 is zero
@@ -390,9 +413,9 @@ static int cufft_ok(cufftResult r, const char *what) {
 
 static int grid1(int64_t n) { return grid_for(n, 256, (int64_t)sm_count() * 8); }
 
-// conv part of the operator from conv_in / reg_in / modes already loaded
-static int apply_operator_core(spf_merge_s *G, bool direct, cudaStream_t s) {
-  if (!direct && G->conv64) {
+// the Toeplitz product on the L grid
+static int conv_product(spf_merge_s *G, cudaStream_t s) {
+  if (G->conv64) {
     cufftSetStream(G->d2z_L, s);
     cufftSetStream(G->z2d_L, s);
     SPF_TRY(cufft_ok(cufftExecD2Z(G->d2z_L, G->conv_in64,
@@ -403,7 +426,7 @@ static int apply_operator_core(spf_merge_s *G, bool direct, cudaStream_t s) {
     SPF_TRY(cufft_ok(cufftExecZ2D(G->z2d_L, reinterpret_cast<cufftDoubleComplex *>(G->conv_freq64),
                                   G->conv_out64),
                      "conv Z2D"));
-  } else if (!direct) {
+  } else {
     cufftSetStream(G->r2c_L, s);
     cufftSetStream(G->c2r_L, s);
     SPF_TRY(cufft_ok(cufftExecR2C(G->r2c_L, G->conv_in, reinterpret_cast<cufftComplex *>(G->conv_freq)),
@@ -412,7 +435,13 @@ static int apply_operator_core(spf_merge_s *G, bool direct, cudaStream_t s) {
     SPF_TRY(check_launch("k_mul_real"));
     SPF_TRY(cufft_ok(cufftExecC2R(G->c2r_L, reinterpret_cast<cufftComplex *>(G->conv_freq), G->conv_out),
                      "conv C2R"));
-  } else {
+  }
+  return SPF_OK;
+}
+
+// the direct form's data term, and the regulariser
+static int direct_and_filter(spf_merge_s *G, bool direct, cudaStream_t s) {
+  if (direct) {
     SPF_TRY(spf_nufft_t2_set_modes(G->nufft, G->modes, nullptr, -1, 0, s));
     SPF_TRY(spf_nufft_t1_zero(G->nufft, s));
     if (G->sorted)
@@ -438,6 +467,27 @@ static int apply_operator_core(spf_merge_s *G, bool direct, cudaStream_t s) {
                   "reg Z2D");
 }
 
+// The operator from conv_in / reg_in / modes already loaded.  The
+// Toeplitz product (bound by memory) and the regulariser (by the FP64 pipe)
+// are independent: the product runs on the operator's own stream, whose
+// priority lets its CTAs in between the regulariser's, joined at both ends.
+// An iteration at M = 81: 346 us one after the other, 275 overlapped; at M =
+// 111 1,173 and 1,072; at M = 41, where launches dominate, 228 and 224.
+static int apply_operator_core(spf_merge_s *G, bool direct, cudaStream_t s) {
+  if (!direct) {
+    SPF_TRY(check_cuda(cudaEventRecord(G->fork, s), "merge operator"));
+    SPF_TRY(check_cuda(cudaStreamWaitEvent(G->side, G->fork, 0), "merge operator"));
+    const int st = conv_product(G, G->side);
+    SPF_TRY(check_cuda(cudaEventRecord(G->join, G->side), "merge operator"));
+    if (st != SPF_OK) {
+      cudaStreamWaitEvent(s, G->join, 0);
+      return st;
+    }
+  }
+  const int st = direct_and_filter(G, direct, s);
+  if (!direct) SPF_TRY(check_cuda(cudaStreamWaitEvent(s, G->join, 0), "merge operator"));
+  return st;
+}
 }  // namespace cg
 }  // namespace spf
 
@@ -490,7 +540,18 @@ int spf_merge_create(int M, int M_ups, double rlambda, double flambda, const flo
   alloc((void **)&G->r, G->n * sizeof(double));
   alloc((void **)&G->p, G->n * sizeof(double));
   alloc((void **)&G->q, G->n * sizeof(double));
-  alloc((void **)&G->partial, RED_BLOCKS * sizeof(double));
+  alloc((void **)&G->partial, 2 * RED_BLOCKS * sizeof(double));
+  G->rr_partial = G->partial + RED_BLOCKS;
+  if (st == SPF_OK) {
+    int least = 0, greatest = 0;
+    cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    st = check_cuda(cudaStreamCreateWithPriority(&G->side, cudaStreamNonBlocking, greatest),
+                    "spf_merge_create");
+  }
+  if (st == SPF_OK)
+    st = check_cuda(cudaEventCreateWithFlags(&G->fork, cudaEventDisableTiming), "spf_merge_create");
+  if (st == SPF_OK)
+    st = check_cuda(cudaEventCreateWithFlags(&G->join, cudaEventDisableTiming), "spf_merge_create");
   alloc((void **)&G->scal, S_COUNT * sizeof(double));
   alloc((void **)&G->flags, 2 * sizeof(int));
   if (st == SPF_OK) {
@@ -538,6 +599,9 @@ int spf_merge_destroy(spf_merge_s *G) {
                   G->r, G->p, G->q, G->partial, G->scal, G->flags, G->mask_full,
                   G->kernel_hat64, G->conv_in64, G->conv_freq64, G->conv_out64};
   for (void *b : bufs) cudaFree(b);
+  if (G->fork) cudaEventDestroy(G->fork);
+  if (G->join) cudaEventDestroy(G->join);
+  if (G->side) cudaStreamDestroy(G->side);
   free_sweep(G->sweep);
   prime_dft_free(G->pd);
   if (G->plans_ok) {
@@ -696,15 +760,13 @@ int spf_merge_cg(spf_merge_s *G, int form, const double *d_b, double *d_x, int x
   k_cg_init<<<1, RED_THREADS, 0, s>>>(G->partial, rtol, G->scal, G->flags);
   SPF_TRY(check_launch("k_cg_init"));
   SPF_TRY(check_cuda(cudaMemsetAsync(G->p, 0, n * sizeof(double), s), "spf_merge_cg"));
+  k_dot_partial<<<RED_BLOCKS, RED_THREADS, 0, s>>>(G->r, G->r, n, G->rr_partial);
+  SPF_TRY(check_launch("k_dot_partial"));
   for (int it = 0; it < maxiter; ++it) {
-    k_dot_partial<<<RED_BLOCKS, RED_THREADS, 0, s>>>(G->r, G->r, n, G->partial);
-    SPF_TRY(check_launch("k_dot_partial"));
-    k_cg_stage1<<<1, RED_THREADS, 0, s>>>(G->partial, it, G->scal, G->flags, d_hist);
-    SPF_TRY(check_launch("k_cg_stage1"));
-    k_cg_update_p<<<grid1(n), 256, 0, s>>>(G->p, G->r, G->scal, G->flags, G->support, G->M, G->L,
-                                           (direct || c64) ? nullptr : G->conv_in,
-                                           c64 ? G->conv_in64 : nullptr, G->reg_in,
-                                           direct ? G->modes : nullptr);
+    k_cg_update_p<<<RED_BLOCKS, RED_THREADS, 0, s>>>(
+        G->p, G->r, G->rr_partial, it, G->scal, G->flags, d_hist, G->support, G->M, G->L,
+        (direct || c64) ? nullptr : G->conv_in, c64 ? G->conv_in64 : nullptr, G->reg_in,
+        direct ? G->modes : nullptr);
     SPF_TRY(check_launch("k_cg_update_p"));
     SPF_TRY(apply_operator_core(G, direct, s));
     k_assemble<<<RED_BLOCKS, RED_THREADS, 0, s>>>(
@@ -713,9 +775,8 @@ int spf_merge_cg(spf_merge_s *G, int form, const double *d_b, double *d_x, int x
         direct ? G->direct_scale : G->conv_scale, G->reg_out, G->rlambda, G->flambda, G->q,
         G->partial);
     SPF_TRY(check_launch("k_assemble"));
-    k_cg_stage2<<<1, RED_THREADS, 0, s>>>(G->partial, G->scal, G->flags);
-    SPF_TRY(check_launch("k_cg_stage2"));
-    k_cg_update_xr<<<grid1(n), 256, 0, s>>>(d_x, G->r, G->p, G->q, G->scal, G->flags, n);
+    k_cg_update_xr<<<RED_BLOCKS, RED_THREADS, 0, s>>>(d_x, G->r, G->p, G->q, G->partial, G->scal,
+                                                      G->flags, n, G->rr_partial);
     SPF_TRY(check_launch("k_cg_update_xr"));
   }
   if (d_iters_out)
