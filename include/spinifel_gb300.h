@@ -45,6 +45,13 @@ const char *spf_last_error(void);
 uint64_t spf_launch_count(void);
 /* Device-side error word written by bounded waits (0 = none); reset to 0. */
 int spf_device_error(void *stream, int *h_code);
+
+/* d_out[0..2] (device) = the largest magnitude in each of three arrays of n
+ * values, floats or (fp64) doubles; NaN for an array that holds one.  The
+ * range check of the NUFFT operators (autocorrelation.py:36-37 compares every
+ * coordinate with 3 pi). */
+int spf_max_abs3(const void *d_x, const void *d_y, const void *d_z, int64_t n, int fp64,
+                 double *d_out, void *stream);
 /* Self-test of the bounded-wait path used by the tensor-core kernels: one
  * thread waits on an mbarrier that nothing completes, gives up after
  * timeout_ms (1..5000), records -SPF_ERR_TIMEOUT in the device error word and

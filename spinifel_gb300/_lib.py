@@ -51,6 +51,7 @@ SIGNATURES = {
     "spf_status_string": [_int],
     "spf_last_error": [],
     "spf_launch_count": [],
+    "spf_max_abs3": [_c_void_p, _c_void_p, _c_void_p, _i64, _int, _c_void_p, _c_void_p],
     "spf_device_error": [_c_void_p, ctypes.POINTER(_int)],
     "spf_selftest_bounded_wait": [_i64, _c_void_p, _c_void_p],
     "spf_tune_set": [_int, _i64],

@@ -16,8 +16,8 @@ from __future__ import annotations
 import numpy as np
 import torch
 
-from . import _arrays, geom
-from .nufft import NufftPlan, make_plan
+from . import _arrays, _lib, geom
+from .nufft import FP32_EPS_FLOOR, NufftPlan, make_plan
 
 DEFAULT_EPS = 1e-6
 _plans: dict = {}
@@ -33,11 +33,28 @@ def plan_for(M, eps=DEFAULT_EPS) -> NufftPlan:
     return p
 
 
+def _dtype(eps) -> torch.dtype:
+    """Device type of the plan for eps: converting to it at once gives what
+    converting through FP64 gives."""
+    return torch.float32 if float(eps) >= FP32_EPS_FLOOR else torch.float64
+
+
 def _numel(a) -> int:
     return a.numel() if _arrays.is_torch(a) else int(np.size(a))
 
 
 def _max_abs(*arrs) -> float:
+    a = arrs[0]
+    if len(arrs) == 3 and all(_arrays.is_torch(t) and t.is_cuda and t.is_contiguous()
+                              and t.dtype == a.dtype and t.device == a.device
+                              and t.numel() == a.numel() for t in arrs) \
+            and a.dtype in (torch.float32, torch.float64) \
+            and a.device.index == torch.cuda.current_device():
+        # one pass over the three arrays and one readback
+        out = torch.empty(3, dtype=torch.float64, device=a.device)
+        _lib.call("spf_max_abs3", *(_lib.ptr(t) for t in arrs), a.numel(),
+                  int(a.dtype == torch.float64), _lib.ptr(out), _lib.stream_handle())
+        return max(out.tolist())
     return max(float(a.abs().max()) if _arrays.is_torch(a) else float(np.max(np.abs(a)))
                for a in arrs)
 
@@ -53,11 +70,11 @@ def forward(ugrid, H_, K_, L_, support, use_recip_sym, N, eps=DEFAULT_EPS):
             assert np.all(np.isreal(ugrid))
     g = _arrays.to_dev(ugrid.real if _arrays.is_torch(ugrid) and torch.is_complex(ugrid)
                        else (np.real(ugrid) if not _arrays.is_torch(ugrid) else ugrid),
-                       torch.float64)
+                       _dtype(eps))
     P = plan_for(g.shape, eps)
     P.set_modes(g, support, isign=-1, want_imag=True)
     x, y, z = (_arrays.to_dev(np.asarray(a).reshape(-1) if not _arrays.is_torch(a) else a,
-                              torch.float64) for a in (H_, K_, L_))
+                              P.dtype) for a in (H_, K_, L_))
     re, im = P.interp(x, y, z, want_imag=True)
     out = torch.complex(re, im)
     assert out.numel() == N

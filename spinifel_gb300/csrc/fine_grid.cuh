@@ -74,11 +74,13 @@ __global__ void k_modes_to_grid(const T *__restrict__ f, const T *__restrict__ s
   }
 }
 
-// re[i] = Re F[(i - off) mod n] (and im = im_sign Im F) for every padded cell
+// re[i] = Re F[(i - off) mod n] for every padded cell, and where asked for
+// im = im_sign Im F or the pairs (re, im)
 template <class T>
 __global__ void k_spectrum_to_padded(const typename Complex<T>::type *__restrict__ half,
                                      GridDims g, T im_sign, T *__restrict__ re,
-                                     T *__restrict__ im) {
+                                     T *__restrict__ im,
+                                     typename Complex<T>::type *__restrict__ cx) {
   const int64_t row = (int64_t)blockIdx.x * ROWS_PER_CTA + threadIdx.y;
   if (row >= (int64_t)g.p1 * g.p2) return;
   const int nh = g.n3 / 2 + 1;
@@ -93,7 +95,14 @@ __global__ void k_spectrum_to_padded(const typename Complex<T>::type *__restrict
     const bool direct = c < nh;
     const auto v = direct ? h[c] : hm[g.n3 - c];
     re[row * g.p3 + k] = v.x;
-    if (im) im[row * g.p3 + k] = direct ? im_sign * v.y : -im_sign * v.y;
+    const T y = direct ? im_sign * v.y : -im_sign * v.y;
+    if (im) im[row * g.p3 + k] = y;
+    if (cx) {
+      typename Complex<T>::type q;
+      q.x = v.x;
+      q.y = y;
+      cx[row * g.p3 + k] = q;
+    }
   }
 }
 

@@ -353,7 +353,8 @@ int spf_nufft64_t2_set_modes(spf_nufft64_plan P, const double *d_modes, const do
   SPF_TRY(check_launch("k_modes_to_grid"));
   SPF_TRY(fft_exec(P, s, "spf_nufft64_t2_set_modes"));
   k_spectrum_to_padded<double><<<row_grid((int64_t)g.p1 * g.p2), row_block(), 0, s>>>(
-      P->half, g, isign < 0 ? double(1) : double(-1), P->re_pad, want_imag ? P->im_pad : nullptr);
+      P->half, g, isign < 0 ? double(1) : double(-1), P->re_pad,
+      want_imag ? P->im_pad : nullptr, nullptr);
   return check_launch("k_spectrum_to_padded");
 }
 

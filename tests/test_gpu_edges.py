@@ -244,3 +244,42 @@ def test_real_transforms_against_direct_sums(m, isign, eps):
     want = onufft.nudft3d1(x.astype(float), y.astype(float), z.astype(float), c.astype(float), m,
                            isign)
     assert np.linalg.norm(got - want) < tol * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("n", [1, 31, 257, 1024, 100003])
+def test_max_abs_equals_torch(dtype, n):
+    """The range check's one-pass maximum is torch's, whichever array and
+    sign holds it, and treats NaN and infinity as the maxima of torch do."""
+    from spinifel_gb300 import autocorrelation as ac
+
+    rng = np.random.default_rng(n)
+    for where in range(3):
+        v = [torch.as_tensor(rng.standard_normal(n), device="cuda", dtype=dtype)
+             for _ in range(3)]
+        v[where][n // 2] = -7.5
+        assert ac._max_abs(*v) == 7.5
+        for bad in (float("inf"), float("-inf"), float("nan")):
+            v[where][n - 1] = bad
+            want = max(float(t.abs().max()) for t in v)
+            got = ac._max_abs(*v)
+            assert got == want or (np.isnan(got) and np.isnan(want))
+    assert ac._max_abs(*(torch.zeros(n, device="cuda", dtype=dtype) for _ in range(3))) == 0.0
+
+
+def test_interp_pairs_equal_single_parts():
+    """Both parts from one walk over the footprint: the real part has the bits
+    of the walk over the real grid, also after a model without the imaginary
+    part was set."""
+    from spinifel_gb300.nufft import NufftPlan
+
+    rng = np.random.default_rng(3)
+    P = NufftPlan((11, 14, 9), 1e-6)
+    x, y, z = (torch.as_tensor(rng.uniform(-3, 3, 501).astype(np.float32), device="cuda")
+               for _ in range(3))
+    for want_imag in (True, False):
+        f = torch.as_tensor(rng.standard_normal((11, 14, 9)).astype(np.float32), device="cuda")
+        P.set_modes(f, want_imag=want_imag)
+        re, im = P.interp(x, y, z, want_imag=True)
+        assert torch.equal(re, P.interp(x, y, z)[0])
+        assert bool(torch.isfinite(im).all())
