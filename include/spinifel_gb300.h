@@ -252,6 +252,12 @@ int spf_nufft64_t2_interp(spf_nufft64_plan plan, const double *d_x, const double
 int spf_slice_t2_f64(spf_nufft64_plan plan, const double *d_quats, int64_t n_orient,
                      const double *d_ppr, int64_t n_pix, double scale, double *d_out,
                      void *stream);
+/* The same on a detector of n_panels x nx x ny pixels (n_pix in that order):
+ * for kernel widths up to 13 the sums run over pairs of floats, accurate to
+ * about 2^-46, from footprint boxes staged in shared memory. */
+int spf_slice_t2_f64_det(spf_nufft64_plan plan, const double *d_quats, int64_t n_orient,
+                         const double *d_ppr, int n_panels, int nx, int ny, double scale,
+                         double *d_out, void *stream);
 /* Type 1 in FP64: zero (allocates the accumulator on first use), spread real
  * strengths at explicit points, fold + FFT + deconvolve onto the modes
  * (NUFFT.adjoint before the support multiply and 1/M^3,

@@ -168,6 +168,8 @@ SIGNATURES = {
     "spf_nufft64_t2_set_modes": [_c_void_p, _c_void_p, _c_void_p, _int, _int, _c_void_p],
     "spf_nufft64_t2_interp": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _i64, _c_void_p,
                               _c_void_p, _c_void_p],
+    "spf_slice_t2_f64_det": [_c_void_p, _c_void_p, _i64, _c_void_p, _int, _int, _int, _dbl,
+                             _c_void_p, _c_void_p],
     "spf_slice_t2_f64": [_c_void_p, _c_void_p, _i64, _c_void_p, _i64, _dbl, _c_void_p,
                          _c_void_p],
     "spf_nufft64_t1_zero": [_c_void_p, _c_void_p],

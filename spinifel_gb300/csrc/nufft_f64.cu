@@ -12,7 +12,7 @@
 // Points (radians) map to fine-grid coordinate t = x n / (2 pi), wrapped into
 // [-n/2, n/2); the footprint is l0 .. l0+w-1 with l0 = ceil(t - w/2).
 //
-// GB300 runs FP64 at about 1/64 of its FP32 rate, so these kernels are
+// GB300 runs FP64 at about 1/64 of its FP32 rate, so the FP64 kernels are
 // bound by the FP64 pipe (W^3 FMAs per point); the grid (tens of MB) stays
 // in L2 and is read through L1 without shared-memory staging.
 #include <cufft.h>
@@ -38,6 +38,11 @@ struct spf_nufft64_plan_s {
   double *re_pad = nullptr;
   double *im_pad = nullptr;
   double *acc_pad = nullptr;
+  // slicing by pairs of floats (w <= PAIR_MAX_W): the padded grid over a power
+  // of two as (high, low) pairs, that power, exp at the table's points
+  float2 *pair_pad = nullptr;
+  unsigned long long *peak = nullptr;  // bits of max |re_pad|
+  float2 *exp_table = nullptr;
   cufftHandle fft = 0;
   bool fft_ok = false;
 };
@@ -141,18 +146,276 @@ __global__ void __launch_bounds__(128)
   }
 }
 
+// 2^-(e + 1) for max |v| in [2^e, 2^(e + 1)), and whether pairs of floats can
+// hold the grid (finite and not all below the normal doubles)
+__device__ __forceinline__ bool pair_scale(unsigned long long peak, double &down, double &up) {
+  const int e = (int)(peak >> 52);  // biased exponent
+  if (e >= 2046 || e < 1) return false;
+  down = __longlong_as_double((long long)(2045 - e) << 52);  // 2^(1022 - e)
+  up = __longlong_as_double((long long)(e + 1) << 52);       // 2^(e - 1022)
+  return e <= 2044;
+}
+
 // Slicing: point (o, p) = scale * R(q_o)^-1 ppr[:, p]; out[o * n_pix + p] = Re c.
 template <int W>
 __global__ void __launch_bounds__(128)
     k_slice(const double *__restrict__ re_pad, Geom g, const double *__restrict__ quats,
             const double *__restrict__ ppr, int64_t n_pix, double s1, double s2, double s3,
-            double *__restrict__ out) {
+            double *__restrict__ out, const unsigned long long *__restrict__ peak) {
+  double down, up;
+  if (peak && pair_scale(*peak, down, up)) return;  // k_slice_pairs has it
   const int64_t o = blockIdx.x;
   const int64_t p = blockIdx.y * (int64_t)blockDim.x + threadIdx.x;
   if (p >= n_pix) return;
   double h, k, l;
   rotate_inv(quats + 4 * o, ppr[p], ppr[n_pix + p], ppr[2 * n_pix + p], h, k, l);
   out[o * n_pix + p] = interp_point<W>(re_pad, g, h, s1, k, s2, l, s3);
+}
+
+// ---------------------------------------------------------------------------
+// Slicing with pairs of floats
+//
+// A warp's FP64 instruction holds its quarter of the SM for 64 clocks, so the
+// W^3 FMAs and 3 W kernel values of a point (39 exponentials and roots at
+// eps 1e-12, about as dear as 1,500 FMAs) take 2.66 ms for 409,600 points.
+// The same sums over unevaluated pairs of floats (error-free products and
+// sums: Dekker 1971, Knuth TAOCP 2, 4.2.2) take twelve FP32 instructions a
+// term and are good to about 2^-46 of the terms' magnitudes, far below the
+// interpolation error of a kernel of W <= 13 (4.8e-13 against the direct sums
+// at W = 13, before and now); wider kernels resolve less than that and stay
+// in FP64.  409,600 points at 41^3 take 0.83 ms (2.69 in FP64 throughout),
+// 262,144 at 81^3 on 4 x 128 x 128 pixels 0.53 (1.72).
+//
+// A CTA takes a 4 x 8 pixel patch of one panel at one orientation: three
+// warps compute its grid coordinates in FP64 (one axis each), all eight the
+// kernel values, then the box of the footprints is staged in shared memory
+// and each warp sums every eighth of the W^2 footprint rows for the 32 pixels.
+// The grid is scaled by a power of two to at most 1, so that the low halves
+// stay in FP32's range.
+// ---------------------------------------------------------------------------
+constexpr int PAIR_MAX_W = 13;
+constexpr int PAIR_PX = 4, PAIR_PY = 8, PAIR_PIX = 32, PAIR_WARPS = 8;
+constexpr int PAIR_CELLS = 10240;    // 80 KB: two CTAs an SM
+constexpr int EXP_PER_UNIT = 32;     // exp(-j / 32) in the table
+
+struct Pair {
+  float h, l;
+};
+__device__ __forceinline__ Pair two_sum(float a, float b) {
+  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+  return Pair{s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t))};
+}
+__device__ __forceinline__ Pair fast_two_sum(float a, float b) {  // |a| >= |b|
+  const float s = __fadd_rn(a, b);
+  return Pair{s, __fsub_rn(b, __fsub_rn(s, a))};
+}
+__device__ __forceinline__ Pair mul(Pair a, Pair b) {
+  const float p = __fmul_rn(a.h, b.h);
+  float e = __fmaf_rn(a.h, b.h, -p);
+  e = __fmaf_rn(a.h, b.l, e);
+  e = __fmaf_rn(a.l, b.h, e);
+  return fast_two_sum(p, e);
+}
+__device__ __forceinline__ Pair add(Pair a, float b) {
+  const Pair s = two_sum(a.h, b);
+  return fast_two_sum(s.h, __fadd_rn(s.l, a.l));
+}
+
+// sum of products: h + l; the terms' errors collect in l
+__device__ __forceinline__ void accumulate(Pair &acc, float wh, float wl, float gh, float gl) {
+  const float p = __fmul_rn(wh, gh);
+  float l = __fadd_rn(acc.l, __fmaf_rn(wh, gh, -p));
+  l = __fmaf_rn(wh, gl, l);
+  l = __fmaf_rn(wl, gh, l);
+  const Pair s = two_sum(acc.h, p);
+  acc.h = s.h;
+  acc.l = __fadd_rn(l, s.l);
+}
+
+// exp(beta (sqrt(1 - z^2) - 1)), z = (f + a) / half_w, by exp(x) = T[j] exp(t),
+// x = -j / 32 + t, and the Taylor polynomial of exp(t) - 1 (|t| <= 1/64)
+__device__ __forceinline__ Pair es_pair(Pair f, int a, Pair inv_half_w, Pair beta,
+                                        const float2 *__restrict__ table, int table_last) {
+  const Pair z = mul(add(f, (float)a), inv_half_w);
+  const Pair z2 = mul(z, z);
+  Pair q = two_sum(1.0f, -z2.h);
+  q = fast_two_sum(q.h, __fsub_rn(q.l, z2.l));
+  if (!(q.h > 0.0f)) q = Pair{0.0f, 0.0f};
+  const float root = __fsqrt_rn(q.h);
+  const float rest = __fadd_rn(__fmaf_rn(-root, root, q.h), q.l);
+  const Pair r{root, root > 0.0f ? __fdividef(0.5f * rest, root) : 0.0f};
+  const Pair x = mul(add(r, -1.0f), beta);  // -beta .. 0
+  const int j = min(max(__float2int_rn(-EXP_PER_UNIT * x.h), 0), table_last);
+  const float2 T = __ldg(table + j);
+  const Pair t = fast_two_sum(__fadd_rn(x.h, (float)j * (1.0f / EXP_PER_UNIT)), x.l);
+  const float p = __fmul_rn(t.h, t.h);
+  const float pe = __fmaf_rn(2.0f * t.h, t.l, __fmaf_rn(t.h, t.h, -p));
+  const float cube = p * t.h * fmaf(t.h, fmaf(t.h, 1.0f / 120.0f, 1.0f / 24.0f), 1.0f / 6.0f);
+  Pair u = two_sum(t.h, 0.5f * p);
+  u = fast_two_sum(u.h, __fadd_rn(__fadd_rn(u.l, t.l), __fmaf_rn(0.5f, pe, cube)));
+  const Pair Tu = mul(Pair{T.x, T.y}, u);
+  const Pair w = two_sum(T.x, Tu.h);
+  return fast_two_sum(w.h, __fadd_rn(w.l, __fadd_rn(T.y, Tu.l)));
+}
+
+// bits of max |v| (NaN above infinity above all values)
+__global__ void __launch_bounds__(256)
+    k_peak(const double *__restrict__ v, int64_t n, unsigned long long *__restrict__ peak) {
+  unsigned long long m = 0;
+#pragma unroll 4
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v[i]) & ~(1ULL << 63);
+    m = b > m ? b : m;
+  }
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    const unsigned long long u = __shfl_xor_sync(0xffffffffu, m, o);
+    m = u > m ? u : m;
+  }
+  if ((threadIdx.x & 31) == 0) atomicMax(peak, m);
+}
+
+__global__ void k_to_pairs(const double *__restrict__ v, int64_t n,
+                           const unsigned long long *__restrict__ peak,
+                           float2 *__restrict__ out) {
+  double down, up;
+  if (!pair_scale(*peak, down, up)) return;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const double x = v[i] * down;
+    const float h = (float)x;
+    out[i] = make_float2(h, (float)(x - (double)h));
+  }
+}
+
+template <int W>
+__global__ void __launch_bounds__(PAIR_WARPS * 32, 2)
+    k_slice_pairs(const float2 *__restrict__ grid, const unsigned long long *__restrict__ peak,
+                  Geom g, const double *__restrict__ quats, const double *__restrict__ ppr,
+                  int n_panels, int nx, int ny, double s1, double s2, double s3, Pair inv_half_w,
+                  Pair beta, const float2 *__restrict__ exp_table, int table_last,
+                  double *__restrict__ out) {
+  extern __shared__ __align__(16) float2 box[];  // PAIR_CELLS
+  __shared__ float2 wts[3 * W][PAIR_PIX];
+  __shared__ double part[PAIR_WARPS][PAIR_PIX];
+  __shared__ float2 frac[3][PAIR_PIX];
+  __shared__ int first[3][PAIR_PIX], lo[3], hi[3];
+  double down, up;
+  if (!pair_scale(*peak, down, up)) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t o = blockIdx.x;
+  const int patches_y = (ny + PAIR_PY - 1) / PAIR_PY, patches_x = (nx + PAIR_PX - 1) / PAIR_PX;
+  const int panel = blockIdx.y / (patches_x * patches_y), rem = blockIdx.y % (patches_x * patches_y);
+  // pixels past the panel's edge repeat its last row or column
+  const int px = (rem / patches_y) * PAIR_PX + lane / PAIR_PY,
+            py = (rem % patches_y) * PAIR_PY + lane % PAIR_PY;
+  const bool valid = px < nx && py < ny;
+  const int64_t n_pix = (int64_t)n_panels * nx * ny;
+  const int64_t p = ((int64_t)panel * nx + min(px, nx - 1)) * ny + min(py, ny - 1);
+  if (warp < 3) {
+    double h, k, l;
+    rotate_inv(quats + 4 * o, ppr[p], ppr[n_pix + p], ppr[2 * n_pix + p], h, k, l);
+    const int n = warp == 0 ? g.n1 : warp == 1 ? g.n2 : g.n3;
+    const int off = warp == 0 ? g.off1 : warp == 1 ? g.off2 : g.off3;
+    const double x = warp == 0 ? h : warp == 1 ? k : l, s = warp == 0 ? s1 : warp == 1 ? s2 : s3;
+    // the cell of axis_setup, operation by operation
+    const double fn = (double)n;
+    double t = __dmul_rn(x, s);
+    t = __dsub_rn(t, __dmul_rn(fn, floor(__dadd_rn(__ddiv_rn(t, fn), 0.5))));
+    const double l0 = ceil(__dsub_rn(t, 0.5 * W));
+    const double f = __dsub_rn(l0, t);
+    const float fh = (float)f;
+    frac[warp][lane] = make_float2(fh, (float)(f - (double)fh));
+    const int i0 = (int)l0 + off;
+    first[warp][lane] = i0;
+    const int a = __reduce_min_sync(0xffffffffu, i0), b = __reduce_max_sync(0xffffffffu, i0);
+    if (lane == 0) {
+      lo[warp] = a;
+      hi[warp] = b + W;
+    }
+  }
+  __syncthreads();
+  // the box from an even cell on: rows of the padded grid (even length) and of
+  // the box start on 16 bytes, and half a warp copies a row, 16 bytes a lane
+  const int i0 = lo[0], j0 = lo[1], k0 = lo[2] & ~1;
+  const int di = hi[0] - i0, dj = hi[1] - j0, dk = (hi[2] - k0 + 1) & ~1;
+  const int sk = dk | 2, sj = dj | 1;  // strides that spread rows over the banks
+  const bool staged = (int64_t)di * sj * sk <= PAIR_CELLS;
+  if (staged) {
+    constexpr int STEP = 2 * PAIR_WARPS;  // rows at a time
+    int jj = 2 * warp + (lane >> 4), ii = 0;
+    while (jj >= dj) {
+      jj -= dj;
+      ++ii;
+    }
+    const int c0 = 2 * (lane & 15);
+    const float2 *src = grid + ((size_t)i0 * g.p2 + j0) * g.p3 + k0 + c0;
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(box + c0);
+    while (ii < di) {
+      const float2 *row = src + (ii * g.p2 + jj) * g.p3;
+      const unsigned to = dst + (unsigned)((ii * sj + jj) * sk) * (unsigned)sizeof(float2);
+      for (int c = c0; c < dk; c += 32)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                         to + (unsigned)((c - c0) * sizeof(float2))),
+                     "l"(row + (c - c0))
+                     : "memory");
+      jj += STEP;
+      while (jj >= dj) {
+        jj -= dj;
+        ++ii;
+      }
+    }
+  }
+  // the kernel values while the box is on its way (plain loads, a
+  // warp a row, took most of the kernel: 1,297 us in all)
+  for (int e = warp; e < 3 * W; e += PAIR_WARPS) {
+    const float2 f = frac[e / W][lane];
+    const Pair w = es_pair(Pair{f.x, f.y}, e % W, inv_half_w, beta, exp_table, table_last);
+    wts[e][lane] = make_float2(w.h, w.l);
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  float2 w3[W];
+#pragma unroll
+  for (int c = 0; c < W; ++c) w3[c] = wts[2 * W + c][lane];
+  const int li = first[0][lane], lj = first[1][lane], lk = first[2][lane];
+  Pair sum{0.0f, 0.0f};
+  auto rows = [&](auto cell) {
+    for (int r = warp; r < W * W; r += PAIR_WARPS) {
+      const int a = r / W, b = r - a * W;
+      const auto row = cell(a, b);
+      Pair acc{0.0f, 0.0f};
+#pragma unroll
+      for (int c = 0; c < W; ++c) {
+        const float2 v = row(c);
+        accumulate(acc, w3[c].x, w3[c].y, v.x, v.y);
+      }
+      const float2 u = wts[a][lane], v = wts[W + b][lane];
+      const Pair w12 = mul(Pair{u.x, u.y}, Pair{v.x, v.y});
+      const Pair n = fast_two_sum(acc.h, acc.l);
+      accumulate(sum, w12.h, w12.l, n.h, n.l);
+    }
+  };
+  if (staged) {
+    const float2 *base = box + ((li - i0) * sj + (lj - j0)) * sk + (lk - k0);
+    rows([&](int a, int b) {
+      const float2 *row = base + (a * sj + b) * sk;
+      return [row](int c) { return row[c]; };
+    });
+  } else {
+    const float2 *base = grid + ((size_t)li * g.p2 + lj) * g.p3 + lk;
+    rows([&](int a, int b) {
+      const float2 *row = base + ((size_t)a * g.p2 + b) * g.p3;
+      return [row](int c) { return __ldg(row + c); };
+    });
+  }
+  part[warp][lane] = (double)sum.h + (double)sum.l;
+  __syncthreads();
+  if (warp != 0 || !valid) return;
+  double v = part[0][lane];
+  for (int q = 1; q < PAIR_WARPS; ++q) v += part[q][lane];
+  out[o * n_pix + p] = v * up;
 }
 
 template <int W>
@@ -275,6 +538,9 @@ int spf_nufft64_plan_create(int m1, int m2, int m3, double eps, double upsampfac
     P->n[d] = es_next_smooth_even(want);
     P->np[d] = P->n[d] + 2 * P->pad;
   }
+  // rows of the float-pair grid start on 16-byte boundaries; the extra cell is
+  // never inside a footprint
+  P->np[2] = (P->np[2] + 1) & ~1;
   int st = SPF_OK;
   const size_t nfine = (size_t)P->n[0] * P->n[1] * P->n[2];
   const size_t npad = (size_t)P->np[0] * P->np[1] * P->np[2];
@@ -319,6 +585,9 @@ int spf_nufft64_plan_destroy(spf_nufft64_plan P) {
   cudaFree(P->re_pad);
   cudaFree(P->im_pad);
   cudaFree(P->acc_pad);
+  cudaFree(P->pair_pad);
+  cudaFree(P->peak);
+  cudaFree(P->exp_table);
   if (P->fft_ok) cufftDestroy(P->fft);
   if (prev != P->dev && prev >= 0) cudaSetDevice(prev);
   delete P;
@@ -335,6 +604,45 @@ int spf_nufft64_plan_info(spf_nufft64_plan P, int *n_fine, int *width, double *b
   if (width) *width = P->w;
   if (beta) *beta = P->beta;
   return SPF_OK;
+}
+
+static Pair pair_of(double v) {
+  Pair p;
+  p.h = (float)v;
+  p.l = (float)(v - (double)p.h);
+  return p;
+}
+
+// the float-pair copy of the padded grid, part of setting a model (so that a
+// captured slicing reads the model set last)
+static int make_pairs(spf_nufft64_plan P, cudaStream_t s) {
+  const int64_t npad = (int64_t)P->np[0] * P->np[1] * P->np[2];
+  const char *what = "spf_nufft64_t2_set_modes";
+  if (!P->exp_table) {
+    const int n = (int)ceil(EXP_PER_UNIT * P->beta) + 2;
+    std::vector<float2> t(n);
+    for (int j = 0; j < n; ++j) {
+      const Pair p = pair_of(exp(-(double)j / EXP_PER_UNIT));
+      t[j] = make_float2(p.h, p.l);
+    }
+    float2 *d = nullptr;
+    SPF_TRY(check_cuda(cudaMalloc(&d, n * sizeof(float2)), what));
+    const int st = check_cuda(cudaMemcpy(d, t.data(), n * sizeof(float2), cudaMemcpyHostToDevice),
+                              what);
+    if (st != SPF_OK) {
+      cudaFree(d);
+      return st;
+    }
+    P->exp_table = d;
+  }
+  if (!P->peak) SPF_TRY(check_cuda(cudaMalloc(&P->peak, sizeof(*P->peak)), what));
+  if (!P->pair_pad) SPF_TRY(check_cuda(cudaMalloc(&P->pair_pad, npad * sizeof(float2)), what));
+  SPF_TRY(check_cuda(cudaMemsetAsync(P->peak, 0, sizeof(*P->peak), s), what));
+  k_peak<<<grid_for(npad, 1024, (int64_t)sm_count() * 8), 256, 0, s>>>(P->re_pad, npad, P->peak);
+  SPF_TRY(check_launch("k_peak"));
+  k_to_pairs<<<grid_for(npad, 256, (int64_t)sm_count() * 16), 256, 0, s>>>(P->re_pad, npad, P->peak,
+                                                                          P->pair_pad);
+  return check_launch("k_to_pairs");
 }
 
 int spf_nufft64_t2_set_modes(spf_nufft64_plan P, const double *d_modes, const double *d_support,
@@ -355,7 +663,8 @@ int spf_nufft64_t2_set_modes(spf_nufft64_plan P, const double *d_modes, const do
   k_spectrum_to_padded<double><<<row_grid((int64_t)g.p1 * g.p2), row_block(), 0, s>>>(
       P->half, g, isign < 0 ? double(1) : double(-1), P->re_pad,
       want_imag ? P->im_pad : nullptr, nullptr);
-  return check_launch("k_spectrum_to_padded");
+  SPF_TRY(check_launch("k_spectrum_to_padded"));
+  return P->w <= PAIR_MAX_W ? make_pairs(P, s) : SPF_OK;
 }
 
 int spf_nufft64_t2_interp(spf_nufft64_plan P, const double *d_x, const double *d_y,
@@ -375,6 +684,18 @@ int spf_nufft64_t2_interp(spf_nufft64_plan P, const double *d_x, const double *d
   return check_launch("k_interp (f64)");
 }
 
+static int slice_f64(spf_nufft64_plan P, const double *d_quats, int64_t n_orient,
+                     const double *d_ppr, int64_t n_pix, double scale, double *d_out,
+                     const unsigned long long *peak, cudaStream_t s) {
+  const Geom g = geom_of(P);
+  double sc[3];
+  grid_scales(P, scale, sc);
+  const dim3 grid((unsigned)n_orient, (unsigned)((n_pix + 127) / 128));
+  SPF_W64_DISPATCH(P->w, (k_slice<W><<<grid, 128, 0, s>>>(P->re_pad, g, d_quats, d_ppr, n_pix,
+                                                             sc[0], sc[1], sc[2], d_out, peak)));
+  return check_launch("k_slice (f64)");
+}
+
 int spf_slice_t2_f64(spf_nufft64_plan P, const double *d_quats, int64_t n_orient,
                      const double *d_ppr, int64_t n_pix, double scale, double *d_out,
                      void *stream) {
@@ -383,14 +704,59 @@ int spf_slice_t2_f64(spf_nufft64_plan P, const double *d_quats, int64_t n_orient
   if (n_orient == 0 || n_pix == 0) return SPF_OK;
   SPF_REQUIRE(d_quats && d_ppr && d_out, "spf_slice_t2_f64: NULL pointer");
   SPF_REQUIRE(n_orient < (1LL << 31) && n_pix <= 65535LL * 128, "spf_slice_t2_f64: size too large");
+  return slice_f64(P, d_quats, n_orient, d_ppr, n_pix, scale, d_out, nullptr, as_stream(stream));
+}
+
+int spf_slice_t2_f64_det(spf_nufft64_plan P, const double *d_quats, int64_t n_orient,
+                         const double *d_ppr, int n_panels, int nx, int ny, double scale,
+                         double *d_out, void *stream) {
+  SPF_TRY(check_plan(P, "spf_slice_t2_f64_det"));
+  SPF_REQUIRE(n_orient >= 0 && n_panels >= 0 && nx >= 0 && ny >= 0,
+              "spf_slice_t2_f64_det: negative size");
+  if (n_orient == 0 || n_panels == 0 || nx == 0 || ny == 0) return SPF_OK;
+  const int64_t patches =
+      (int64_t)n_panels * ((nx + PAIR_PX - 1) / PAIR_PX) * ((ny + PAIR_PY - 1) / PAIR_PY);
+  const int64_t n_pix = (int64_t)n_panels * nx * ny;
+  if (P->w > PAIR_MAX_W || patches > 65535)
+    return spf_slice_t2_f64(P, d_quats, n_orient, d_ppr, n_pix, scale, d_out, stream);
+  SPF_REQUIRE(d_quats && d_ppr && d_out, "spf_slice_t2_f64_det: NULL pointer");
+  SPF_REQUIRE(n_orient < (1LL << 31) && n_pix <= 65535LL * 128,
+              "spf_slice_t2_f64_det: size too large");
   cudaStream_t s = as_stream(stream);
+  SPF_REQUIRE(P->pair_pad != nullptr, "spf_slice_t2_f64_det: no model set");
   const Geom g = geom_of(P);
   double sc[3];
   grid_scales(P, scale, sc);
-  const dim3 grid((unsigned)n_orient, (unsigned)((n_pix + 127) / 128));
-  SPF_W64_DISPATCH(P->w, (k_slice<W><<<grid, 128, 0, s>>>(P->re_pad, g, d_quats, d_ppr, n_pix,
-                                                             sc[0], sc[1], sc[2], d_out)));
-  return check_launch("k_slice (f64)");
+  const dim3 grid((unsigned)n_orient, (unsigned)patches);
+  const int smem = PAIR_CELLS * (int)sizeof(float2);
+  const Pair ihw = pair_of(2.0 / P->w), beta = pair_of(P->beta);
+  const int last = (int)ceil(EXP_PER_UNIT * P->beta) + 1;
+#define SPF_PAIR_CASE(w_)                                                                        \
+  case w_:                                                                                       \
+    cudaFuncSetAttribute(k_slice_pairs<w_>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);  \
+    k_slice_pairs<w_><<<grid, PAIR_WARPS * 32, smem, s>>>(                                       \
+        P->pair_pad, P->peak, g, d_quats, d_ppr, n_panels, nx, ny, sc[0], sc[1], sc[2], ihw,     \
+        beta, P->exp_table, last, d_out);                                                        \
+    break;
+  switch (P->w) {
+    SPF_PAIR_CASE(2)
+    SPF_PAIR_CASE(3)
+    SPF_PAIR_CASE(4)
+    SPF_PAIR_CASE(5)
+    SPF_PAIR_CASE(6)
+    SPF_PAIR_CASE(7)
+    SPF_PAIR_CASE(8)
+    SPF_PAIR_CASE(9)
+    SPF_PAIR_CASE(10)
+    SPF_PAIR_CASE(11)
+    SPF_PAIR_CASE(12)
+    SPF_PAIR_CASE(13)
+    default: set_error("unsupported kernel width %d", P->w); return SPF_ERR_UNSUPPORTED;
+  }
+#undef SPF_PAIR_CASE
+  SPF_TRY(check_launch("k_slice_pairs"));
+  // a grid that pairs of floats cannot hold (NaN, infinity, nothing normal)
+  return slice_f64(P, d_quats, n_orient, d_ppr, n_pix, scale, d_out, P->peak, s);
 }
 
 int spf_nufft64_t1_zero(spf_nufft64_plan P, void *stream) {

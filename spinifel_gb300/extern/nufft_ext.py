@@ -98,9 +98,9 @@ class NUFFT:
     def slice_real(self, P, st: int, en: int, out=None, out_bf16=None):
         """Real part of the type 2 at reference orientations st:en, [en-st, N_pixels]
         (float64 from an FP64 plan)."""
-        if P.dtype == torch.float64:
-            return P.slice(self._quats64[st:en], self._ppr64, self.mult, out=out)
         det = self.reduced_det_shape if len(self.reduced_det_shape) == 3 else None
+        if P.dtype == torch.float64:
+            return P.slice(self._quats64[st:en], self._ppr64, self.mult, out=out, det_shape=det)
         return P.slice(self._quats[st:en], self._ppr, self.mult, out=out, out_bf16=out_bf16,
                        det_shape=det)
 

@@ -194,8 +194,9 @@ class NufftPlan:
 class NufftPlan64:
     """FP64 type 2 / type 1 at explicit points and FP64 slicing at
     orientation points (thread per point; quaternions, pixel positions and
-    the rotation in double).  Same call surface as NufftPlan for the methods
-    it has; no bin-sorted passes."""
+    the rotation in double; sums over pairs of floats on panel detectors).
+    Same call surface as NufftPlan for the methods it has; no bin-sorted
+    passes."""
 
     dtype = torch.float64
     supports_sort = False
@@ -267,11 +268,14 @@ class NufftPlan64:
 
     def slice(self, quats, ppr, scale: float, out: torch.Tensor | None = None,
               out_bf16=None, det_shape: tuple | None = None):
-        """FP64 slices [n_orient, n_pix] (real part) at the given orientations
-        (det_shape is accepted for symmetry with NufftPlan and not needed)."""
+        """FP64 slices [n_orient, n_pix] (real part) at the given orientations.
+        With det_shape = (n_panels, nx, ny) the sums run over pairs of floats
+        (about 2^-46) where the plan's kernel is no wider than 13."""
         if out_bf16 is not None:
             raise ValueError("the FP64 plan writes no bf16 copy")
         quats = self._f64(quats)
+        if det_shape is None and torch.is_tensor(ppr) and ppr.dim() == 4:
+            det_shape = tuple(ppr.shape[1:])
         ppr = self._f64(ppr).reshape(3, -1)
         n_o, n_p = quats.shape[0], ppr.shape[1]
         if out is None:
@@ -279,8 +283,14 @@ class NufftPlan64:
         _lib.require_cuda(out, "out", torch.float64)
         if out.numel() != n_o * n_p:
             raise ValueError("out has the wrong size")
-        _lib.call("spf_slice_t2_f64", self._h, _lib.ptr(quats), n_o, _lib.ptr(ppr), n_p,
-                  float(scale), _lib.ptr(out), _lib.stream_handle())
+        if self.has_modes and det_shape is not None and len(det_shape) == 3 and \
+                int(np.prod(det_shape)) == n_p:
+            _lib.call("spf_slice_t2_f64_det", self._h, _lib.ptr(quats), n_o, _lib.ptr(ppr),
+                      int(det_shape[0]), int(det_shape[1]), int(det_shape[2]), float(scale),
+                      _lib.ptr(out), _lib.stream_handle())
+        else:
+            _lib.call("spf_slice_t2_f64", self._h, _lib.ptr(quats), n_o, _lib.ptr(ppr), n_p,
+                      float(scale), _lib.ptr(out), _lib.stream_handle())
         return out
 
     def spread_zero(self):

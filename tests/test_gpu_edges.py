@@ -283,3 +283,52 @@ def test_interp_pairs_equal_single_parts():
         re, im = P.interp(x, y, z, want_imag=True)
         assert torch.equal(re, P.interp(x, y, z)[0])
         assert bool(torch.isfinite(im).all())
+
+
+@pytest.mark.parametrize("eps", [1e-2, 1e-5, 1e-9, 1e-11, 1e-12, 1e-13, 1e-14])
+@pytest.mark.parametrize("M,det,n", [(21, (4, 16, 16), 6), (13, (2, 9, 21), 5), (41, (1, 4, 8), 3),
+                                     (31, (3, 5, 7), 4), (9, (1, 1, 1), 7)])
+def test_fp64_slices_by_pairs(eps, M, det, n):
+    """FP64 slices from pairs of floats against the direct sums: the plan's
+    tolerance (20 eps, and 1e-13 for what the pairs and FP64 resolve), no
+    further off than the FP64 kernel by more than a tenth and 1e-14."""
+    from oracle import nufft as onufft
+    from spinifel_gb300 import geom
+    from spinifel_gb300.nufft import NufftPlan64
+
+    rng = np.random.default_rng(M + n)
+    ppr, pdr = geom.flat_detector(*det)
+    q = geom.uniform_quaternions(n, rng)
+    mult = np.pi / pdr.max()
+    f = rng.standard_normal((M, M, M))
+    P = NufftPlan64(M, eps)
+    H, K, L = geom.hkl(q, ppr)
+    want = onufft.nudft3d2(H.reshape(-1) * mult, K.reshape(-1) * mult, L.reshape(-1) * mult, f,
+                           -1).real.reshape(n, -1)
+    for scale in (1.0, 1e-200, 1e200, 3e-30):
+        P.set_modes(torch.as_tensor(f * scale, device="cuda"))
+        flat = P.slice(q, torch.as_tensor(ppr.reshape(3, -1), device="cuda"), mult)
+        pair = P.slice(q, torch.as_tensor(ppr.reshape(3, -1), device="cuda"), mult, det_shape=det)
+        e = [np.linalg.norm(v.cpu().numpy() / scale - want) / np.linalg.norm(want)
+             for v in (flat, pair)]
+        assert e[1] < max(20 * eps, 1e-13)
+        assert e[1] <= 1.1 * e[0] + 1e-14
+
+
+@pytest.mark.parametrize("bad", [0.0, 1e-310, float("inf"), float("nan")])
+def test_fp64_slices_of_grids_pairs_cannot_hold(bad):
+    """Zero, subnormal, infinite and NaN models take the FP64 kernel."""
+    from spinifel_gb300 import geom
+    from spinifel_gb300.nufft import NufftPlan64
+
+    rng = np.random.default_rng(5)
+    ppr, pdr = geom.flat_detector(2, 8, 8)
+    q = geom.uniform_quaternions(3, rng)
+    P = NufftPlan64(11, 1e-12)
+    f = np.zeros((11, 11, 11))
+    f[3, 4, 5] = bad
+    P.set_modes(torch.as_tensor(f, device="cuda"))
+    p = torch.as_tensor(ppr.reshape(3, -1), device="cuda")
+    a = P.slice(q, p, np.pi / pdr.max())
+    b = P.slice(q, p, np.pi / pdr.max(), det_shape=(2, 8, 8))
+    assert torch.equal(torch.nan_to_num(a, nan=7.0), torch.nan_to_num(b, nan=7.0))
