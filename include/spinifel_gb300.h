@@ -427,6 +427,15 @@ int64_t spf_dist_topk_bf16_tile_refs(void);
 int spf_dist_topk_bf16(const void *d_img_bf16, int64_t n_img, const void *d_ref_bf16,
                        int64_t n_ref, int64_t n_pix, int64_t ld, const float *d_ref_sq,
                        float *d_cand_d, int32_t *d_cand_i, void *stream);
+/* The same lists with device scratch of spf_dist_topk_bf16_work_bytes bytes
+ * (16-byte aligned; 0 bytes or a NULL scratch: spf_dist_topk_bf16): calls with
+ * few tiles are cut along the pixels too, so that every SM has a part.  The
+ * approximate distances differ in the order of their FP32 sums only. */
+int64_t spf_dist_topk_bf16_work_bytes(int64_t n_img, int64_t n_ref, int64_t n_pix);
+int spf_dist_topk_bf16_work(const void *d_img_bf16, int64_t n_img, const void *d_ref_bf16,
+                            int64_t n_ref, int64_t n_pix, int64_t ld, const float *d_ref_sq,
+                            float *d_cand_d, int32_t *d_cand_i, void *d_work,
+                            int64_t work_bytes, void *stream);
 
 /* Merge the candidates of all tiles into the per-frame top-8 (written over
  * tile 0 of the candidate buffers, so each candidate set is re-ranked once),

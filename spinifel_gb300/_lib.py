@@ -108,6 +108,9 @@ SIGNATURES = {
     "spf_dist_topk_bf16_tile_refs": [],
     "spf_dist_topk_bf16": [_c_void_p, _i64, _c_void_p, _i64, _i64, _i64, _c_void_p, _c_void_p,
                            _c_void_p, _c_void_p],
+    "spf_dist_topk_bf16_work_bytes": [_i64, _i64, _i64],
+    "spf_dist_topk_bf16_work": [_c_void_p, _i64, _c_void_p, _i64, _i64, _i64, _c_void_p,
+                                _c_void_p, _c_void_p, _c_void_p, _i64, _c_void_p],
     "spf_rerank_fp32": [_c_void_p, _c_void_p, _i64, _c_void_p, _c_void_p, _i64, _c_void_p,
                         _c_void_p, _c_void_p, ctypes.c_float, _i64, _i64, _i64, _c_void_p,
                         _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
@@ -202,6 +205,7 @@ _RESTYPES = {
     "spf_launch_count": ctypes.c_uint64,
     "spf_argmin_f64_work_bytes": ctypes.c_int64,
     "spf_dist_topk_bf16_tiles": ctypes.c_int64,
+    "spf_dist_topk_bf16_work_bytes": ctypes.c_int64,
     "spf_dist_topk_bf16_tile_refs": ctypes.c_int64,
     "spf_serve_clock": ctypes.c_double,
 }

@@ -173,18 +173,23 @@ __device__ __forceinline__ void tile_of(int64_t t, int64_t n_m, int64_t n_n, int
   n = r / gm;
 }
 
-// RANGE = false: per-tile top-8 into cand_d / cand_i.
-// RANGE = true : every reference with s2 - 2 acc <= thresh[row] is appended to
-//                list[row * cap ..] (count[row] holds the number found, which
-//                may exceed cap: the caller then treats the row as overflowed).
-template <bool RANGE>
+// TOP8 : per-tile top-8 into cand_d / cand_i.
+// RANGE: every reference with s2 - 2 acc <= thresh[row] is appended to
+//        list[row * cap ..] (count[row] holds the number found, which may
+//        exceed cap: the caller then treats the row as overflowed).
+// SPLIT: a tile's pixels are cut into `splits` parts, each a tile of its own;
+//        the products go to part[split][n tile][row][BN] (cand_d) and
+//        k_split_top8 adds them up.
+enum class Out { TOP8, RANGE, SPLIT };
+
+template <Out OUT>
 __global__ void __launch_bounds__(THREADS, 1)
     k_dist_topk_bf16(const __grid_constant__ CUtensorMap tmap_a,
                      const __grid_constant__ CUtensorMap tmap_b, const float *__restrict__ ref_sq,
                      int64_t n_img, int64_t n_ref, int64_t n_pix, float *__restrict__ cand_d,
                      int32_t *__restrict__ cand_i, const float *__restrict__ thresh,
                      int32_t *__restrict__ list, int32_t *__restrict__ count, int cap,
-                     int group_m, unsigned int *__restrict__ err) {
+                     int group_m, unsigned int *__restrict__ err, int splits) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -203,8 +208,16 @@ __global__ void __launch_bounds__(THREADS, 1)
   const int lane = threadIdx.x & 31;
   const int64_t n_m = (n_img + BM - 1) / BM;
   const int64_t n_n = (n_ref + BN - 1) / BN;
-  const int64_t n_tiles = n_m * n_n;
-  const int nkb = (int)((n_pix + BK - 1) / BK);
+  const int S = OUT == Out::SPLIT ? splits : 1;
+  const int64_t n_tiles = n_m * n_n * S;
+  const int nkb_all = (int)((n_pix + BK - 1) / BK);
+  // tile t: part t % S of the pixels' blocks of tile t / S
+  auto kb_from = [&](int64_t t) {
+    return OUT == Out::SPLIT ? (int)((t % S) * nkb_all / S) : 0;
+  };
+  auto kb_to = [&](int64_t t) {
+    return OUT == Out::SPLIT ? (int)((t % S + 1) * nkb_all / S) : nkb_all;
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -238,8 +251,9 @@ __global__ void __launch_bounds__(THREADS, 1)
       bool ok = true;
       for (int64_t t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
         int64_t m, n;
-        tile_of(t, n_m, n_n, group_m, m, n);
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
+        tile_of(t / S, n_m, n_n, group_m, m, n);
+        const int kb1 = kb_to(t);
+        for (int kb = kb_from(t); kb < kb1; ++kb, ++it) {
           int s = it % STAGES;
           uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait(&empty[s], ph ^ 1, abort)) {
@@ -271,7 +285,8 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (!mbar_wait(&acc_empty[b], (use & 1) ^ 1, abort)) break;
         tc_fence_after();
         uint32_t d_tmem = tmem_base + b * ACC_STRIDE;
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
+        const int kb0 = kb_from(t), kb1 = kb_to(t);
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
           int s = it % STAGES;
           uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait(&full[s], ph, abort)) {
@@ -284,7 +299,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
             umma_bf16(d_tmem, sdesc_sw128(a0 + k * 32), sdesc_sw128(b0 + k * 32),
-                      (kb | k) != 0 ? 1u : 0u);
+                      ((kb - kb0) | k) != 0 ? 1u : 0u);
           }
           umma_commit(&empty[s]);
         }
@@ -303,7 +318,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     uint32_t tc = 0;
     for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x, ++tc) {
       int64_t m, n;
-      tile_of(t, n_m, n_n, group_m, m, n);
+      tile_of(t / S, n_m, n_n, group_m, m, n);
       uint32_t b = tc & 1, use = tc >> 1;
       // one lane waits, the warp follows (tcgen05.ld below is warp-collective)
       int ok = 1;
@@ -313,7 +328,24 @@ __global__ void __launch_bounds__(THREADS, 1)
       tc_fence_after();
       const int64_t row = m * BM + q * 32 + lane;
       const int64_t col0 = n * BN;
-      if constexpr (RANGE) {
+      if constexpr (OUT == Out::SPLIT) {
+        float4 *dst = reinterpret_cast<float4 *>(
+            cand_d + (((t % S) * n_n + n) * n_img + (row < n_img ? row : 0)) * BN);
+#pragma unroll 1
+        for (int c = 0; c < BN / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + b * ACC_STRIDE + c * 32, r);
+          if (row < n_img) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              dst[c * 8 + j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                                           __uint_as_float(r[4 * j + 2]),
+                                           __uint_as_float(r[4 * j + 3]));
+          }
+        }
+        tc_fence_before();
+        mbar_arrive(&acc_empty[b]);
+      } else if constexpr (OUT == Out::RANGE) {
         const float thr = row < n_img ? thresh[row] : -__int_as_float(0x7f800000);
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
@@ -371,6 +403,58 @@ __global__ void __launch_bounds__(THREADS, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
                  "r"(TMEM_COLS)
                  : "memory");
+  }
+}
+
+// The top-8 of every (n tile, image) from the products of its parts, a warp
+// each: the values and lists that the undivided tile's epilogue gives, but
+// for the order of the FP32 sum over the parts.
+__global__ void __launch_bounds__(256)
+    k_split_top8(const float *__restrict__ part, int splits, const float *__restrict__ ref_sq,
+                 int64_t n_img, int64_t n_ref, int64_t n_n, float *__restrict__ cand_d,
+                 int32_t *__restrict__ cand_i) {
+  constexpr int PER = BN / 32;
+  const int lane = threadIdx.x & 31;
+  const int64_t row = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= n_n * n_img) return;
+  const int64_t n = row / n_img;
+  float v[PER];
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int64_t col = n * BN + u * 32 + lane;
+    float acc = 0.0f;
+    for (int s = 0; s < splits; ++s)
+      acc += part[((int64_t)s * n_n * n_img + row) * BN + u * 32 + lane];
+    v[u] = col < n_ref ? ref_sq[col] - 2.0f * acc : __int_as_float(0x7f800000);
+  }
+  float *od = cand_d + row * TOPK;
+  int32_t *oi = cand_i + row * TOPK;
+  // eight rounds of the smallest (value, column) left; NaN and infinity are
+  // never listed, as in TopK::push
+  unsigned taken = 0;
+  for (int r = 0; r < TOPK; ++r) {
+    float bv = __int_as_float(0x7f800000);
+    int bc = BN;
+#pragma unroll
+    for (int u = 0; u < PER; ++u)
+      if (!(taken >> u & 1) && v[u] < bv) {
+        bv = v[u];
+        bc = u * 32 + lane;
+      }
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+      const int oc = __shfl_xor_sync(0xffffffffu, bc, o);
+      if (ov < bv || (ov == bv && oc < bc)) {
+        bv = ov;
+        bc = oc;
+      }
+    }
+    if (bc < BN && (bc & 31) == lane) taken |= 1u << (bc >> 5);
+    if (lane == 0) {
+      od[r] = bv;
+      oi[r] = bc < BN ? (int32_t)(n * BN + bc) : INT32_MAX;
+    }
   }
 }
 
@@ -1169,7 +1253,8 @@ int64_t spf_dist_topk_bf16_tiles(int64_t n_ref) { return (n_ref + BN - 1) / BN; 
 
 int64_t spf_dist_topk_bf16_tile_refs(void) { return BN; }
 
-static int launch_bf16(bool range, const void *d_img_bf16, int64_t n_img, const void *d_ref_bf16,
+static int launch_bf16(Out out, int splits, float *d_part, const void *d_img_bf16,
+                       int64_t n_img, const void *d_ref_bf16,
                        int64_t n_ref, int64_t n_pix, int64_t ld, const float *d_ref_sq,
                        float *d_cand_d, int32_t *d_cand_i, const float *d_thresh,
                        int32_t *d_list, int32_t *d_count, int cap, void *stream,
@@ -1195,31 +1280,40 @@ static int launch_bf16(bool range, const void *d_img_bf16, int64_t n_img, const 
   CUtensorMap ma, mb;
   SPF_TRY(make_map(&ma, d_img_bf16, n_img, ld, BM));
   SPF_TRY(make_map(&mb, d_ref_bf16, n_ref, ld, BN));
-  static bool attr_set[2][64] = {{false}};
-  if (dev >= 0 && dev < 64 && !attr_set[range][dev]) {
-    cudaError_t e = range ? cudaFuncSetAttribute(k_dist_topk_bf16<true>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 SMEM_BYTES)
-                          : cudaFuncSetAttribute(k_dist_topk_bf16<false>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 SMEM_BYTES);
+  static bool attr_set[3][64] = {{false}};
+  if (dev >= 0 && dev < 64 && !attr_set[(int)out][dev]) {
+    const void *fn = out == Out::RANGE   ? (const void *)k_dist_topk_bf16<Out::RANGE>
+                     : out == Out::SPLIT ? (const void *)k_dist_topk_bf16<Out::SPLIT>
+                                         : (const void *)k_dist_topk_bf16<Out::TOP8>;
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         SMEM_BYTES);
     SPF_TRY(check_cuda(e, name));
-    attr_set[range][dev] = true;
+    attr_set[(int)out][dev] = true;
   }
   unsigned int *err = device_error_word();
   SPF_REQUIRE(err != nullptr, "%s: no device error word", name);
-  int64_t tiles = ((n_img + BM - 1) / BM) * ((n_ref + BN - 1) / BN);
+  const int64_t n_n = (n_ref + BN - 1) / BN;
+  int64_t tiles = ((n_img + BM - 1) / BM) * n_n * splits;
   int64_t max_grid = tune_get(SPF_TUNE_BF16_GRID, sm_count());
   int grid = (int)(tiles < max_grid ? tiles : max_grid);
   int group_m = (int)tune_get(SPF_TUNE_BF16_GROUP_M, GROUP_M);
-  if (range)
-    k_dist_topk_bf16<true><<<grid, THREADS, SMEM_BYTES, as_stream(stream)>>>(
+  cudaStream_t s = as_stream(stream);
+  if (out == Out::RANGE) {
+    k_dist_topk_bf16<Out::RANGE><<<grid, THREADS, SMEM_BYTES, s>>>(
         ma, mb, d_ref_sq, n_img, n_ref, n_pix, nullptr, nullptr, d_thresh, d_list, d_count, cap,
-        group_m, err);
-  else
-    k_dist_topk_bf16<false><<<grid, THREADS, SMEM_BYTES, as_stream(stream)>>>(
+        group_m, err, 1);
+  } else if (out == Out::SPLIT) {
+    k_dist_topk_bf16<Out::SPLIT><<<grid, THREADS, SMEM_BYTES, s>>>(
+        ma, mb, d_ref_sq, n_img, n_ref, n_pix, d_part, nullptr, nullptr, nullptr, nullptr, 0,
+        group_m, err, splits);
+    SPF_TRY(check_launch(name));
+    k_split_top8<<<grid_for(n_n * n_img, 8), 256, 0, s>>>(d_part, splits, d_ref_sq, n_img, n_ref,
+                                                          n_n, d_cand_d, d_cand_i);
+  } else {
+    k_dist_topk_bf16<Out::TOP8><<<grid, THREADS, SMEM_BYTES, s>>>(
         ma, mb, d_ref_sq, n_img, n_ref, n_pix, d_cand_d, d_cand_i, nullptr, nullptr, nullptr, 0,
-        group_m, err);
+        group_m, err, 1);
+  }
   return check_launch(name);
 }
 
@@ -1230,8 +1324,65 @@ int spf_dist_topk_bf16(const void *d_img_bf16, int64_t n_img, const void *d_ref_
               "spf_dist_topk_bf16: NULL candidate buffer");
   SPF_REQUIRE(aligned(d_cand_d, 16) && aligned(d_cand_i, 16),
               "spf_dist_topk_bf16: candidate buffers must be 16-byte aligned");
-  return launch_bf16(false, d_img_bf16, n_img, d_ref_bf16, n_ref, n_pix, ld, d_ref_sq, d_cand_d,
-                     d_cand_i, nullptr, nullptr, nullptr, 0, stream, "spf_dist_topk_bf16");
+  return launch_bf16(Out::TOP8, 1, nullptr, d_img_bf16, n_img, d_ref_bf16, n_ref, n_pix, ld,
+                     d_ref_sq, d_cand_d, d_cand_i, nullptr, nullptr, nullptr, 0, stream,
+                     "spf_dist_topk_bf16");
+}
+
+// Parts to cut every tile's pixels into: a call with fewer than two tiles an
+// SM leaves SMs idle in its last wave (90 of 152 busy with 20,000 references
+// and one tile of images), and each tile then takes as long as one SM needs
+// to stream its operands, whatever the number of references: 6.4 ns a pixel
+// (320 us at 65,536 with few SMs at work, 430 with all).  The number of parts
+// with the least waves x part (2% more for each part), plus writing the
+// products and reading them back (3 TB/s, and a launch), if that is a tenth
+// faster; at least 16 blocks
+// of 64 pixels a part.  Undivided and divided, us (images x references x
+// pixels): 5 x 2,000 x 65,536: 317, 82; 5 x 10,000: 337, 221; 5 x 20,000:
+// 434, 409 (387 is HBM's time); 5 x 36,000: 941, 762; 300 x 5,000: 320, 193;
+// 1,000 x 2,000: 317, 186; 5 x 2,000 x 16,384: 103, 40.
+static int pick_splits(int64_t n_img, int64_t n_ref, int64_t n_pix) {
+  const int64_t n_n = (n_ref + BN - 1) / BN;
+  const int64_t t = ((n_img + BM - 1) / BM) * n_n, sms = sm_count();
+  if (t == 0 || t >= 2 * sms) return 1;
+  const int64_t nkb = (n_pix + BK - 1) / BK;
+  const double tile_us = 6.4e-3 * (double)n_pix;
+  int best = 1;
+  double best_us = 0.9 * (double)((t + sms - 1) / sms) * tile_us;
+  for (int s = 2; s <= 16 && nkb / s >= 16 && t * s <= 4 * sms; ++s) {
+    const double us = (1.0 + 0.02 * s) * (double)((t * s + sms - 1) / sms) / s * tile_us + 8.0 +
+                      (double)s * n_n * n_img * BN * 8 / 3e6;
+    if (us < best_us) {
+      best_us = us;
+      best = s;
+    }
+  }
+  return best;
+}
+
+int64_t spf_dist_topk_bf16_work_bytes(int64_t n_img, int64_t n_ref, int64_t n_pix) {
+  if (n_img <= 0 || n_ref <= 0 || n_pix <= 0) return 0;
+  const int s = pick_splits(n_img, n_ref, n_pix);
+  return s == 1 ? 0 : (int64_t)s * ((n_ref + BN - 1) / BN) * n_img * BN * (int64_t)sizeof(float);
+}
+
+int spf_dist_topk_bf16_work(const void *d_img_bf16, int64_t n_img, const void *d_ref_bf16,
+                            int64_t n_ref, int64_t n_pix, int64_t ld, const float *d_ref_sq,
+                            float *d_cand_d, int32_t *d_cand_i, void *d_work, int64_t work_bytes,
+                            void *stream) {
+  const int64_t need = spf_dist_topk_bf16_work_bytes(n_img, n_ref, n_pix);
+  if (need == 0 || !d_work)
+    return spf_dist_topk_bf16(d_img_bf16, n_img, d_ref_bf16, n_ref, n_pix, ld, d_ref_sq, d_cand_d,
+                              d_cand_i, stream);
+  SPF_REQUIRE(work_bytes >= need && aligned(d_work, 16),
+              "spf_dist_topk_bf16_work: workspace too small or not 16-byte aligned");
+  SPF_REQUIRE(d_cand_d && d_cand_i, "spf_dist_topk_bf16_work: NULL candidate buffer");
+  SPF_REQUIRE(aligned(d_cand_d, 16) && aligned(d_cand_i, 16),
+              "spf_dist_topk_bf16_work: candidate buffers must be 16-byte aligned");
+  return launch_bf16(Out::SPLIT, pick_splits(n_img, n_ref, n_pix),
+                     reinterpret_cast<float *>(d_work), d_img_bf16, n_img, d_ref_bf16, n_ref, n_pix,
+                     ld, d_ref_sq, d_cand_d, d_cand_i, nullptr, nullptr, nullptr, 0, stream,
+                     "spf_dist_topk_bf16_work");
 }
 
 int spf_dist_range_bf16(const void *d_img_bf16, int64_t n_img, const void *d_ref_bf16,
@@ -1244,8 +1395,8 @@ int spf_dist_range_bf16(const void *d_img_bf16, int64_t n_img, const void *d_ref
   if (n_img > 0)
     SPF_TRY(check_cuda(cudaMemsetAsync(d_count, 0, n_img * sizeof(int32_t), as_stream(stream)),
                        "spf_dist_range_bf16"));
-  return launch_bf16(true, d_img_bf16, n_img, d_ref_bf16, n_ref, n_pix, ld, d_ref_sq, nullptr,
-                     nullptr, d_thresh, d_list, d_count, cap, stream, "spf_dist_range_bf16");
+  return launch_bf16(Out::RANGE, 1, nullptr, d_img_bf16, n_img, d_ref_bf16, n_ref, n_pix, ld,
+                     d_ref_sq, nullptr, nullptr, d_thresh, d_list, d_count, cap, stream, "spf_dist_range_bf16");
 }
 
 int spf_rerank_list_fp32(const int32_t *d_list, const int32_t *d_count, int cap,
@@ -1595,7 +1746,7 @@ static int static_scratch(int dev, unsigned char **out) {
     g_static_ptr[dev] = static_cast<unsigned char *>(p);
   }
   if (!g_static_attr[dev]) {
-    SPF_TRY(check_cuda(cudaFuncSetAttribute(k_dist_topk_bf16<false>,
+    SPF_TRY(check_cuda(cudaFuncSetAttribute(k_dist_topk_bf16<Out::TOP8>,
                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             SMEM_BYTES),
                        "spf_match_bf16_static"));
@@ -1673,9 +1824,9 @@ extern "C" int spf_match_bf16_static(const void *d_img_bf16, const float *d_img,
   SPF_TRY(make_map(&mb, d_ref_bf16, n_ref, ld, BN));
   int64_t gemm_tiles = ((n_img + BM - 1) / BM) * tiles;
   int grid = (int)(gemm_tiles < sm_count() ? gemm_tiles : sm_count());
-  k_dist_topk_bf16<false><<<grid, THREADS, SMEM_BYTES, s>>>(ma, mb, d_ref_sq, n_img, n_ref,
+  k_dist_topk_bf16<Out::TOP8><<<grid, THREADS, SMEM_BYTES, s>>>(ma, mb, d_ref_sq, n_img, n_ref,
                                                             n_pix, cand_d, cand_i, nullptr,
-                                                            nullptr, nullptr, 0, GROUP_M, err);
+                                                            nullptr, nullptr, 0, GROUP_M, err, 1);
   SPF_TRY(check_launch("k_dist_topk_bf16 (static scratch)"));
   if (tune_get(SPF_TUNE_STATIC_ABORT_TEST, 0)) {
     k_static_inject_timeout<<<1, 32, 0, s>>>(err);

@@ -333,8 +333,11 @@ def match_bf16(frames: FrameSet, refs: ReferenceSet, exact_fallback: bool = True
     dist = torch.empty(n_img, dtype=torch.float32, device=dev)
     unc = torch.empty(n_img, dtype=torch.int32, device=dev)
     sh = _lib.stream_handle(stream)
-    _lib.call("spf_dist_topk_bf16", _lib.ptr(frames.bf16), n_img, _lib.ptr(refs.bf16), refs.n_ref,
-              refs.n_pix, refs.ld, _lib.ptr(refs.sq), _lib.ptr(cand_d), _lib.ptr(cand_i), sh)
+    size = int(_lib.lib().spf_dist_topk_bf16_work_bytes(n_img, refs.n_ref, refs.n_pix))
+    part = _ws.get("parts", size, torch.uint8, dev) if size else None
+    _lib.call("spf_dist_topk_bf16_work", _lib.ptr(frames.bf16), n_img, _lib.ptr(refs.bf16),
+              refs.n_ref, refs.n_pix, refs.ld, _lib.ptr(refs.sq), _lib.ptr(cand_d),
+              _lib.ptr(cand_i), _lib.ptr(part), size, sh)
     _lib.call("spf_rerank_fp32_keep", _lib.ptr(cand_d), _lib.ptr(cand_i), tiles,
               _lib.ptr(frames.f32), _lib.ptr(frames.sq), n_img, _lib.ptr(refs.f32),
               _lib.ptr(refs.sq), _lib.ptr(refs.m2), float(refs.sq_max), refs.n_ref, refs.n_pix,

@@ -332,3 +332,46 @@ def test_fp64_slices_of_grids_pairs_cannot_hold(bad):
     a = P.slice(q, p, np.pi / pdr.max())
     b = P.slice(q, p, np.pi / pdr.max(), det_shape=(2, 8, 8))
     assert torch.equal(torch.nan_to_num(a, nan=7.0), torch.nan_to_num(b, nan=7.0))
+
+
+@pytest.mark.parametrize("n_img,n_ref,n_pix", [(1, 1, 4096), (5, 7, 2048), (5, 223, 3000),
+                                               (3, 225, 4104), (128, 900, 2049),
+                                               (129, 3000, 5000), (300, 20000, 2112),
+                                               (1, 36000, 2050), (5, 7, 6400), (2, 223, 8200),
+                                               (128, 900, 8193), (1, 36000, 8200)])
+def test_split_tiles_give_the_same_lists(n_img, n_ref, n_pix):
+    """Tiles cut along the pixels (where the rule cuts them) list, per tile and image, the 8 references
+    of the undivided tile with the same distances up to FP32 rounding (no more
+    than n_pix / 64 partial sums of x.s, so 1e-5 of its size), and the match
+    is the plain path's."""
+    from spinifel_gb300 import _lib, matching
+
+    size = int(_lib.lib().spf_dist_topk_bf16_work_bytes(n_img, n_ref, n_pix))
+    if n_pix > 6000:
+        assert size > 0
+    counts, refs = _frames_refs(n_img, n_ref, n_pix, n_img + n_ref, mean=1.0)
+    fs = matching.FrameSet.from_counts(torch.as_tensor(counts.view(np.int16), device="cuda"))
+    rs = matching.ReferenceSet(torch.as_tensor(refs, device="cuda"))
+    tiles = int(_lib.lib().spf_dist_topk_bf16_tiles(n_ref))
+    got = []
+    for work in (None, torch.empty(max(size, 16), dtype=torch.uint8, device="cuda")):
+        d = torch.full((tiles, n_img, 8), -1.0, device="cuda")
+        i = torch.full((tiles, n_img, 8), -7, dtype=torch.int32, device="cuda")
+        _lib.call("spf_dist_topk_bf16_work", _lib.ptr(fs.bf16), n_img, _lib.ptr(rs.bf16), n_ref,
+                  n_pix, rs.ld, _lib.ptr(rs.sq), _lib.ptr(d), _lib.ptr(i),
+                  _lib.ptr(work) if work is not None else None, size, _lib.stream_handle())
+        got.append((d, i))
+    (d0, i0), (d1, i1) = got
+    tol = 1e-5 * float(rs.sq.max() + 2 * (rs.sq.max() * fs.sq.max()).sqrt())
+    fin = torch.isfinite(d0)
+    assert torch.equal(fin, torch.isfinite(d1))
+    assert float((d0[fin] - d1[fin]).abs().max()) <= tol
+    assert torch.equal(i0[~fin], i1[~fin])
+    # a listed reference may differ only where its distance ties within rounding
+    other = (i0 != i1) & fin
+    assert float(other.float().mean()) < 0.01
+    idx, dist = matching.match_bf16(fs, rs)
+    pidx, pdist = matching.argmin_fp32(fs.f32, rs.f32, images_sq=fs.sq, refs_sq=rs.sq)
+    assert torch.equal(idx, pidx)
+    assert torch.equal(dist, pdist)
+    matching.check_device_error()
