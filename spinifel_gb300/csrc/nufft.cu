@@ -1588,11 +1588,11 @@ int spf_slice_t2(spf_nufft_plan P, const float *d_quats, int64_t n_orient, const
 // memory; the stride search (16 reductions a warp) pays unless the footprints
 // of a warp all but coincide.  Times in us with 16 x 16 patches, 16 x 16 with
 // the search, 8 x 16 without and with it (grid, detector, orientations):
-//   0.35 cells  90^3,  4 x 128 x 128,  100:   384   420   378   417
-//   0.63 cells 162^3,  4 x 128 x 128,  500:  2474  2061  2119  2050
-//   1.25 cells 320^3,  4 x 128 x 128,  200:  1622  1474  1469  1349
-//   1.41 cells  90^3,  4 x 32 x 32,   2000:  1308  1187   989   911
-//   1.72 cells 128^3,  3 x 50 x 37,    500:   362   315   313   294
+//   0.35 cells  90^3,  4 x 128 x 128,  100:   384   420   377   417
+//   0.63 cells 162^3,  4 x 128 x 128,  500:  2474  2061  2119  2001
+//   1.25 cells 320^3,  4 x 128 x 128,  200:  1622  1474  1469  1312
+//   1.41 cells  90^3,  4 x 32 x 32,   2000:  1308  1187   989   893
+//   1.72 cells 128^3,  3 x 50 x 37,    500:   362   315   313   284
 //   2.53 cells 162^3,  4 x 32 x 32,   1000:  1639  1629  3793  1779
 // (A detector with more 8 x 16 patches than a launch takes keeps 16 x 16.)
 static int default_shape(const spf_nufft_plan_s *P, int n_panels, int nx, int ny) {
@@ -1624,8 +1624,11 @@ int spf_slice_t2_det(spf_nufft_plan P, const float *d_quats, int64_t n_orient, c
   dim3 grid((unsigned)n_orient, (unsigned)patches);
   auto *bf = reinterpret_cast<__nv_bfloat16 *>(d_out_bf16);
   const int threads = ps.px * ps.py;
-  // five CTAs an SM of 256 threads, six of 128
-  const int floats = threads == 256 ? SLICE_SMEM_FLOATS : SLICE_SMEM_FLOATS * 5 / 6;
+  // 44 KB for 256 threads (five CTAs an SM); 30 KB for 128, of which registers
+  // allow six: the rest serves the box fills as L1 (81^3, 4 x 128 x 128 x 500
+  // with 37, 30, 25, 22 KB: 2,051, 2,001, 1,998, 1,999 us; 41^3, 4 x 32 x 32 x
+  // 2,000, where boxes are large: 909, 893, 1,018, 1,239)
+  const int floats = threads == 256 ? SLICE_SMEM_FLOATS : SLICE_SMEM_FLOATS * 11 / 16;
   const size_t smem = floats * sizeof(float);
   if (ps.search) {
     SPF_W_DISPATCH(P->w, (k_slice_t2_det<W, true><<<grid, threads, smem, s>>>(
