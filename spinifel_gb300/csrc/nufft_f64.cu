@@ -515,6 +515,31 @@ using namespace spf::f64;
 
 extern "C" {
 
+static Pair pair_of(double v) {
+  Pair p;
+  p.h = (float)v;
+  p.l = (float)(v - (double)p.h);
+  return p;
+}
+
+// The float-pair grid, its peak and the table of exponentials in one
+// allocation, made with the plan (setting a model then allocates nothing and
+// can be captured).
+static int alloc_pairs(spf_nufft64_plan P) {
+  const size_t npad = (size_t)P->np[0] * P->np[1] * P->np[2];
+  const int n = (int)ceil(EXP_PER_UNIT * P->beta) + 2;
+  std::vector<float2> t(n);
+  for (int j = 0; j < n; ++j) {
+    const Pair p = pair_of(exp(-(double)j / EXP_PER_UNIT));
+    t[j] = make_float2(p.h, p.l);
+  }
+  SPF_TRY(check_cuda(cudaMalloc(&P->pair_pad, (npad + n + 1) * sizeof(float2)), "plan64_create"));
+  P->exp_table = P->pair_pad + npad;
+  P->peak = reinterpret_cast<unsigned long long *>(P->exp_table + n);
+  return check_cuda(cudaMemcpy(P->exp_table, t.data(), n * sizeof(float2), cudaMemcpyHostToDevice),
+                    "plan64_create");
+}
+
 int spf_nufft64_plan_create(int m1, int m2, int m3, double eps, double upsampfac,
                             spf_nufft64_plan *out) {
   SPF_REQUIRE(out != nullptr, "spf_nufft64_plan_create: out is NULL");
@@ -557,6 +582,7 @@ int spf_nufft64_plan_create(int m1, int m2, int m3, double eps, double upsampfac
                                              (P->n[2] / 2 + 1) * sizeof(double2)), "plan64_create");
   if (st == SPF_OK) P->half = reinterpret_cast<double2 *>(P->fine + nfine);
   if (st == SPF_OK) st = check_cuda(cudaMalloc(&P->re_pad, npad * sizeof(double)), "plan64_create");
+  if (st == SPF_OK && P->w <= PAIR_MAX_W) st = alloc_pairs(P);
   if (st == SPF_OK) {
     cufftResult r = cufftPlan3d(&P->fft, P->n[0], P->n[1], P->n[2], CUFFT_D2Z);
     if (r != CUFFT_SUCCESS) {
@@ -586,8 +612,6 @@ int spf_nufft64_plan_destroy(spf_nufft64_plan P) {
   cudaFree(P->im_pad);
   cudaFree(P->acc_pad);
   cudaFree(P->pair_pad);
-  cudaFree(P->peak);
-  cudaFree(P->exp_table);
   if (P->fft_ok) cufftDestroy(P->fft);
   if (prev != P->dev && prev >= 0) cudaSetDevice(prev);
   delete P;
@@ -606,38 +630,11 @@ int spf_nufft64_plan_info(spf_nufft64_plan P, int *n_fine, int *width, double *b
   return SPF_OK;
 }
 
-static Pair pair_of(double v) {
-  Pair p;
-  p.h = (float)v;
-  p.l = (float)(v - (double)p.h);
-  return p;
-}
-
 // the float-pair copy of the padded grid, part of setting a model (so that a
 // captured slicing reads the model set last)
 static int make_pairs(spf_nufft64_plan P, cudaStream_t s) {
   const int64_t npad = (int64_t)P->np[0] * P->np[1] * P->np[2];
-  const char *what = "spf_nufft64_t2_set_modes";
-  if (!P->exp_table) {
-    const int n = (int)ceil(EXP_PER_UNIT * P->beta) + 2;
-    std::vector<float2> t(n);
-    for (int j = 0; j < n; ++j) {
-      const Pair p = pair_of(exp(-(double)j / EXP_PER_UNIT));
-      t[j] = make_float2(p.h, p.l);
-    }
-    float2 *d = nullptr;
-    SPF_TRY(check_cuda(cudaMalloc(&d, n * sizeof(float2)), what));
-    const int st = check_cuda(cudaMemcpy(d, t.data(), n * sizeof(float2), cudaMemcpyHostToDevice),
-                              what);
-    if (st != SPF_OK) {
-      cudaFree(d);
-      return st;
-    }
-    P->exp_table = d;
-  }
-  if (!P->peak) SPF_TRY(check_cuda(cudaMalloc(&P->peak, sizeof(*P->peak)), what));
-  if (!P->pair_pad) SPF_TRY(check_cuda(cudaMalloc(&P->pair_pad, npad * sizeof(float2)), what));
-  SPF_TRY(check_cuda(cudaMemsetAsync(P->peak, 0, sizeof(*P->peak), s), what));
+  SPF_TRY(check_cuda(cudaMemsetAsync(P->peak, 0, sizeof(*P->peak), s), "spf_nufft64_t2_set_modes"));
   k_peak<<<grid_for(npad, 1024, (int64_t)sm_count() * 8), 256, 0, s>>>(P->re_pad, npad, P->peak);
   SPF_TRY(check_launch("k_peak"));
   k_to_pairs<<<grid_for(npad, 256, (int64_t)sm_count() * 16), 256, 0, s>>>(P->re_pad, npad, P->peak,
@@ -723,7 +720,6 @@ int spf_slice_t2_f64_det(spf_nufft64_plan P, const double *d_quats, int64_t n_or
   SPF_REQUIRE(n_orient < (1LL << 31) && n_pix <= 65535LL * 128,
               "spf_slice_t2_f64_det: size too large");
   cudaStream_t s = as_stream(stream);
-  SPF_REQUIRE(P->pair_pad != nullptr, "spf_slice_t2_f64_det: no model set");
   const Geom g = geom_of(P);
   double sc[3];
   grid_scales(P, scale, sc);
