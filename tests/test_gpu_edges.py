@@ -161,12 +161,14 @@ def test_minima_equal_full_fp64_block(kind, n_img, n_ref, n_pix):
 
 @pytest.mark.parametrize("w,eps", [(3, 1e-2), (5, 1e-4), (7, 1e-6), (8, 1e-7)])
 @pytest.mark.parametrize("n,spread", [(1, 3.0), (33, 3.0), (1025, 0.02), (5000, 3.0), (20000, 0.3),
-                                      (70001, 3.1)])
+                                      (70001, 3.1), ((1 << 19) - 1, 3.1), ((1 << 19) + 77, 3.1),
+                                      (1 << 19, 0.05)])
 def test_sorted_spread_equals_per_point_spread(w, eps, n, spread):
-    """Bin sort and pencil spreading against one thread per point: the same
-    sums to FP32 rounding (each cell adds at most n terms of one sign here),
+    """Bin sort and pencil spreading against one thread per point in the FP64
+    plan of the same kernel width (in FP32 that form loses 5e-5 itself where
+    2^19 points of one sign add to one cell): the same sums to FP32 rounding,
     for one point, points of one cell, dense clusters and whole grids."""
-    from spinifel_gb300.nufft import NufftPlan
+    from spinifel_gb300.nufft import NufftPlan, NufftPlan64
 
     rng = np.random.default_rng(n + w)
     P = NufftPlan((19, 24, 31), eps)
@@ -174,9 +176,11 @@ def test_sorted_spread_equals_per_point_spread(w, eps, n, spread):
     x, y, z = (torch.as_tensor(rng.uniform(-spread, spread, n).astype(np.float32), device="cuda")
                for _ in range(3))
     c = torch.as_tensor(rng.random(n).astype(np.float32), device="cuda")
-    P.spread_zero()
-    P.spread(x, y, z, c)
-    want = P.finish(+1, want_imag=True)
+    P64 = NufftPlan64((19, 24, 31), eps)
+    assert P64.width == w
+    P64.spread_zero()
+    P64.spread(x, y, z, c)
+    want = P64.finish(+1, want_imag=True)
     for values in (c, c):  # a second pass over one sort
         P.sort_points(x, y, z)
         P.spread_zero()
