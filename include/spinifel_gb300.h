@@ -184,6 +184,9 @@ int spf_nufft_sort_orient(spf_nufft_plan plan, const float *d_quats, int64_t n_o
  * from d_x, d_y, d_z, which must stay valid. */
 int spf_nufft_sort_points(spf_nufft_plan plan, const float *d_x, const float *d_y,
                           const float *d_z, int64_t n, void *stream);
+/* How many sorts the plan has made (0: none): tells whether the sorted points
+ * it holds are still those of an earlier sort. */
+int64_t spf_nufft_sort_count(spf_nufft_plan plan);
 int spf_nufft_interp_spread_sorted(spf_nufft_plan plan, const float *d_weights, void *stream);
 /* Type-1 spreading of real values (d_values[o*n_pix + p], or 1 for every
  * point when NULL) over the points sorted by spf_nufft_sort_orient, into the

@@ -84,6 +84,7 @@ SIGNATURES = {
                              _int, _dbl, _c_void_p],
     "spf_nufft_sort_orient": [_c_void_p, _c_void_p, _i64, _c_void_p, _i64, _dbl, _c_void_p],
     "spf_nufft_sort_points": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _i64, _c_void_p],
+    "spf_nufft_sort_count": [_c_void_p],
     "spf_nufft_interp_spread_sorted": [_c_void_p, _c_void_p, _c_void_p],
     "spf_nufft_spread_sorted": [_c_void_p, _c_void_p, _c_void_p],
     "spf_nufft_t1_spread_det": [_c_void_p, _c_void_p, _i64, _c_void_p, _int, _int, _int, _dbl,
@@ -204,6 +205,7 @@ _RESTYPES = {
     "spf_last_error": ctypes.c_char_p,
     "spf_launch_count": ctypes.c_uint64,
     "spf_argmin_f64_work_bytes": ctypes.c_int64,
+    "spf_nufft_sort_count": ctypes.c_int64,
     "spf_dist_topk_bf16_tiles": ctypes.c_int64,
     "spf_dist_topk_bf16_work_bytes": ctypes.c_int64,
     "spf_dist_topk_bf16_tile_refs": ctypes.c_int64,

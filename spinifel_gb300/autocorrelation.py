@@ -92,8 +92,9 @@ SORTED_SPREAD_MIN_POINTS = 1 << 17
 def adjoint(nuvect, H_, K_, L_, M, use_recip_sym=True, support=None, eps=DEFAULT_EPS,
             isign=+1, plan=None, sort=None):
     """Type 1 onto M^3 (isign +1), times support, real part, divided by M^3.
-    sort: None picks the sorted spreading for large point sets; True / False
-    forces it on or off."""
+    sort: None picks the sorted spreading for large point sets (a smaller one
+    never replaces points that the plan's caller sorted: NufftPlan.may_sort);
+    True / False forces it on or off."""
     if _numel(H_):
         assert _max_abs(H_, K_, L_) < 3 * np.pi
     P = plan if plan is not None else plan_for(M, eps)
@@ -103,10 +104,13 @@ def adjoint(nuvect, H_, K_, L_, M, use_recip_sym=True, support=None, eps=DEFAULT
     c = c.to(_arrays.device()).reshape(-1)
     cre = (c.real if torch.is_complex(c) else c).to(P.dtype).contiguous()
     cim = c.imag.to(P.dtype).contiguous() if torch.is_complex(c) else None
+    auto = sort is None and hasattr(P, "may_sort")
     use_sorted = (x.numel() >= SORTED_SPREAD_MIN_POINTS) if sort is None else bool(sort)
-    use_sorted = use_sorted and P.supports_sort
+    use_sorted = use_sorted and P.supports_sort and (not auto or P.may_sort(x.numel()))
     if use_sorted:
         P.sort_points(x, y, z)
+        if auto:
+            P.sorted_automatically()
 
     def spread(values):
         if use_sorted:

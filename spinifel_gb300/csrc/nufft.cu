@@ -46,6 +46,7 @@ struct spf_nufft_plan_s {
   int4 *items = nullptr;     // (bin, start, count, 0) work items, their number in bins
   int32_t *bins = nullptr;   // per bin: points, then next free place; the two totals
   int64_t n_sorted = 0, max_items = 0, sorted_cap = 0, items_cap = 0;
+  int64_t sort_count = 0;    // sorts made so far: which set of points the plan holds
   int nb[3] = {0, 0, 0};
 };
 
@@ -1812,6 +1813,7 @@ static int sort_points(spf_nufft_plan P, PointSrc src, int64_t n, double scale, 
   // items: one per non-empty bin and one more per full chunk at most
   const int64_t max_items = (n < n_bins ? n : n_bins) + n / chunk;
   P->n_sorted = 0;
+  ++P->sort_count;
   if (!P->bins)
     SPF_TRY(check_cuda(cudaMalloc(&P->bins, (2 * n_bins + 2) * sizeof(int32_t)), "spf_nufft_sort"));
   if (n > P->sorted_cap) {
@@ -1888,6 +1890,8 @@ int spf_nufft_sort_points(spf_nufft_plan P, const float *d_x, const float *d_y,
   SPF_REQUIRE(n == 0 || (d_x && d_y && d_z), "spf_nufft_sort_points: NULL pointer");
   return sort_points(P, PointSrc{nullptr, nullptr, 1, d_x, d_y, d_z}, n, 1.0, stream);
 }
+
+int64_t spf_nufft_sort_count(spf_nufft_plan P) { return P ? P->sort_count : 0; }
 
 static int sorted_pass(spf_nufft_plan P, const float *d_weights, bool interp, const char *what,
                        void *stream) {

@@ -139,6 +139,23 @@ class NufftPlan:
     # the patch kernel (2.1e9 points/s; the sort and its pass take as long at
     # about 1.5e5 points) or the thread-per-point kernel
     SORTED_MIN_POINTS = 1 << 18
+    # up to this many points an automatic sort never replaces points that the
+    # caller sorted (sort_points, sort=True, MergeOperator.set_direct): passes
+    # over them would read the others.  From here on (2.0e6 points: 3.4 ms one
+    # by one, 0.7 sorted) it sorts whatever the plan holds.
+    KEEP_SORT_POINTS = 1 << 21
+    _auto_sort = 0  # spf_nufft_sort_count of the last automatic sort
+
+    def may_sort(self, n: int) -> bool:
+        """Whether an automatic choice may bin-sort n points on this plan."""
+        if n >= self.KEEP_SORT_POINTS or not self._h:
+            return True
+        return int(_lib.lib().spf_nufft_sort_count(self._h)) in (0, self._auto_sort)
+
+    def sorted_automatically(self):
+        """Notes that the points the plan holds are not its caller's."""
+        if self._h:
+            self._auto_sort = int(_lib.lib().spf_nufft_sort_count(self._h))
 
     def spread_orient(self, quats, ppr, scale, c, det_shape: tuple | None = None,
                       sort: bool | None = None):
@@ -149,12 +166,15 @@ class NufftPlan:
         c = c.to(device=self.device, dtype=torch.float32).contiguous()
         if c.numel() != quats.shape[0] * ppr.shape[1]:
             raise ValueError("strengths must be n_orient * n_pix")
-        if sort is None:
-            sort = c.numel() >= self.SORTED_MIN_POINTS
+        auto = sort is None
+        if auto:
+            sort = c.numel() >= self.SORTED_MIN_POINTS and self.may_sort(c.numel())
         if sort:
             self._sorted_points = (quats, ppr)
             _lib.call("spf_nufft_sort_orient", self._h, _lib.ptr(quats), quats.shape[0],
                       _lib.ptr(ppr), ppr.shape[1], float(scale), _lib.stream_handle())
+            if auto:
+                self.sorted_automatically()
             _lib.call("spf_nufft_spread_sorted", self._h, _lib.ptr(c), _lib.stream_handle())
         elif det_shape is not None and len(det_shape) == 3 and \
                 int(np.prod(det_shape)) == ppr.shape[1]:

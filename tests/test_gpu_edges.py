@@ -379,3 +379,52 @@ def test_split_tiles_give_the_same_lists(n_img, n_ref, n_pix):
     assert torch.equal(idx, pidx)
     assert torch.equal(dist, pdist)
     matching.check_device_error()
+
+
+def test_automatic_sort_leaves_the_callers_points():
+    """Points that a caller sorted on a plan stay its sorted points when an
+    automatic choice spreads others there (below 2^21): spread_sorted and the
+    direct merge operator give the same sums after as before (to the FP32
+    rounding of sums in another order)."""
+    from spinifel_gb300 import autocorrelation as ac
+    from spinifel_gb300 import geom
+    from spinifel_gb300.merge import MergeOperator, antisupport
+    from spinifel_gb300.nufft import NufftPlan
+
+    rng = np.random.default_rng(8)
+    M, n = 21, 1 << 18
+    P = NufftPlan(M, 1e-6)
+    mine, other = (tuple(torch.as_tensor(rng.uniform(-3, 3, n).astype(np.float32), device="cuda")
+                         for _ in range(3)) for _ in range(2))
+    c = torch.as_tensor(rng.random(n).astype(np.float32), device="cuda")
+    ppr, pdr = geom.flat_detector(4, 32, 32)
+    q = torch.as_tensor(geom.uniform_quaternions(n // 4096, rng).astype(np.float32),
+                        device="cuda")
+    ppr_t = torch.as_tensor(ppr.reshape(3, -1).astype(np.float32), device="cuda")
+    mult = np.pi / pdr.max()
+    half = tuple(v[:n // 2].contiguous() for v in other)
+
+    def spread():
+        P.spread_zero()
+        P.spread_sorted(c)
+        return P.finish(+1)[0]
+
+    P.sort_points(*mine)
+    want = spread()
+    P.spread_zero()
+    P.spread_orient(q, ppr_t, mult, c, det_shape=(4, 32, 32))
+    got = spread()
+    assert float((got - want).norm() / want.norm()) < 1e-5
+    a = ac.adjoint(c[:n // 2], *half, M, plan=P)
+    b = ac.adjoint(c[:n // 2], *half, M, plan=NufftPlan(M, 1e-6))
+    assert float((a - b).norm() / b.norm()) < 1e-4  # per-point sums against sorted ones
+    got = spread()
+    assert float((got - want).norm() / want.norm()) < 1e-5
+
+    op = MergeOperator(M, 2 * M, 1e-3, 1.0, torch.ones(M, M, M, device="cuda"), antisupport(M, 1))
+    op.set_direct(P, q, ppr_t, mult)
+    x = torch.as_tensor(rng.random(M ** 3), device="cuda")
+    want = op.apply(x, form=op.DIRECT)
+    ac.adjoint(c[:n // 2], *half, M, plan=P)
+    got = op.apply(x, form=op.DIRECT)
+    assert float((got - want).norm() / want.norm()) < 1e-5
