@@ -147,7 +147,11 @@ class NufftPlan:
     _auto_sort = 0  # spf_nufft_sort_count of the last automatic sort
 
     def may_sort(self, n: int) -> bool:
-        """Whether an automatic choice may bin-sort n points on this plan."""
+        """Whether an automatic choice may bin-sort n points on this plan: never
+        under graph capture, where a sort may not allocate, and a graph would
+        keep addresses that the next larger sort frees."""
+        if self.device.type == "cuda" and torch.cuda.is_current_stream_capturing():
+            return False
         if n >= self.KEEP_SORT_POINTS or not self._h:
             return True
         return int(_lib.lib().spf_nufft_sort_count(self._h)) in (0, self._auto_sort)

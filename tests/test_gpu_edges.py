@@ -428,3 +428,36 @@ def test_automatic_sort_leaves_the_callers_points():
     ac.adjoint(c[:n // 2], *half, M, plan=P)
     got = op.apply(x, form=op.DIRECT)
     assert float((got - want).norm() / want.norm()) < 1e-5
+
+
+def test_automatic_sort_is_not_captured():
+    """spread_orient at a size that it sorts by itself is captured unsorted,
+    on a plan that never sorted and on one that did; replays give the eager
+    sums."""
+    from spinifel_gb300 import geom
+    from spinifel_gb300.nufft import NufftPlan
+
+    rng = np.random.default_rng(9)
+    M, n = 21, 1 << 18
+    ppr, pdr = geom.flat_detector(4, 32, 32)
+    q = torch.as_tensor(geom.uniform_quaternions(n // 4096, rng).astype(np.float32),
+                        device="cuda")
+    ppr_t = torch.as_tensor(ppr.reshape(3, -1).astype(np.float32), device="cuda")
+    c = torch.as_tensor(rng.random(n).astype(np.float32), device="cuda")
+    mult = np.pi / pdr.max()
+    P = NufftPlan(M, 1e-6)
+
+    def step():
+        P.spread_zero()
+        P.spread_orient(q, ppr_t, mult, c, det_shape=(4, 32, 32))
+        return P.finish(+1)[0]
+
+    for _ in range(2):
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            out = step()
+        want = step()  # eager: sorted
+        g.replay()
+        torch.cuda.synchronize()
+        assert float((out - want).norm() / want.norm()) < 1e-5
