@@ -174,7 +174,7 @@ int spf_nufft_interp_spread_det(spf_nufft_plan plan, const float *d_quats, int64
  * places every point o*n_pix + p in its 8^3-cell bin of the padded fine grid
  * (a counting sort on the device; large bins split into 2048-point work
  * items) and keeps the order in the plan (allocates; synchronises the
- * stream once).  spf_nufft_interp_spread_sorted then does the fused
+ * stream once; refused under stream capture).  spf_nufft_interp_spread_sorted then does the fused
  * interpolate / weight / spread with each work item's grid box staged in
  * shared memory.  The points' geometry pointers must stay valid. */
 int spf_nufft_sort_orient(spf_nufft_plan plan, const float *d_quats, int64_t n_orient,

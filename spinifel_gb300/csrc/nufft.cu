@@ -1812,6 +1812,13 @@ static int sort_points(spf_nufft_plan P, PointSrc src, int64_t n, double scale, 
     chunk = n < BIN_CHUNK_FEW ? BIN_CHUNK / 2 : BIN_CHUNK;
   // items: one per non-empty bin and one more per full chunk at most
   const int64_t max_items = (n < n_bins ? n : n_bins) + n / chunk;
+  // a graph would keep addresses that the next larger sort frees
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  SPF_TRY(check_cuda(cudaStreamIsCapturing(s, &capture), "spf_nufft_sort"));
+  if (capture != cudaStreamCaptureStatusNone) {
+    set_error("spf_nufft_sort: points cannot be sorted under stream capture");
+    return SPF_ERR_UNSUPPORTED;
+  }
   P->n_sorted = 0;
   ++P->sort_count;
   if (!P->bins)

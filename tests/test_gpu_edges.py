@@ -461,3 +461,30 @@ def test_automatic_sort_is_not_captured():
         g.replay()
         torch.cuda.synchronize()
         assert float((out - want).norm() / want.norm()) < 1e-5
+
+
+def test_sorts_are_refused_under_capture():
+    """A sort called for under graph capture is an error (also where it would
+    not have to allocate), and the plan's sorted points stay usable."""
+    from spinifel_gb300 import _lib
+    from spinifel_gb300.nufft import NufftPlan
+
+    rng = np.random.default_rng(10)
+    P = NufftPlan(21, 1e-6)
+    pts = tuple(torch.as_tensor(rng.uniform(-3, 3, 3000).astype(np.float32), device="cuda")
+                for _ in range(3))
+
+    def spread():
+        P.spread_zero()
+        P.spread_sorted()
+        return P.finish(+1)[0]
+
+    P.sort_points(*pts)
+    want = spread()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with pytest.raises(_lib.SpfError, match="capture"):
+        with torch.cuda.graph(g):
+            P.sort_points(*pts)
+    got = spread()
+    assert float((got - want).norm() / want.norm()) < 1e-5
