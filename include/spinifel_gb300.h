@@ -172,16 +172,19 @@ int spf_nufft_interp_spread_det(spf_nufft_plan plan, const float *d_quats, int64
 /* Bin-sorted points for repeated type 2 -> type 1 products over a fixed set
  * of orientation points (the direct merge operator): spf_nufft_sort_orient
  * places every point o*n_pix + p in its 8^3-cell bin of the padded fine grid
- * (a counting sort on the device; large bins split into 2048-point work
- * items) and keeps the order in the plan (allocates; synchronises the
- * stream once; refused under stream capture).  spf_nufft_interp_spread_sorted then does the fused
+ * (a counting sort on the device; large bins split into work items of
+ * SPF_TUNE_SORT_ITEM points) and keeps the sorted points, 16 bytes each, in the
+ * plan (allocates; refused under stream capture).  It returns before the sort
+ * has run; passes over the sorted points and later sorts wait for it on
+ * whatever stream they are enqueued (a pass that is captured in a graph
+ * does not: synchronise before the capture).  The geometry arrays are read by
+ * the sort alone.  spf_nufft_interp_spread_sorted then does the fused
  * interpolate / weight / spread with each work item's grid box staged in
- * shared memory.  The points' geometry pointers must stay valid. */
+ * shared memory. */
 int spf_nufft_sort_orient(spf_nufft_plan plan, const float *d_quats, int64_t n_orient,
                           const float *d_ppr, int64_t n_pix, double scale, void *stream);
 /* The same bin sort for n explicit points (coordinates in radians, as
- * spf_nufft_t1_spread takes them); the sorted passes then read the points
- * from d_x, d_y, d_z, which must stay valid. */
+ * spf_nufft_t1_spread takes them). */
 int spf_nufft_sort_points(spf_nufft_plan plan, const float *d_x, const float *d_y,
                           const float *d_z, int64_t n, void *stream);
 /* How many sorts the plan has made (0: none): tells whether the sorted points

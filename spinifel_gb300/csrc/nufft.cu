@@ -47,6 +47,7 @@ struct spf_nufft_plan_s {
   int32_t *bins = nullptr;   // per bin: points, then next free place; the two totals
   int64_t n_sorted = 0, max_items = 0, sorted_cap = 0, items_cap = 0;
   int64_t sort_count = 0;    // sorts made so far: which set of points the plan holds
+  cudaEvent_t sorted_use = nullptr;  // after the last sort or pass over the sorted points
   int nb[3] = {0, 0, 0};
 };
 
@@ -1554,6 +1555,7 @@ int spf_nufft_plan_destroy(spf_nufft_plan P) {
   cudaFree(P->sorted);
   cudaFree(P->items);
   cudaFree(P->bins);
+  if (P->sorted_use) cudaEventDestroy(P->sorted_use);
   if (P->fft_ok) cufftDestroy(P->fft);
   if (prev != P->dev && prev >= 0) cudaSetDevice(prev);
   delete P;
@@ -1797,6 +1799,15 @@ int spf_nufft_interp_spread_det(spf_nufft_plan P, const float *d_quats, int64_t 
 }
 
 // bin sort of n points (orientation or explicit) for the sorted passes
+// Sorts and passes over the sorted points run one after the other whatever
+// their streams: each waits for the one before it (a sort makes its tables on
+// the device and returns before they are there).
+static int order_sorted_use(spf_nufft_plan P, cudaStream_t s, const char *what) {
+  if (P->sorted_use)
+    return check_cuda(cudaStreamWaitEvent(s, P->sorted_use, 0), what);
+  return check_cuda(cudaEventCreateWithFlags(&P->sorted_use, cudaEventDisableTiming), what);
+}
+
 static int sort_points(spf_nufft_plan P, PointSrc src, int64_t n, double scale, void *stream) {
   SPF_REQUIRE(n < (1LL << 31), "spf_nufft_sort: more than 2^31 points");
   cudaStream_t s = as_stream(stream);
@@ -1819,6 +1830,7 @@ static int sort_points(spf_nufft_plan P, PointSrc src, int64_t n, double scale, 
     set_error("spf_nufft_sort: points cannot be sorted under stream capture");
     return SPF_ERR_UNSUPPORTED;
   }
+  SPF_TRY(order_sorted_use(P, s, "spf_nufft_sort"));
   P->n_sorted = 0;
   ++P->sort_count;
   if (!P->bins)
@@ -1876,7 +1888,7 @@ static int sort_points(spf_nufft_plan P, PointSrc src, int64_t n, double scale, 
                             g, bd, P->items, totals + 1, P->sorted, chunk)));
   SPF_TRY(check_launch("k_item_cellsort"));
   P->n_sorted = n;
-  return SPF_OK;
+  return check_cuda(cudaEventRecord(P->sorted_use, s), "spf_nufft_sort");
 }
 
 int spf_nufft_sort_orient(spf_nufft_plan P, const float *d_quats, int64_t n_orient,
@@ -1905,6 +1917,11 @@ static int sorted_pass(spf_nufft_plan P, const float *d_weights, bool interp, co
   SPF_TRY(check_plan(P, what));
   if (P->n_sorted == 0) return SPF_OK;
   cudaStream_t s = as_stream(stream);
+  // a captured pass cannot wait for work outside its graph: its caller orders it
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  SPF_TRY(check_cuda(cudaStreamIsCapturing(s, &capture), what));
+  const bool ordered = capture == cudaStreamCaptureStatusNone;
+  if (ordered) SPF_TRY(order_sorted_use(P, s, what));
   GridGeom g = geom_of(P);
   BinDims bd;
   for (int d = 0; d < 3; ++d) bd.nb[d] = P->nb[d];
@@ -1937,7 +1954,8 @@ static int sorted_pass(spf_nufft_plan P, const float *d_weights, bool interp, co
                              P->acc_pad, g, bd, P->items, n_items, P->sorted, d_weights,
                              device_error_word())));
   }
-  return check_launch(what);
+  SPF_TRY(check_launch(what));
+  return ordered ? check_cuda(cudaEventRecord(P->sorted_use, s), what) : SPF_OK;
 }
 
 int spf_nufft_interp_spread_sorted(spf_nufft_plan P, const float *d_weights, void *stream) {

@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+import threading
 
 import numpy as np
 
@@ -145,6 +146,7 @@ class NufftPlan:
     # by one, 0.7 sorted) it sorts whatever the plan holds.
     KEEP_SORT_POINTS = 1 << 21
     _auto_sort = 0  # spf_nufft_sort_count of the last automatic sort
+    _sort_lock = threading.RLock()  # keeps a sort and its pass together, for all plans
 
     def may_sort(self, n: int) -> bool:
         """Whether an automatic choice may bin-sort n points on this plan: never
@@ -171,16 +173,18 @@ class NufftPlan:
         if c.numel() != quats.shape[0] * ppr.shape[1]:
             raise ValueError("strengths must be n_orient * n_pix")
         auto = sort is None
-        if auto:
-            sort = c.numel() >= self.SORTED_MIN_POINTS and self.may_sort(c.numel())
-        if sort:
-            self._sorted_points = (quats, ppr)
-            _lib.call("spf_nufft_sort_orient", self._h, _lib.ptr(quats), quats.shape[0],
-                      _lib.ptr(ppr), ppr.shape[1], float(scale), _lib.stream_handle())
+        with self._sort_lock:
             if auto:
-                self.sorted_automatically()
-            _lib.call("spf_nufft_spread_sorted", self._h, _lib.ptr(c), _lib.stream_handle())
-        elif det_shape is not None and len(det_shape) == 3 and \
+                sort = c.numel() >= self.SORTED_MIN_POINTS and self.may_sort(c.numel())
+            if sort:
+                self._sorted_points = (quats, ppr)
+                _lib.call("spf_nufft_sort_orient", self._h, _lib.ptr(quats), quats.shape[0],
+                          _lib.ptr(ppr), ppr.shape[1], float(scale), _lib.stream_handle())
+                if auto:
+                    self.sorted_automatically()
+                _lib.call("spf_nufft_spread_sorted", self._h, _lib.ptr(c), _lib.stream_handle())
+                return
+        if det_shape is not None and len(det_shape) == 3 and \
                 int(np.prod(det_shape)) == ppr.shape[1]:
             _lib.call("spf_nufft_t1_spread_det", self._h, _lib.ptr(quats), quats.shape[0],
                       _lib.ptr(ppr), int(det_shape[0]), int(det_shape[1]), int(det_shape[2]),
@@ -195,9 +199,10 @@ class NufftPlan:
         coordinate tensors are kept alive by the plan."""
         x, y, z = (t.to(device=self.device, dtype=torch.float32).contiguous().reshape(-1)
                    for t in (x, y, z))
-        self._sorted_points = (x, y, z)
-        _lib.call("spf_nufft_sort_points", self._h, _lib.ptr(x), _lib.ptr(y), _lib.ptr(z),
-                  x.numel(), _lib.stream_handle())
+        with self._sort_lock:
+            self._sorted_points = (x, y, z)
+            _lib.call("spf_nufft_sort_points", self._h, _lib.ptr(x), _lib.ptr(y), _lib.ptr(z),
+                      x.numel(), _lib.stream_handle())
 
     def spread_sorted(self, c=None):
         """Type-1 spreading of c (or ones) over the points of the last sort

@@ -488,3 +488,60 @@ def test_sorts_are_refused_under_capture():
             P.sort_points(*pts)
     got = spread()
     assert float((got - want).norm() / want.norm()) < 1e-5
+
+
+def test_sorted_points_are_ordered_across_streams():
+    """Sorts and passes over a plan's sorted points run in the order of their
+    calls on whatever streams: a pass on another stream than its sort's
+    waits for the sort, and the next sort for the pass."""
+    from spinifel_gb300 import geom
+    from spinifel_gb300.nufft import NufftPlan
+
+    rng = np.random.default_rng(11)
+    M, n = 21, 1 << 18
+    P = NufftPlan(M, 1e-6)
+    ppr, pdr = geom.flat_detector(4, 32, 32)
+    ppr_t = torch.as_tensor(ppr.reshape(3, -1).astype(np.float32), device="cuda")
+    quats = [torch.as_tensor(geom.uniform_quaternions(n // 4096, rng).astype(np.float32),
+                             device="cuda") for _ in range(2)]
+    pts = tuple(torch.as_tensor(rng.uniform(-3, 3, n).astype(np.float32), device="cuda")
+                for _ in range(3))
+    c = torch.as_tensor(rng.random(n).astype(np.float32), device="cuda")
+    mult = np.pi / pdr.max()
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+
+    def sums(a, b):
+        """two orientation spreads of one sum, a's stream held up"""
+        P.spread_zero()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(a):
+            if a is not b:
+                torch.cuda._sleep(20_000_000)  # about 10 ms
+            P.spread_orient(quats[0], ppr_t, mult, c)
+        with torch.cuda.stream(b):
+            P.spread_orient(quats[1], ppr_t, mult, c)
+        torch.cuda.synchronize()
+        return P.finish(+1)[0]
+
+    want = sums(s1, s1)
+    for a, b in ((s1, s2), (s2, s1)):
+        got = sums(a, b)
+        assert float((got - want).norm() / want.norm()) < 1e-5
+
+    def passed(a, b):
+        P.spread_zero()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(a):
+            if a is not b:
+                torch.cuda._sleep(20_000_000)
+            P.sort_points(*pts)
+        with torch.cuda.stream(b):
+            P.spread_sorted(c)
+            out = P.finish(+1)[0]
+        torch.cuda.synchronize()
+        return out
+
+    want = passed(s1, s1)
+    P.sort_points(*(v.flip(0) for v in pts))
+    got = passed(s1, s2)
+    assert float((got - want).norm() / want.norm()) < 1e-5
