@@ -82,10 +82,12 @@ int spf_selftest_bounded_wait(int64_t timeout_ms, int *d_result, void *stream);
  *                           below 2^22 points; 256 .. 8192)
  *   SPF_TUNE_STATIC_ABORT_TEST : 1 makes spf_match_bf16_static record a
  *                           given-up GEMM wait (SPF_ERR_TIMEOUT in its
- *                           error word, after the GEMM) so that tests can
- *                           check the void answers and the report through
- *                           spf_device_error without a device hang; 0
- *                           (default) in production */
+ *                           error word, after the GEMM), and the re-rank of
+ *                           up to 13 frames an SM treat every odd frame as
+ *                           one whose copies gave no sign, so that tests can
+ *                           check the void answers, their completion and the
+ *                           report through spf_device_error without a device
+ *                           hang; 0 (default) in production */
 #define SPF_TUNE_BF16_GROUP_M 1
 #define SPF_TUNE_FP32_GROUP_M 2
 #define SPF_TUNE_BF16_GRID 3

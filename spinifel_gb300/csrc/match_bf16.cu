@@ -940,7 +940,7 @@ __global__ void __launch_bounds__(RF_THREADS)
                    float *__restrict__ work, int32_t *__restrict__ out_idx,
                    float *__restrict__ out_dist, int32_t *__restrict__ uncertified,
                    int32_t *__restrict__ out_top, unsigned int *__restrict__ err,
-                   int ring_floats) {
+                   int ring_floats, int late_odd) {
   extern __shared__ __align__(16) float ring[];  // ring_floats
   __shared__ __align__(8) uint64_t full[RF_MAX_STAGES], empty[RF_MAX_STAGES];
   __shared__ int late;
@@ -953,7 +953,7 @@ __global__ void __launch_bounds__(RF_THREADS)
       mbar_init(&full[s], vec ? 1 : 32);
       mbar_init(&empty[s], 1);
     }
-    late = 0;
+    late = late_odd && (im & 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // candidates whose rows are read: an index outside [0, n_ref) (a candidate
@@ -971,6 +971,7 @@ __global__ void __launch_bounds__(RF_THREADS)
   const int stages = min(RF_MAX_STAGES, ring_floats / (nr * (C + 4)));
   __syncthreads();
   float acc = 0.0f;
+  int64_t ch = 0;  // warp 1: chunks whose copies were issued
   if (warp == 1) {
     // lane r < nr copies row r
     const float *src = img + im * n_pix;
@@ -982,7 +983,6 @@ __global__ void __launch_bounds__(RF_THREADS)
     const int64_t nchunks = (n_pix + C - 1) / C;
     int s = 0;
     uint32_t ph = 1;  // the first round finds every stage empty
-    int64_t ch = 0;
     for (; ch < nchunks; ++ch) {
       if (!__all_sync(0xffffffffu, mbar_wait_for(&empty[s], ph, TIMEOUT_NS))) break;
       const int64_t base = ch * C;
@@ -1008,12 +1008,7 @@ __global__ void __launch_bounds__(RF_THREADS)
         ph ^= 1;
       }
     }
-    if (ch < nchunks) {
-      // the chains gave up: let the copies in flight land before the CTA ends
-      late = 1;
-      for (int64_t f = ch > stages ? ch - stages : 0; f < ch; ++f)
-        mbar_wait_for(&full[f % stages], (uint32_t)((f / stages) & 1), TIMEOUT_NS);
-    }
+    if (ch < nchunks) late = 1;
   } else {
     const bool ok = C == 256   ? rerank_chain<256>(ring, slot, nr, stages, n_pix, full, empty, acc)
                     : C == 128 ? rerank_chain<128>(ring, slot, nr, stages, n_pix, full, empty, acc)
@@ -1021,15 +1016,21 @@ __global__ void __launch_bounds__(RF_THREADS)
     if (!ok) late = 1;
   }
   __syncthreads();
+  // either side gave up: the copies in flight land before the CTA ends
+  if (late && warp == 1)
+    for (int64_t f = ch > stages ? ch - stages : 0; f < ch; ++f)
+      mbar_wait_for(&full[f % stages], (uint32_t)((f / stages) & 1), TIMEOUT_NS);
   if (threadIdx.x >= TOPK) return;
   if (late) {
-    // a copy gave no sign within the bound: report it, the frame has no answer
+    // a copy gave no sign within the bound: report it; the frame has no answer
+    // and is left open, to be searched among all references
     if (out_top) out_top[im * TOPK + c] = -1;
     if (c == 0) {
       if (err) atomicExch(err, (unsigned int)(-SPF_ERR_TIMEOUT));
       out_idx[im] = -1;
       if (out_dist) out_dist[im] = __int_as_float(0x7fc00000);
-      if (uncertified) uncertified[im] = 0;
+      if (uncertified) uncertified[im] = 1;
+      work[im] = __int_as_float(0x7f800000);
     }
     return;
   }
@@ -1217,7 +1218,8 @@ static int launch_rerank(const float *cand_d, const int32_t *cand_i, const float
     const int ring = n_img <= (int64_t)RF_RESIDENT_FEW * sm_count() ? RF_RING_FEW : RF_RING_MANY;
     k_rerank_frame<<<(unsigned)n_img, RF_THREADS, ring * sizeof(float), s>>>(
         cand_d, cand_i, img, img_sq, n_img, ref, ref_sq, n_ref, ref_sq_max, n_pix, ref_offset,
-        work, idx, dist, uncertified, top8, err, ring);
+        work, idx, dist, uncertified, top8, err, ring,
+        (int)tune_get(SPF_TUNE_STATIC_ABORT_TEST, 0));
     return check_launch("k_rerank_frame");
   }
   SPF_TRY(rerank_smem_attr());
@@ -1441,7 +1443,8 @@ namespace bf16mm {
 // The tile lists hold each tile's 8 smallest approximate distances, so they
 // contain every in-bound reference of the tile unless all 8 are in bound: the
 // tile may then hold more, and count[r] is set above the cap so that the
-// caller searches that frame by the range GEMM.
+// caller searches that frame by the range GEMM.  So it is for an infinite
+// bound, that of a frame about which nothing is known.
 __global__ void __launch_bounds__(256)
     k_scan_band(const float *__restrict__ cand_d, const int32_t *__restrict__ cand_i,
                 int64_t n_tiles, int64_t n_img, const int64_t *__restrict__ rows,
@@ -1453,7 +1456,7 @@ __global__ void __launch_bounds__(256)
   const float T = thresh[r];
   if (threadIdx.x == 0) {
     cnt = 0;
-    sat = 0;
+    sat = T == __int_as_float(0x7f800000);
   }
   __syncthreads();
   for (int64_t t = threadIdx.x; t < n_tiles; t += blockDim.x) {

@@ -545,3 +545,36 @@ def test_sorted_points_are_ordered_across_streams():
     P.sort_points(*(v.flip(0) for v in pts))
     got = passed(s1, s2)
     assert float((got - want).norm() / want.norm()) < 1e-5
+
+
+def _match_operands(n_img, n_ref, n_pix, seed):
+    from spinifel_gb300 import matching
+
+    rng = np.random.default_rng(seed)
+    refs = rng.gamma(0.5, 1.0, (n_ref, n_pix)).astype(np.float32)
+    x = rng.poisson(refs[rng.integers(0, n_ref, n_img)]).astype(np.float32)
+    fr = matching.FrameSet(torch.as_tensor(x, device="cuda"))
+    return fr, matching.ReferenceSet(torch.as_tensor(refs, device="cuda"))
+
+
+@pytest.mark.parametrize("n_pix", [1024, 1001])
+def test_late_rerank_frames_are_left_open(n_pix):
+    """Frames whose re-rank gave up a wait (the test switch: every odd frame)
+    are reported and uncertified, and their completion searches all references."""
+    from spinifel_gb300 import _lib, matching
+
+    fr, rs = _match_operands(9, 700, n_pix, 12)
+    want_i, want_d = matching.argmin_fp32(fr.f32, rs.f32, images_sq=fr.sq, refs_sq=rs.sq)
+    _lib.call("spf_tune_set", _lib.SPF_TUNE_STATIC_ABORT_TEST, 1)
+    try:
+        raw_i, raw_d = matching.match_bf16(fr, rs, exact_fallback=False)
+        st = {}
+        idx, dist = matching.match_bf16(fr, rs, stats=st)
+    finally:
+        _lib.call("spf_tune_set", _lib.SPF_TUNE_STATIC_ABORT_TEST, 0)
+    with pytest.raises(_lib.SpfError, match="gave up"):
+        matching.check_device_error()
+    assert bool((raw_i[1::2] == -1).all()) and bool(raw_d[1::2].isnan().all())
+    assert st["uncertified"] >= 4
+    assert torch.equal(idx.to(want_i.dtype), want_i) and torch.equal(dist, want_d)
+    matching.check_device_error()
