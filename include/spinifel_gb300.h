@@ -82,9 +82,10 @@ int spf_selftest_bounded_wait(int64_t timeout_ms, int *d_result, void *stream);
  *                           below 2^22 points; 256 .. 8192)
  *   SPF_TUNE_STATIC_ABORT_TEST : 1 makes spf_match_bf16_static record a
  *                           given-up GEMM wait (SPF_ERR_TIMEOUT in its
- *                           error word, after the GEMM), and the re-rank of
- *                           up to 13 frames an SM treat every odd frame as
- *                           one whose copies gave no sign, so that tests can
+ *                           error word, after the GEMM), the other bf16
+ *                           GEMMs give up at each CTA's last tile, and the
+ *                           re-rank of up to 13 frames an SM treat every odd
+ *                           frame as one whose copies gave no sign, so that tests can
  *                           check the void answers, their completion and the
  *                           report through spf_device_error without a device
  *                           hang; 0 (default) in production */
@@ -456,7 +457,10 @@ int spf_dist_topk_bf16_work(const void *d_img_bf16, int64_t n_img, const void *d
  * per-pixel max over references of s^2 (spf_col_maxsq_f32), ref_sq_max the
  * largest s2; d_work (n_img floats) is scratch that on return holds each
  * frame's search bound for spf_dist_range_bf16.  d_top8 (may be NULL)
- * receives the 8 candidates. */
+ * receives the 8 candidates.  A frame without an answer because a bounded wait
+ * ran out, here or in the GEMM (which marks the lists of the tiles that it left
+ * out), gets index -1, distance NaN, uncertified 1 and the bound +infinity,
+ * with which its completion searches all references. */
 int spf_rerank_fp32(float *d_cand_d, int32_t *d_cand_i, int64_t n_tiles,
                     const float *d_img, const float *d_img_sq, int64_t n_img,
                     const float *d_ref, const float *d_ref_sq, const float *d_ref_m2,

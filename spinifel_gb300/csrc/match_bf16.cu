@@ -182,6 +182,14 @@ __device__ __forceinline__ void tile_of(int64_t t, int64_t n_m, int64_t n_n, int
 //        k_split_top8 adds them up.
 enum class Out { TOP8, RANGE, SPLIT };
 
+// Tiles that a CTA leaves out after a wait has run out are marked, so that their
+// frames are left open and not answered from what the buffers held before: a
+// list that starts with reference LOST_TILE (TOP8), a count above the cap
+// (RANGE), a row of products that starts with the bits LOST_PART (SPLIT; a NaN
+// that no product has).
+constexpr int32_t LOST_TILE = -1;
+constexpr uint32_t LOST_PART = 0x7fffdeadu;
+
 template <Out OUT>
 __global__ void __launch_bounds__(THREADS, 1)
     k_dist_topk_bf16(const __grid_constant__ CUtensorMap tmap_a,
@@ -189,7 +197,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                      int64_t n_img, int64_t n_ref, int64_t n_pix, float *__restrict__ cand_d,
                      int32_t *__restrict__ cand_i, const float *__restrict__ thresh,
                      int32_t *__restrict__ list, int32_t *__restrict__ count, int cap,
-                     int group_m, unsigned int *__restrict__ err, int splits) {
+                     int group_m, unsigned int *__restrict__ err, int splits, int give_up) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -316,13 +324,20 @@ __global__ void __launch_bounds__(THREADS, 1)
     // ---------------- epilogue (warps 2..5) ----------------
     const int q = warp & 3;  // TMEM lane quarter this warp may access
     uint32_t tc = 0;
-    for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x, ++tc) {
+    int64_t t = blockIdx.x;
+    for (; t < n_tiles; t += gridDim.x, ++tc) {
       int64_t m, n;
       tile_of(t / S, n_m, n_n, group_m, m, n);
       uint32_t b = tc & 1, use = tc >> 1;
       // one lane waits, the warp follows (tcgen05.ld below is warp-collective)
       int ok = 1;
-      if (lane == 0) ok = mbar_wait(&acc_full[b], use & 1, abort) ? 1 : 0;
+      if (lane == 0) {
+        ok = mbar_wait(&acc_full[b], use & 1, abort) ? 1 : 0;
+        if (give_up && t + gridDim.x >= n_tiles) {  // test: as if it had run out
+          *abort = 1;
+          ok = 0;
+        }
+      }
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) break;
       tc_fence_after();
@@ -394,6 +409,23 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
       }
     }
+    for (; t < n_tiles; t += gridDim.x) {  // after a wait that ran out
+      int64_t m, n;
+      tile_of(t / S, n_m, n_n, group_m, m, n);
+      const int64_t row = m * BM + q * 32 + lane;
+      if (row >= n_img) continue;
+      if constexpr (OUT == Out::SPLIT) {
+        cand_d[(((t % S) * n_n + n) * n_img + row) * BN] = __uint_as_float(LOST_PART);
+      } else if constexpr (OUT == Out::RANGE) {
+        atomicMax(count + row, cap + 1);
+      } else {
+        const size_t base = ((size_t)n * n_img + row) * TOPK;
+        for (int k = 0; k < TOPK; ++k) {
+          cand_d[base + k] = __int_as_float(k == 0 ? 0xff800000 : 0x7f800000);
+          cand_i[base + k] = k == 0 ? LOST_TILE : INT32_MAX;
+        }
+      }
+    }
   }
 
   __syncthreads();
@@ -423,11 +455,17 @@ __global__ void __launch_bounds__(256)
   float v[PER];
 #pragma unroll
   for (int u = 0; u < PER; ++u) v[u] = 0.0f;
+  bool lost = false;
   for (int s = 0; s < splits; ++s) {  // a part's loads are in flight together
     const float *src = part + ((int64_t)s * n_n * n_img + row) * BN + lane;
+    float p[PER];
 #pragma unroll
-    for (int u = 0; u < PER; ++u) v[u] += __ldg(src + u * 32);
+    for (int u = 0; u < PER; ++u) p[u] = __ldg(src + u * 32);
+    lost |= lane == 0 && __float_as_uint(p[0]) == LOST_PART;
+#pragma unroll
+    for (int u = 0; u < PER; ++u) v[u] += p[u];
   }
+  lost = __any_sync(0xffffffffu, lost);
 #pragma unroll
   for (int u = 0; u < PER; ++u) {
     const int64_t col = n * BN + u * 32 + lane;
@@ -458,8 +496,9 @@ __global__ void __launch_bounds__(256)
     }
     if (bc < BN && (bc & 31) == lane) taken |= 1u << (bc >> 5);
     if (lane == 0) {
-      od[r] = bv;
-      oi[r] = bc < BN ? (int32_t)(n * BN + bc) : INT32_MAX;
+      od[r] = lost ? __int_as_float(r == 0 ? 0xff800000 : 0x7f800000) : bv;
+      oi[r] = lost ? (r == 0 ? LOST_TILE : INT32_MAX)
+                   : bc < BN ? (int32_t)(n * BN + bc) : INT32_MAX;
     }
   }
 }
@@ -743,9 +782,21 @@ __device__ __forceinline__ void rerank_finish(
       jj = oj;
     }
   }
+  // a tile of the frame's was left out: it has no answer and is left open, to
+  // be searched among all references
+  const bool lost =
+      ((__ballot_sync(mask, j == LOST_TILE) >> (threadIdx.x & 24)) & 0xffu) != 0;
   if (!live) return;
-  if (out_top) out_top[im * TOPK + c] = (j == INT32_MAX) ? -1 : (int32_t)(j + ref_offset);
+  if (out_top)
+    out_top[im * TOPK + c] = lost || j == INT32_MAX ? -1 : (int32_t)(j + ref_offset);
   if (c != 0) return;
+  if (lost) {
+    out_idx[im] = -1;
+    if (out_dist) out_dist[im] = __int_as_float(0x7fc00000);
+    if (uncertified) uncertified[im] = 1;
+    work[im] = __int_as_float(0x7f800000);
+    return;
+  }
   out_idx[im] = jj == INT32_MAX ? -1 : (int32_t)(jj + ref_offset);
   if (out_dist) out_dist[im] = dist;
   if (!uncertified) return;
@@ -1305,22 +1356,23 @@ static int launch_bf16(Out out, int splits, float *d_part, const void *d_img_bf1
   int64_t max_grid = tune_get(SPF_TUNE_BF16_GRID, sm_count());
   int grid = (int)(tiles < max_grid ? tiles : max_grid);
   int group_m = (int)tune_get(SPF_TUNE_BF16_GROUP_M, GROUP_M);
+  const int give_up = (int)tune_get(SPF_TUNE_STATIC_ABORT_TEST, 0);
   cudaStream_t s = as_stream(stream);
   if (out == Out::RANGE) {
     k_dist_topk_bf16<Out::RANGE><<<grid, THREADS, SMEM_BYTES, s>>>(
         ma, mb, d_ref_sq, n_img, n_ref, n_pix, nullptr, nullptr, d_thresh, d_list, d_count, cap,
-        group_m, err, 1);
+        group_m, err, 1, give_up);
   } else if (out == Out::SPLIT) {
     k_dist_topk_bf16<Out::SPLIT><<<grid, THREADS, SMEM_BYTES, s>>>(
         ma, mb, d_ref_sq, n_img, n_ref, n_pix, d_part, nullptr, nullptr, nullptr, nullptr, 0,
-        group_m, err, splits);
+        group_m, err, splits, give_up);
     SPF_TRY(check_launch(name));
     k_split_top8<<<grid_for(n_n * n_img, 8), 256, 0, s>>>(d_part, splits, d_ref_sq, n_img, n_ref,
                                                           n_n, d_cand_d, d_cand_i);
   } else {
     k_dist_topk_bf16<Out::TOP8><<<grid, THREADS, SMEM_BYTES, s>>>(
         ma, mb, d_ref_sq, n_img, n_ref, n_pix, d_cand_d, d_cand_i, nullptr, nullptr, nullptr, 0,
-        group_m, err, 1);
+        group_m, err, 1, give_up);
   }
   return check_launch(name);
 }
@@ -1465,7 +1517,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
     for (int k = 0; k < TOPK; ++k) {
       const int32_t j = cand_i[off + k];
-      if (j == INT32_MAX) continue;
+      if (j < 0 || j == INT32_MAX) continue;
       ++valid;
       if (cand_d[off + k] <= T) {
         ++inband;
@@ -1835,7 +1887,7 @@ extern "C" int spf_match_bf16_static(const void *d_img_bf16, const float *d_img,
   int grid = (int)(gemm_tiles < sm_count() ? gemm_tiles : sm_count());
   k_dist_topk_bf16<Out::TOP8><<<grid, THREADS, SMEM_BYTES, s>>>(ma, mb, d_ref_sq, n_img, n_ref,
                                                             n_pix, cand_d, cand_i, nullptr,
-                                                            nullptr, nullptr, 0, GROUP_M, err, 1);
+                                                            nullptr, nullptr, 0, GROUP_M, err, 1, 0);
   SPF_TRY(check_launch("k_dist_topk_bf16 (static scratch)"));
   if (tune_get(SPF_TUNE_STATIC_ABORT_TEST, 0)) {
     k_static_inject_timeout<<<1, 32, 0, s>>>(err);

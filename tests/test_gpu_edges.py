@@ -578,3 +578,37 @@ def test_late_rerank_frames_are_left_open(n_pix):
     assert st["uncertified"] >= 4
     assert torch.equal(idx.to(want_i.dtype), want_i) and torch.equal(dist, want_d)
     matching.check_device_error()
+
+
+@pytest.mark.parametrize("n_img,n_ref,n_pix,divided", [
+    (9, 1500, 16384, True),    # parts of tiles
+    (9, 700, 1000, False),     # whole tiles, one CTA a frame in the re-rank
+    (2100, 40000, 64, False),  # several tiles a CTA, four frames a CTA
+])
+def test_gemm_that_gave_up_leaves_its_frames_open(n_img, n_ref, n_pix, divided):
+    """When a wait of the tensor-core GEMM runs out (the test switch: at each
+    CTA's last tile) the frames of the tiles left out are uncertified, whatever the
+    candidate buffers held before, and their completion is exact."""
+    from spinifel_gb300 import _lib, matching
+
+    fr, rs = _match_operands(n_img, n_ref, n_pix, 13)
+    size = int(_lib.lib().spf_dist_topk_bf16_work_bytes(n_img, n_ref, n_pix))
+    assert (size > 0) == divided
+    want_i, want_d = matching.argmin_fp32(fr.f32, rs.f32, images_sq=fr.sq, refs_sq=rs.sq)
+    first = {}
+    matching.match_bf16(fr, rs, stats=first)  # leaves its candidates in the buffers
+    _lib.call("spf_tune_set", _lib.SPF_TUNE_STATIC_ABORT_TEST, 1)
+    try:
+        st = {}
+        idx, dist = matching.match_bf16(fr, rs, stats=st)
+    finally:
+        _lib.call("spf_tune_set", _lib.SPF_TUNE_STATIC_ABORT_TEST, 0)
+    with pytest.raises(_lib.SpfError, match="gave up"):
+        matching.check_device_error()
+    # as many tiles as CTAs were left out (every one of the small calls)
+    tiles = int(_lib.lib().spf_dist_topk_bf16_tiles(n_ref)) * ((n_img + 127) // 128)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert st["uncertified"] == n_img or (tiles > sms and
+                                          st["uncertified"] > first["uncertified"])
+    assert torch.equal(idx.to(want_i.dtype), want_i) and torch.equal(dist, want_d)
+    matching.check_device_error()
