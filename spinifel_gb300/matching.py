@@ -297,44 +297,47 @@ class FrameSet:
         return out
 
 
-class _Workspace:
-    def __init__(self):
-        self.bufs = {}
-
-    def get(self, name, numel, dtype, device):
-        t = self.bufs.get((name, device))
-        if t is None or t.numel() < numel or t.dtype != dtype:
-            t = torch.empty(max(numel, 1), dtype=dtype, device=device)
-            self.bufs[(name, device)] = t
-        return t[:numel]
-
-
-_ws = _Workspace()
-
-
 def match_bf16(frames: FrameSet, refs: ReferenceSet, exact_fallback: bool = True,
                stats: dict | None = None, stream=None):
     """Best reference per frame: bf16 tensor-core distances, per-frame top-8,
     exact FP32 re-rank (bit-identical to the plain path's values); frames the
     certificate cannot settle are completed exactly from the kept per-tile
     candidate lists (spf_complete_open: list re-rank, and the range GEMM or
-    the plain pass only where those lists may hide references)."""
+    the plain pass only where those lists may hide references).  With `stream`
+    everything runs there; calls may overlap on several streams and threads."""
     if frames.n_pix != refs.n_pix or frames.ld != refs.ld:
         raise ValueError("frames and references differ in pixel count")
+    if stream is None:
+        return _match_bf16(frames, refs, exact_fallback, stats)
+    caller = torch.cuda.current_stream(frames.f32.device)
+    with torch.cuda.stream(stream):
+        out = _match_bf16(frames, refs, exact_fallback, stats)
+    for t in out:  # made on `stream`; the caller may go on to use them on its own
+        t.record_stream(caller)
+    return out
+
+
+def _match_bf16(frames: FrameSet, refs: ReferenceSet, exact_fallback: bool, stats):
+    """match_bf16 on the current stream.  The scratch belongs to the call: one
+    kept from call to call would be shared by calls in flight on other streams."""
     dev = frames.f32.device
     n_img = frames.n
     tiles = int(_lib.lib().spf_dist_topk_bf16_tiles(refs.n_ref))
-    cand_d = _ws.get("cand_d", tiles * n_img * 8, torch.float32, dev)
-    cand_i = _ws.get("cand_i", tiles * n_img * 8, torch.int32, dev)
-    mrg_d = _ws.get("merged_d", n_img * 8, torch.float32, dev)
-    mrg_i = _ws.get("merged_i", n_img * 8, torch.int32, dev)
-    work = _ws.get("rerank_work", n_img, torch.float32, dev)
+
+    def scratch(numel, dtype):  # never a NULL pointer
+        return torch.empty(max(numel, 1), dtype=dtype, device=dev)
+
+    cand_d = scratch(tiles * n_img * 8, torch.float32)
+    cand_i = scratch(tiles * n_img * 8, torch.int32)
+    mrg_d = scratch(n_img * 8, torch.float32)
+    mrg_i = scratch(n_img * 8, torch.int32)
+    work = scratch(n_img, torch.float32)
     idx = torch.empty(n_img, dtype=torch.int32, device=dev)
     dist = torch.empty(n_img, dtype=torch.float32, device=dev)
     unc = torch.empty(n_img, dtype=torch.int32, device=dev)
-    sh = _lib.stream_handle(stream)
+    sh = _lib.stream_handle()
     size = int(_lib.lib().spf_dist_topk_bf16_work_bytes(n_img, refs.n_ref, refs.n_pix))
-    part = _ws.get("parts", size, torch.uint8, dev) if size else None
+    part = scratch(size, torch.uint8) if size else None
     _lib.call("spf_dist_topk_bf16_work", _lib.ptr(frames.bf16), n_img, _lib.ptr(refs.bf16),
               refs.n_ref, refs.n_pix, refs.ld, _lib.ptr(refs.sq), _lib.ptr(cand_d),
               _lib.ptr(cand_i), _lib.ptr(part), size, sh)

@@ -612,3 +612,32 @@ def test_gemm_that_gave_up_leaves_its_frames_open(n_img, n_ref, n_pix, divided):
                                           st["uncertified"] > first["uncertified"])
     assert torch.equal(idx.to(want_i.dtype), want_i) and torch.equal(dist, want_d)
     matching.check_device_error()
+
+
+@pytest.mark.parametrize("n_ref", [1500, 200])
+def test_overlapping_matches_keep_their_scratch_apart(n_ref):
+    """match_bf16 calls in flight on several streams, from several threads,
+    give each its own answer (products of divided tiles among the scratch)."""
+    import threading
+
+    from spinifel_gb300 import matching
+
+    pairs = [_match_operands(n, n_ref, 16384, 20 + n) for n in (3, 5, 8, 13)]
+    want = [matching.match_bf16(fr, rs) for fr, rs in pairs]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in pairs]
+    got = [None] * len(pairs)
+
+    def work(k):
+        for _ in range(10):
+            got[k] = matching.match_bf16(*pairs[k], stream=streams[k])
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(pairs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for (i, d), (wi, wd) in zip(got, want):
+        assert torch.equal(i, wi) and torch.equal(d, wd)
+    matching.check_device_error()
