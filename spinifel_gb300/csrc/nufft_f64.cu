@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(128)
 constexpr int PAIR_MAX_W = 13;
 constexpr int PAIR_PX = 4, PAIR_PY = 8, PAIR_PIX = 32, PAIR_WARPS = 8;
 constexpr int PAIR_CELLS = 10240;    // 80 KB: two CTAs an SM
-constexpr int EXP_PER_UNIT = 32;     // exp(-j / 32) in the table
+constexpr int EXP_PER_UNIT = 128;    // exp(-j / 128) in the table
 
 struct Pair {
   float h, l;
@@ -221,30 +221,45 @@ __device__ __forceinline__ Pair add(Pair a, float b) {
   return fast_two_sum(s.h, __fadd_rn(s.l, a.l));
 }
 
-// sum of products: h + l; the terms' errors collect in l
+// sum of products: h + l; the terms' errors collect in l (a term's own first:
+// the large sum is rounded once a term)
 __device__ __forceinline__ void accumulate(Pair &acc, float wh, float wl, float gh, float gl) {
   const float p = __fmul_rn(wh, gh);
-  float l = __fadd_rn(acc.l, __fmaf_rn(wh, gh, -p));
-  l = __fmaf_rn(wh, gl, l);
-  l = __fmaf_rn(wl, gh, l);
+  const float e = __fmaf_rn(wl, gh, __fmaf_rn(wh, gl, __fmaf_rn(wh, gh, -p)));
   const Pair s = two_sum(acc.h, p);
   acc.h = s.h;
-  acc.l = __fadd_rn(l, s.l);
+  acc.l = __fadd_rn(acc.l, __fadd_rn(s.l, e));
 }
 
-// exp(beta (sqrt(1 - z^2) - 1)), z = (f + a) / half_w, by exp(x) = T[j] exp(t),
-// x = -j / 32 + t, and the Taylor polynomial of exp(t) - 1 (|t| <= 1/64)
-__device__ __forceinline__ Pair es_pair(Pair f, int a, Pair inv_half_w, Pair beta,
+// The kernel's constants: with u the distance in cells, z^2 = per_z2 u^2 and
+// beta z^2 = -expo u^2.
+struct PairKernel {
+  Pair per_z2, expo;
+};
+
+// exp(beta (sqrt(1 - z^2) - 1)) at u = f + a, good to about 2^-46 (sums of the
+// W values to 1e-14; the same operations replayed on the host, 4e5
+// fractions, W = 7, 10, 13).  The exponent is taken as
+// x = -beta z^2 / (1 + sqrt(1 - z^2)), which keeps its relative error where
+// sqrt - 1 cancels, and exp(x) = T[j] exp(t), x = -j / 128 + t, with the Taylor
+// polynomial of exp(t) - 1: for |t| <= 1/256 its cube is small enough to be
+// rounded to FP32 (with 32 entries a unit that rounding alone was 2^-42.2).
+__device__ __forceinline__ Pair es_pair(Pair f, int a, const PairKernel &k,
                                         const float2 *__restrict__ table, int table_last) {
-  const Pair z = mul(add(f, (float)a), inv_half_w);
-  const Pair z2 = mul(z, z);
+  const Pair u1 = add(f, (float)a);
+  const Pair u2 = mul(u1, u1);
+  const Pair z2 = mul(u2, k.per_z2), num = mul(u2, k.expo);
   Pair q = two_sum(1.0f, -z2.h);
   q = fast_two_sum(q.h, __fsub_rn(q.l, z2.l));
   if (!(q.h > 0.0f)) q = Pair{0.0f, 0.0f};
   const float root = __fsqrt_rn(q.h);
   const float rest = __fadd_rn(__fmaf_rn(-root, root, q.h), q.l);
-  const Pair r{root, root > 0.0f ? __fdividef(0.5f * rest, root) : 0.0f};
-  const Pair x = mul(add(r, -1.0f), beta);  // -beta .. 0
+  Pair d = two_sum(1.0f, root);  // 1 + the root
+  d = fast_two_sum(d.h, __fadd_rn(d.l, root > 0.0f ? __fdividef(0.5f * rest, root) : 0.0f));
+  const float inv = __fdividef(1.0f, d.h);
+  const float y = __fmul_rn(num.h, inv);
+  const float left = __fadd_rn(__fmaf_rn(-y, d.h, num.h), __fmaf_rn(-y, d.l, num.l));
+  const Pair x = fast_two_sum(y, __fmul_rn(left, inv));  // -beta .. 0
   const int j = min(max(__float2int_rn(-EXP_PER_UNIT * x.h), 0), table_last);
   const float2 T = __ldg(table + j);
   const Pair t = fast_two_sum(__fadd_rn(x.h, (float)j * (1.0f / EXP_PER_UNIT)), x.l);
@@ -293,8 +308,8 @@ template <int W>
 __global__ void __launch_bounds__(PAIR_WARPS * 32, 2)
     k_slice_pairs(const float2 *__restrict__ grid, const unsigned long long *__restrict__ peak,
                   Geom g, const double *__restrict__ quats, const double *__restrict__ ppr,
-                  int n_panels, int nx, int ny, double s1, double s2, double s3, Pair inv_half_w,
-                  Pair beta, const float2 *__restrict__ exp_table, int table_last,
+                  int n_panels, int nx, int ny, double s1, double s2, double s3, PairKernel kernel,
+                  const float2 *__restrict__ exp_table, int table_last,
                   double *__restrict__ out) {
   extern __shared__ __align__(16) float2 box[];  // PAIR_CELLS
   __shared__ float2 wts[3 * W][PAIR_PIX];
@@ -371,7 +386,7 @@ __global__ void __launch_bounds__(PAIR_WARPS * 32, 2)
   // warp a row, took most of the kernel: 1,297 us in all)
   for (int e = warp; e < 3 * W; e += PAIR_WARPS) {
     const float2 f = frac[e / W][lane];
-    const Pair w = es_pair(Pair{f.x, f.y}, e % W, inv_half_w, beta, exp_table, table_last);
+    const Pair w = es_pair(Pair{f.x, f.y}, e % W, kernel, exp_table, table_last);
     wts[e][lane] = make_float2(w.h, w.l);
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
@@ -725,14 +740,15 @@ int spf_slice_t2_f64_det(spf_nufft64_plan P, const double *d_quats, int64_t n_or
   grid_scales(P, scale, sc);
   const dim3 grid((unsigned)n_orient, (unsigned)patches);
   const int smem = PAIR_CELLS * (int)sizeof(float2);
-  const Pair ihw = pair_of(2.0 / P->w), beta = pair_of(P->beta);
+  const double per_z2 = 4.0 / ((double)P->w * P->w);
+  const PairKernel kernel{pair_of(per_z2), pair_of(-P->beta * per_z2)};
   const int last = (int)ceil(EXP_PER_UNIT * P->beta) + 1;
 #define SPF_PAIR_CASE(w_)                                                                        \
   case w_:                                                                                       \
     cudaFuncSetAttribute(k_slice_pairs<w_>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);  \
     k_slice_pairs<w_><<<grid, PAIR_WARPS * 32, smem, s>>>(                                       \
-        P->pair_pad, P->peak, g, d_quats, d_ppr, n_panels, nx, ny, sc[0], sc[1], sc[2], ihw,     \
-        beta, P->exp_table, last, d_out);                                                        \
+        P->pair_pad, P->peak, g, d_quats, d_ppr, n_panels, nx, ny, sc[0], sc[1], sc[2], kernel,  \
+        P->exp_table, last, d_out);                                                        \
     break;
   switch (P->w) {
     SPF_PAIR_CASE(2)

@@ -319,6 +319,29 @@ def test_fp64_slices_by_pairs(eps, M, det, n):
         assert e[1] <= 1.1 * e[0] + 1e-14
 
 
+@pytest.mark.parametrize("eps", [1e-6, 1e-9, 1e-12])
+def test_fp64_slices_by_pairs_kernel_values(eps):
+    """Every pixel of a slice of a flat grid (one mode), which is the product of the
+    three axes' sums of kernel values: pairs against the FP64 kernel to 6e-14
+    (three axes of 1.1e-14, the largest error of a sum of pair values, and
+    2^-46 for the sums over the footprint)."""
+    from spinifel_gb300 import geom
+    from spinifel_gb300.nufft import NufftPlan64
+
+    rng = np.random.default_rng(21)
+    M, det = 21, (4, 64, 64)
+    ppr, pdr = geom.flat_detector(*det)
+    q = geom.uniform_quaternions(16, rng)
+    P = NufftPlan64(M, eps)
+    f = np.zeros((M, M, M))
+    f[M // 2, M // 2, M // 2] = 1.0
+    P.set_modes(torch.as_tensor(f, device="cuda"))
+    p = torch.as_tensor(ppr.reshape(3, -1), device="cuda")
+    flat = P.slice(q, p, np.pi / pdr.max())
+    pair = P.slice(q, p, np.pi / pdr.max(), det_shape=det)
+    assert float(((pair - flat) / flat).abs().max()) < 6e-14
+
+
 @pytest.mark.parametrize("bad", [0.0, 1e-310, float("inf"), float("nan")])
 def test_fp64_slices_of_grids_pairs_cannot_hold(bad):
     """Zero, subnormal, infinite and NaN models take the FP64 kernel."""
