@@ -154,11 +154,11 @@ __global__ void k_best64_init(double *best_dist, int64_t *best_idx, int64_t n) {
 }
 
 // Sum of squares per row, rounded to FP32, by one warp a row (W = 1) or one
-// CTA of W warps.  Each thread keeps its sum as an unevaluated pair of floats
-// (error-free product and sum: Dekker 1971, Knuth TAOCP 2, 4.2.2), good to
-// about 2^-40 of it, and the pairs are added in FP64.  FP64 in the loop (a
+// CTA of W warps.  Each thread keeps its sum as three unevaluated floats
+// (error-free products and sums: Dekker 1971, Knuth TAOCP 2, 4.2.2), which loses
+// less than FP64 does, and the parts are added in FP64.  FP64 in the loop (a
 // conversion and an FMA an element) runs at this chip's FP64 rate: 8,000 rows
-// of 16,384 pixels took 530 us, 107 us now.  A row whose sum overflows FP32 or
+// of 16,384 pixels took 530 us, 113 us now.  A row whose sum overflows FP32 or
 // is so small that squares are lost to underflow is summed in FP64.
 template <int W>
 __global__ void __launch_bounds__(256) k_row_sqnorm(const float *__restrict__ x, int64_t n_rows,
@@ -182,12 +182,18 @@ __global__ void __launch_bounds__(256) k_row_sqnorm(const float *__restrict__ x,
   const int64_t step = (int64_t)gridDim.x * RPB;
   for (int64_t r = (int64_t)blockIdx.x * RPB + threadIdx.x / T; r < n_rows; r += step) {
     const float *p = x + r * n_pix;
-    float s = 0.0f, c = 0.0f;
+    float s = 0.0f, c = 0.0f, l = 0.0f;  // the sum, its errors, their errors
+    auto exact_add = [](float &to, float v) {  // returns what the rounding lost
+      const float u = __fadd_rn(to, v), z = __fsub_rn(u, to);
+      const float lost = __fadd_rn(__fsub_rn(to, __fsub_rn(u, z)), __fsub_rn(v, z));
+      to = u;
+      return lost;
+    };
     auto add = [&](float v) {
       const float q = __fmul_rn(v, v), e = __fmaf_rn(v, v, -q);
-      const float u = __fadd_rn(s, q), z = __fsub_rn(u, s);
-      c = __fadd_rn(c, __fadd_rn(__fadd_rn(__fsub_rn(s, __fsub_rn(u, z)), __fsub_rn(q, z)), e));
-      s = u;
+      const float d = exact_add(s, q);
+      l = __fadd_rn(l, exact_add(c, d));
+      l = __fadd_rn(l, exact_add(c, e));
     };
     if (vec) {
       const float4 *p4 = reinterpret_cast<const float4 *>(p);
@@ -216,7 +222,7 @@ __global__ void __launch_bounds__(256) k_row_sqnorm(const float *__restrict__ x,
         for (int u = 0; u < U; ++u) add(v[u]);
       }
     }
-    double sum = row_sum((double)s + (double)c);
+    double sum = row_sum((double)s + ((double)c + (double)l));
     if (!(sum > 1e-24 && sum < 3e38)) {  // the same for all threads of the row
       double d = 0.0;
       for (int64_t k = t; k < n_pix; k += T) d = fma((double)p[k], (double)p[k], d);

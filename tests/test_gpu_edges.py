@@ -75,6 +75,23 @@ def test_row_sqnorm_is_the_rounded_sum(n_pix, scale):
                                atol=2 ** -149)
 
 
+@pytest.mark.parametrize("n_pix,step", [(1024, 1), (1001, 32), (8192, 1), (8001, 256)])
+def test_row_sqnorm_near_ties(n_pix, step):
+    """Rows whose sum lies 2^-52 of itself past the middle between two floats,
+    in elements that one thread adds up: as the rounded FP64 sum, which is exact."""
+    from spinifel_gb300 import matching
+
+    x = np.zeros((3, n_pix), dtype=np.float32)
+    for r, first in enumerate((2.0 ** 12, 2.0 ** 20, 2.0 ** -8)):  # 2^2k + 2^(2k - 24)
+        x[r, 0] = first
+        x[r, step] = first * 2.0 ** -12
+        x[r, 2 * step] = first * 2.0 ** -26
+    got = matching.row_sqnorm(torch.as_tensor(x, device="cuda")).cpu().numpy()
+    want = (x.astype(np.float64) ** 2).sum(axis=1).astype(np.float32)
+    assert (want > x[:, 0].astype(np.float64) ** 2).all()
+    np.testing.assert_array_equal(got, want)
+
+
 @pytest.mark.parametrize("n_img,n_ref,n_pix", [(1, 1, 1), (31, 33, 17), (64, 64, 16), (65, 129, 63),
                                                (128, 128, 64), (129, 2000, 100), (700, 1300, 37),
                                                (1500, 1400, 48), (33, 5000, 130)])
