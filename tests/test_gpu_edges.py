@@ -681,3 +681,26 @@ def test_overlapping_matches_keep_their_scratch_apart(n_ref):
     for (i, d), (wi, wd) in zip(got, want):
         assert torch.equal(i, wi) and torch.equal(d, wd)
     matching.check_device_error()
+
+
+def test_argmin_fp64_of_very_many_references():
+    """More references than a launch has rows of blocks (65,535 x 512), with a frame
+    that is compared with all of them: the FP64 minimum, lowest index on ties."""
+    from spinifel_gb300 import _lib, matching
+
+    n_ref = 65535 * 512 + 7
+    g = torch.Generator(device="cuda").manual_seed(3)
+    refs = torch.rand(n_ref, 1, dtype=torch.float64, device="cuda", generator=g)
+    img = torch.tensor([[0.5], [2.0 ** 51]], dtype=torch.float64, device="cuda")
+    refs[-1, 0] = 1.5 + 2.0 ** -3  # the large frame's nearest, in the last block
+    size = int(_lib.lib().spf_argmin_f64_work_bytes(2, n_ref, 1))
+    ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+    t = matching.BestTracker64(2, img.device)
+    _lib.call("spf_argmin_f64", _lib.ptr(img), 2, _lib.ptr(refs), n_ref, 1, 0, _lib.ptr(ws), size,
+              _lib.ptr(t.best_dist), _lib.ptr(t.best_idx), _lib.stream_handle())
+    idx, dist = t.result()
+    for i in range(2):
+        d = (img[i, 0] - refs[:, 0]) ** 2
+        m = d.min()
+        assert float(dist[i]) == float(m)
+        assert int(idx[i]) == int(torch.nonzero(d == m)[0, 0])
