@@ -1005,7 +1005,8 @@ __device__ __forceinline__ int cell_in_bin(float t, int off, int b0) {
 template <int W>
 __global__ void __launch_bounds__(256)
     k_item_cellsort(GridGeom g, BinDims bd, const int4 *__restrict__ items,
-                    const int32_t *__restrict__ n_items, float4 *__restrict__ sorted, int chunk) {
+                    const int32_t *__restrict__ n_items, float4 *__restrict__ sorted, int chunk,
+                    unsigned int *__restrict__ err) {
   constexpr int NC = BIN * BIN * BIN;
   extern __shared__ __align__(16) unsigned char cs_smem[];
   float4 *pt = reinterpret_cast<float4 *>(cs_smem);
@@ -1013,6 +1014,10 @@ __global__ void __launch_bounds__(256)
   __shared__ int32_t cnt[NC];
   if ((int)blockIdx.x >= *n_items) return;
   const int4 it = items[blockIdx.x];
+  if (it.z > chunk) {  // an item larger than the staging arrays is never read
+    if (threadIdx.x == 0 && err) atomicExch(err, (unsigned int)(-SPF_ERR_ARG));
+    return;
+  }
   const int b = it.x;
   const int bi = b / (bd.nb[1] * bd.nb[2]), bj = (b / bd.nb[2]) % bd.nb[1], bk = b % bd.nb[2];
   for (int t = threadIdx.x; t < NC; t += blockDim.x) cnt[t] = 0;
@@ -1885,7 +1890,8 @@ static int sort_points(spf_nufft_plan P, PointSrc src, int64_t n, double scale, 
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)(CELLSORT_POINT * BIN_CHUNK_MAX)),
                         k_item_cellsort<W><<<(unsigned)max_items, 256, smem, s>>>(
-                            g, bd, P->items, totals + 1, P->sorted, chunk)));
+                            g, bd, P->items, totals + 1, P->sorted, chunk,
+                            device_error_word())));
   SPF_TRY(check_launch("k_item_cellsort"));
   P->n_sorted = n;
   return check_cuda(cudaEventRecord(P->sorted_use, s), "spf_nufft_sort");
