@@ -113,10 +113,12 @@ __global__ void k_fold_padded(const T *__restrict__ acc, GridDims g, T *__restri
   if (row >= (int64_t)g.n1 * g.n2) return;
   const int i0 = wrap((int)(row / g.n2) + g.off1, g.n1), j0 = wrap((int)(row % g.n2) + g.off2, g.n2);
   T *dst = grid + row * g.n3;
-  if (i0 + g.n1 >= g.p1 && j0 + g.n2 >= g.p2 && g.off3 + 2 * g.n3 > g.p3) {
+  if (i0 + g.n1 >= g.p1 && j0 + g.n2 >= g.p2 && g.off3 + g.n3 >= g.p3 &&
+      g.off3 <= g.n3) {
     // one row of the accumulator (all but the halo's): a cell is its cells k -
-    // n3 and k = c + off3, four cells' loads in flight (98 us for 320^3 cells
-    // through the loops below)
+    // n3 and k = c + off3 (the conditions on n3, which every but the smallest
+    // grid meets: k + n3 is past the row for all c, and k - 2 n3 before it),
+    // four cells' loads in flight (98 us for 320^3 cells through the loops below)
     const T *r = acc + ((int64_t)i0 * g.p2 + j0) * g.p3;
 #pragma unroll 4
     for (int c = threadIdx.x; c < g.n3; c += 32) {

@@ -704,3 +704,24 @@ def test_argmin_fp64_of_very_many_references():
         m = d.min()
         assert float(dist[i]) == float(m)
         assert int(idx[i]) == int(torch.nonzero(d == m)[0, 0])
+
+
+@pytest.mark.parametrize("eps", [1e-1, 1e-2, 1e-3, 1e-4, 1e-5, 1e-6, 1e-9])
+def test_type1_of_the_smallest_grids(eps):
+    """Grids of twice the kernel's width, whose halo wraps onto itself: type 1
+    against the direct sums (20 eps, and 1e-5 for FP32)."""
+    from oracle import nufft as onufft
+    from spinifel_gb300.nufft import make_plan
+
+    rng = np.random.default_rng(31)
+    x, y, z = rng.uniform(-3, 3, (3, 500)).astype(np.float32)
+    c = rng.random(500).astype(np.float32)
+    dev = [torch.as_tensor(v, device="cuda") for v in (x, y, z, c)]
+    for m in ((1, 1, 1), (2, 3, 4), (4, 1, 7), (5, 6, 2)):
+        P = make_plan(m, eps)
+        P.spread_zero()
+        P.spread(*dev)
+        re, im = P.finish(+1, want_imag=True)
+        got = re.cpu().numpy() + 1j * im.cpu().numpy()
+        want = onufft.nudft3d1(x, y, z, c, m, +1)
+        assert np.linalg.norm(got - want) < max(20 * eps, 1e-5) * np.linalg.norm(want)
