@@ -38,8 +38,8 @@ struct spf_nufft64_plan_s {
   double *re_pad = nullptr;
   double *im_pad = nullptr;
   double *acc_pad = nullptr;
-  // slicing by pairs of floats (w <= PAIR_MAX_W): the padded grid over a power
-  // of two as (high, low) pairs, that power, exp at the table's points
+  // slicing by pairs of floats (NULL: in FP64): the padded grid over a power of
+  // two as (high, low) pairs, that power, exp at the table's points
   float2 *pair_pad = nullptr;
   unsigned long long *peak = nullptr;  // bits of max |re_pad|
   float2 *exp_table = nullptr;
@@ -539,7 +539,8 @@ static Pair pair_of(double v) {
 
 // The float-pair grid, its peak and the table of exponentials in one
 // allocation, made with the plan (setting a model then allocates nothing and
-// can be captured).
+// can be captured).  Where there is no memory for it the plan does without, and
+// slices in FP64.
 static int alloc_pairs(spf_nufft64_plan P) {
   const size_t npad = (size_t)P->np[0] * P->np[1] * P->np[2];
   const int n = (int)ceil(EXP_PER_UNIT * P->beta) + 2;
@@ -548,7 +549,11 @@ static int alloc_pairs(spf_nufft64_plan P) {
     const Pair p = pair_of(exp(-(double)j / EXP_PER_UNIT));
     t[j] = make_float2(p.h, p.l);
   }
-  SPF_TRY(check_cuda(cudaMalloc(&P->pair_pad, (npad + n + 1) * sizeof(float2)), "plan64_create"));
+  if (cudaMalloc(&P->pair_pad, (npad + n + 1) * sizeof(float2)) != cudaSuccess) {
+    cudaGetLastError();
+    P->pair_pad = nullptr;
+    return SPF_OK;
+  }
   P->exp_table = P->pair_pad + npad;
   P->peak = reinterpret_cast<unsigned long long *>(P->exp_table + n);
   return check_cuda(cudaMemcpy(P->exp_table, t.data(), n * sizeof(float2), cudaMemcpyHostToDevice),
@@ -597,7 +602,6 @@ int spf_nufft64_plan_create(int m1, int m2, int m3, double eps, double upsampfac
                                              (P->n[2] / 2 + 1) * sizeof(double2)), "plan64_create");
   if (st == SPF_OK) P->half = reinterpret_cast<double2 *>(P->fine + nfine);
   if (st == SPF_OK) st = check_cuda(cudaMalloc(&P->re_pad, npad * sizeof(double)), "plan64_create");
-  if (st == SPF_OK && P->w <= PAIR_MAX_W) st = alloc_pairs(P);
   if (st == SPF_OK) {
     cufftResult r = cufftPlan3d(&P->fft, P->n[0], P->n[1], P->n[2], CUFFT_D2Z);
     if (r != CUFFT_SUCCESS) {
@@ -608,6 +612,7 @@ int spf_nufft64_plan_create(int m1, int m2, int m3, double eps, double upsampfac
       P->fft_ok = true;
     }
   }
+  if (st == SPF_OK && P->w <= PAIR_MAX_W) st = alloc_pairs(P);
   if (st != SPF_OK) {
     spf_nufft64_plan_destroy(P);
     return st;
@@ -676,7 +681,7 @@ int spf_nufft64_t2_set_modes(spf_nufft64_plan P, const double *d_modes, const do
       P->half, g, isign < 0 ? double(1) : double(-1), P->re_pad,
       want_imag ? P->im_pad : nullptr, nullptr);
   SPF_TRY(check_launch("k_spectrum_to_padded"));
-  return P->w <= PAIR_MAX_W ? make_pairs(P, s) : SPF_OK;
+  return P->pair_pad ? make_pairs(P, s) : SPF_OK;
 }
 
 int spf_nufft64_t2_interp(spf_nufft64_plan P, const double *d_x, const double *d_y,
@@ -729,7 +734,7 @@ int spf_slice_t2_f64_det(spf_nufft64_plan P, const double *d_quats, int64_t n_or
   const int64_t patches =
       (int64_t)n_panels * ((nx + PAIR_PX - 1) / PAIR_PX) * ((ny + PAIR_PY - 1) / PAIR_PY);
   const int64_t n_pix = (int64_t)n_panels * nx * ny;
-  if (P->w > PAIR_MAX_W || patches > 65535)
+  if (!P->pair_pad || patches > 65535)
     return spf_slice_t2_f64(P, d_quats, n_orient, d_ppr, n_pix, scale, d_out, stream);
   SPF_REQUIRE(d_quats && d_ppr && d_out, "spf_slice_t2_f64_det: NULL pointer");
   SPF_REQUIRE(n_orient < (1LL << 31) && n_pix <= 65535LL * 128,
