@@ -195,14 +195,16 @@ class NufftPlan:
                       _lib.stream_handle())
 
     def sort_points(self, x, y, z):
-        """Bin-sort explicit points (radians) once for spread_sorted; the
-        coordinate tensors are kept alive by the plan."""
+        """Bin-sort explicit points (radians) once for spread_sorted; the plan
+        keeps the sorted points (16 bytes each), not the coordinate tensors."""
         x, y, z = (t.to(device=self.device, dtype=torch.float32).contiguous().reshape(-1)
                    for t in (x, y, z))
         with self._sort_lock:
-            self._sorted_points = (x, y, z)
             _lib.call("spf_nufft_sort_points", self._h, _lib.ptr(x), _lib.ptr(y), _lib.ptr(z),
                       x.numel(), _lib.stream_handle())
+            self._sorted_points = ()
+        for v in (x, y, z):  # may belong to another stream, and be dropped before they are read
+            v.record_stream(torch.cuda.current_stream())
 
     def spread_sorted(self, c=None):
         """Type-1 spreading of c (or ones) over the points of the last sort

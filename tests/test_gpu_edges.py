@@ -725,3 +725,29 @@ def test_type1_of_the_smallest_grids(eps):
         got = re.cpu().numpy() + 1j * im.cpu().numpy()
         want = onufft.nudft3d1(x, y, z, c, m, +1)
         assert np.linalg.norm(got - want) < max(20 * eps, 1e-5) * np.linalg.norm(want)
+
+
+def test_plans_do_not_keep_explicit_coordinates():
+    """After sort_points the plan has the points itself: the coordinate tensors
+    may go, and the passes over the sorted points are as before."""
+    import weakref
+
+    from spinifel_gb300.nufft import NufftPlan
+
+    rng = np.random.default_rng(33)
+    P = NufftPlan(21, 1e-6)
+    pts = [torch.as_tensor(rng.uniform(-3, 3, 5000).astype(np.float32), device="cuda")
+           for _ in range(3)]
+    P.spread_zero()
+    P.spread(*pts, torch.ones(5000, device="cuda"))
+    want = P.finish(+1)[0]
+    P.sort_points(*pts)
+    gone = [weakref.ref(v) for v in pts]
+    pts.clear()
+    assert all(r() is None for r in gone)
+    junk = [torch.full((5000,), 7.0, device="cuda") for _ in range(6)]
+    P.spread_zero()
+    P.spread_sorted()
+    got = P.finish(+1)[0]
+    assert float((got - want).norm() / want.norm()) < 1e-5
+    del junk
