@@ -29,6 +29,9 @@ import torch
 from . import _lib
 
 HERE = os.path.dirname(os.path.abspath(__file__))
+# part of every cache key; changes when a tuned kernel or the meaning of a
+# choice does, so that choices timed against other kernels are not taken
+KERNELS = 2
 _lock = threading.Lock()
 
 
@@ -59,9 +62,12 @@ def _bucket(n: int) -> int:
     return 1 << max(0, int(math.ceil(math.log2(max(n, 1)))))
 
 
+def _name() -> str:
+    return f"{torch.cuda.get_device_name()}|kernels {KERNELS}"
+
+
 def _key(kind, n_img, n_ref, n_pix):
-    name = torch.cuda.get_device_name()
-    return f"{name}|{kind}|{_bucket(n_img)}|{_bucket(n_ref)}|{n_pix}"
+    return f"{_name()}|{kind}|{_bucket(n_img)}|{_bucket(n_ref)}|{n_pix}"
 
 
 def _time(fn, reps):
@@ -144,7 +150,10 @@ def tune_fp32(frames_f32, frames_sq, refs, group_sizes=(4, 8, 16), reps=1, force
         return dict(rec, cached=False)
 
 
-SLICE_SHAPES = {0: "16x16 patch, 4x8 warps", 1: "16x16 patch, 8x4 warps",
+# code 0 is no shape but the kernel's own rule; the others hold for every
+# detector and grid of the process until the code is set back
+SLICE_SHAPES = {0: "by the pixels' spacing: 8x16 patch, 4x8 warps (with stride search from "
+                   "0.5 cells), or shape 6 from 2.2 cells", 1: "16x16 patch, 8x4 warps",
                 2: "8x32 patch, 2x16 warps", 3: "8x32 patch, 4x8 warps",
                 4: "32x8 patch, 8x4 warps", 5: "32x8 patch, 16x2 warps",
                 6: "16x16 patch, 4x8 warps, stride search",
@@ -155,8 +164,7 @@ def tune_slice(plan, quats, ppr, scale: float, det_shape, reps=2, force=False):
     """Pick SPF_TUNE_SLICE_SHAPE for spf_slice_t2_det on this model grid and
     detector (quats: the orientations to time on, a few thousand suffice);
     returns {"shape", "tile", "ms", "trials"}."""
-    name = torch.cuda.get_device_name()
-    key = f"{name}|slice|{plan.n_fine}|w{plan.width}|{tuple(det_shape)}"
+    key = f"{_name()}|slice|{plan.n_fine}|w{plan.width}|{tuple(det_shape)}"
     with _lock:
         cache = _load()
         if not force and key in cache:
@@ -183,8 +191,7 @@ def tune_sort_item(plan, sort_fn, pass_fn, sizes=(2048, 4096, 8192), reps=2,
     passes): for each size sort_fn() re-sorts the points and pass_fn() is
     timed; the best size is set and the points re-sorted with it.  Returns
     {"items", "ms", "trials"}."""
-    name = torch.cuda.get_device_name()
-    key = f"{name}|sort_item|{plan.n_fine}|w{plan.width}|{tag}"
+    key = f"{_name()}|sort_item|{plan.n_fine}|w{plan.width}|{tag}"
     with _lock:
         cache = _load()
         if not force and key in cache:

@@ -238,3 +238,31 @@ def test_spread_orient_dispatch_by_size(monkeypatch):
     assert run(2, n_pix, (4, 32, 32)) == ["spf_nufft_t1_spread_det"]
     assert run(2, n_pix) == ["spf_nufft_t1_spread_orient"]
     assert run(2, n_pix, sort=True) == ["spf_nufft_sort_orient", "spf_nufft_spread_sorted"]
+
+
+def test_slice_tuner_names_what_runs(monkeypatch, tmp_path):
+    """The tuner's code 0 is named as the kernel's own rule, and a choice cached for
+    other kernels (a key without their version) is not taken."""
+    import json
+
+    import torch
+
+    from spinifel_gb300 import _lib, autotune
+
+    cache = tmp_path / "tuned.json"
+    monkeypatch.setenv("SPF_TUNE_CACHE", str(cache))
+    monkeypatch.setattr(torch.cuda, "get_device_name", lambda *a: "GPU")
+    monkeypatch.setattr(_lib, "call", lambda *a: None)
+    times = iter(range(100))
+    monkeypatch.setattr(autotune, "_time", lambda fn, reps: float(next(times)))
+
+    class Plan:
+        n_fine, width = (90, 90, 90), 7
+
+    det = (4, 8, 8)
+    cache.write_text(json.dumps({f"GPU|slice|{Plan.n_fine}|w7|{det}":
+                                 {"shape": 3, "tile": "8x32 patch, 4x8 warps", "ms": 1.0}}))
+    args = (Plan(), torch.zeros(2, 4), torch.zeros(3, 256), 1.0, det)
+    best = autotune.tune_slice(*args)
+    assert not best["cached"] and best["shape"] == 0 and "spacing" in best["tile"]
+    assert autotune.tune_slice(*args)["cached"]
