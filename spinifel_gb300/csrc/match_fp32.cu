@@ -479,7 +479,12 @@ using namespace spf;
 template <typename T>
 static int launch_eudist(const T *ref, const T *data, int64_t n_ref, int64_t n_data,
                          int64_t n_pix, int64_t K, T *out, void *stream, const char *name) {
-  const int pairs = pick_tile(n_data, n_ref, 0.9, 0.6);
+  // FP64 tiles are all bound by the FP64 pipe and run at one rate: at the FP32
+  // rates 64 x 20,000 pairs of 512 pixels took 64-pair tiles and 3.37 ms (32-pair
+  // ones 2.81), 640 x 640 x 1,000 2.24 (1.70), 2,000 x 8,000 x 256 128-pair ones
+  // and 15.7 (14.5)
+  const bool fp64 = sizeof(T) == 8;
+  const int pairs = pick_tile(n_data, n_ref, fp64 ? 1.0 : 0.9, fp64 ? 1.0 : 0.6);
   const int64_t tiles = tile_count(n_data, n_ref, pairs);
   SPF_REQUIRE(tiles < (1LL << 31), "%s: too many tiles", name);
   const int group_m = (int)tune_get(SPF_TUNE_FP32_GROUP_M, GROUP_M);

@@ -250,8 +250,9 @@ __device__ __forceinline__ void tile_sums(const T *__restrict__ A, int64_t n_a,
 // (128: 54, 64: 47, 32: 30 TFLOP/s).  The 128-pair tile reads shared memory
 // least per operation; with few tiles most of the chip would idle under it:
 // 333 x 1,999 x 5,550 takes 608 us there and 342 us with 32-pair tiles,
-// 500 x 2,000 x 4,096 takes 436 us and, with 64-pair tiles, 266 us (FP64:
-// 35.9 and 17.8 ms); 1,500 x 8,000 x 8,192 takes 3.65 ms there, 4.2 ms with 64.
+// 500 x 2,000 x 4,096 takes 436 us and, with 64-pair tiles, 266 us (FP64,
+// whose tiles have one rate: 35.9 and 17.8 ms); 1,500 x 8,000 x 8,192 takes
+// 3.65 ms there, 4.2 ms with 64.
 template <int PAIRS>
 inline double tile_cost(int64_t n_a, int64_t n_b, double rate) {
   const int64_t t = ((n_a + PAIRS - 1) / PAIRS) * ((n_b + PAIRS - 1) / PAIRS);

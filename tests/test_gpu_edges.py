@@ -751,3 +751,20 @@ def test_plans_do_not_keep_explicit_coordinates():
     got = P.finish(+1)[0]
     assert float((got - want).norm() / want.norm()) < 1e-5
     del junk
+
+
+@pytest.mark.parametrize("n_data,n_ref", [(64, 20000), (640, 640), (2000, 8000), (129, 127)])
+def test_fp64_distances_where_the_tile_changed(n_data, n_ref):
+    """FP64 distance blocks of sizes that take other tiles than FP32 blocks of
+    theirs, on reals (to the rounding of seven terms) and on integers (exactly)."""
+    from spinifel_gb300 import matching
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.rand(n_data, 7, dtype=torch.float64, device="cuda", generator=g)
+    r = torch.rand(n_ref, 7, dtype=torch.float64, device="cuda", generator=g)
+    got = matching.dist_f64(r, x).reshape(n_data, n_ref)
+    want = ((x[:, None, :] - r[None, :, :]) ** 2).sum(2)
+    assert float((got - want).abs().max()) < 8 * 2 ** -52 * 7
+    xi, ri = (x * 100).round(), (r * 100).round()
+    got = matching.dist_f64(ri, xi).reshape(n_data, n_ref)
+    assert torch.equal(got, ((xi[:, None, :] - ri[None, :, :]) ** 2).sum(2))
