@@ -82,7 +82,9 @@ def argmin_fp32(images: torch.Tensor, refs: torch.Tensor, images_sq=None, refs_s
     return t.result()
 
 
-# below this many pixels the whole FP64 block is as quick as picking minima
+# from this many pixels on, update_fp64 picks minima (500 x 2,000 pairs of 64
+# pixels: 91 us, 339 as a block; 20 x 100: 72 and 118); below, the whole block is
+# little work (500 x 2,000 pairs of 16 pixels: 126 us)
 MINIMA_MIN_PIXELS = 64
 
 
