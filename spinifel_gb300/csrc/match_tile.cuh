@@ -20,7 +20,8 @@ enum class Mode { DIFF, DOT };
 // has two warps, and with few of them on an SM nothing else hides a step's
 // loads (32 x 8,000 pairs of 16,384 pixels: 623 us with one step, 525 with
 // four).  MINB CTAs an SM are asked of the compiler for the 128-pair tile's
-// argmin (54.0 TFLOP/s against 49.3 with one).
+// argmin (54.0 TFLOP/s against 49.3 with one; its bound of 128 registers then
+// spills 124 bytes a thread, which that rate includes).
 template <int TM_, int TN_, int RM_, int RN_, int PF_>
 struct Tile {
   static constexpr int TM = TM_, TN = TN_, RM = RM_, RN = RN_, PF = PF_;

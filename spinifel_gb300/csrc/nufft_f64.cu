@@ -14,7 +14,8 @@
 //
 // GB300 runs FP64 at about 1/64 of its FP32 rate, so the FP64 kernels are
 // bound by the FP64 pipe (W^3 FMAs per point); the grid (tens of MB) stays
-// in L2 and is read through L1 without shared-memory staging.
+// in L2 and is read through L1 without shared-memory staging.  Slices of panel
+// detectors run over pairs of floats instead (k_slice_pairs).
 #include <cufft.h>
 #include <math.h>
 
@@ -180,11 +181,13 @@ __global__ void __launch_bounds__(128)
 // eps 1e-12, about as dear as 1,500 FMAs) take 2.66 ms for 409,600 points.
 // The same sums over unevaluated pairs of floats (error-free products and
 // sums: Dekker 1971, Knuth TAOCP 2, 4.2.2) take twelve FP32 instructions a
-// term and are good to about 2^-46 of the terms' magnitudes, far below the
-// interpolation error of a kernel of W <= 13 (4.8e-13 against the direct sums
-// at W = 13, before and now); wider kernels resolve less than that and stay
-// in FP64.  409,600 points at 41^3 take 0.83 ms (2.69 in FP64 throughout),
-// 262,144 at 81^3 on 4 x 128 x 128 pixels 0.53 (1.72).
+// term and are good to about 2^-46 of the terms' magnitudes: a pixel is at most
+// 3.2e-14 of the largest value off the FP64 kernel's, where the interpolation of
+// a kernel of W <= 13 is off by 5e-13 and more (against the direct sums, FP64 and
+// pairs: 8.3778e-13 and 8.3786e-13 at 21^3, 2.3936e-12 and 2.3927e-12 at 41^3);
+// wider kernels resolve less than that and stay in FP64.  409,600 points at 41^3
+// take 0.85 ms (2.69 in FP64 throughout), 262,144 at 81^3 on 4 x 128 x 128
+// pixels 0.54 (1.72).
 //
 // A CTA takes a 4 x 8 pixel patch of one panel at one orientation: three
 // warps compute its grid coordinates in FP64 (one axis each), all eight the
