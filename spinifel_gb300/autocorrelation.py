@@ -84,8 +84,9 @@ def forward(ugrid, H_, K_, L_, support, use_recip_sym, N, eps=DEFAULT_EPS):
 # from this many points on, the adjoint bin-sorts them once and spreads with
 # the sorted kernel (a pencil's cells summed in registers) instead of one
 # thread per point with global atomics.  Whole adjoint, sorted / per point:
-# 517 / 530 us at 65,536 points on the 81^3 grid (1,108 / 1,072 at 151^3),
-# 489 / 1,015 at 409,600 (41^3), 703 / 3,423 at 2,048,000.
+# 517 / 530 us at 65,536 points on the 81^3 grid, 489 / 1,015 at 409,600 (41^3),
+# 703 / 3,423 at 2,048,000; on grids with few points a bin
+# NufftPlan.SORTED_MIN_PER_BIN decides.
 SORTED_SPREAD_MIN_POINTS = 1 << 17
 
 

@@ -145,17 +145,27 @@ class NufftPlan:
     # over them would read the others.  From here on (2.0e6 points: 3.4 ms one
     # by one, 0.7 sorted) it sorts whatever the plan holds.
     KEEP_SORT_POINTS = 1 << 21
+    # points a bin (8^3 cells) from which the sort and its pass pay: below, most
+    # bins are an item of a few points with a box of its own.  Sorted / unsorted, us:
+    # spread_orient at 0.5 a bin (262,144 points on 640^3) 1,586 / 694, 2.3 955 / 668,
+    # 3.5 540 / 433 and 203 / 229, 4.3 2,504 / 2,325, 5.3 458 / 569, 7.1 1,652 / 2,420;
+    # explicit points on Ewald slices at 1.8 a bin 392 / 253, 3.5 542 / 427,
+    # 6.0 1,692 / 1,687, 7.1 711 / 809, 12 2,042 / 3,379
+    SORTED_MIN_PER_BIN = 5
     _auto_sort = 0  # spf_nufft_sort_count of the last automatic sort
     _sort_lock = threading.RLock()  # keeps a sort and its pass together, for all plans
 
     def may_sort(self, n: int) -> bool:
-        """Whether an automatic choice may bin-sort n points on this plan: never
-        under graph capture, where a sort may not allocate, and a graph would
-        keep addresses that the next larger sort frees."""
+        """Whether an automatic choice may bin-sort n points on this plan: not
+        where the bins would hold too few, and never under graph capture, where
+        a sort may not allocate, and a graph would keep addresses that the next
+        larger sort frees."""
         if self.device.type == "cuda" and torch.cuda.is_current_stream_capturing():
             return False
         if n >= self.KEEP_SORT_POINTS or not self._h:
             return True
+        if n < self.SORTED_MIN_PER_BIN * math.prod(-(-v // 8) for v in self.n_padded):
+            return False
         return int(_lib.lib().spf_nufft_sort_count(self._h)) in (0, self._auto_sort)
 
     def sorted_automatically(self):

@@ -266,3 +266,26 @@ def test_slice_tuner_names_what_runs(monkeypatch, tmp_path):
     best = autotune.tune_slice(*args)
     assert not best["cached"] and best["shape"] == 0 and "spacing" in best["tile"]
     assert autotune.tune_slice(*args)["cached"]
+
+
+def test_automatic_sort_needs_points_in_the_bins(monkeypatch):
+    """NufftPlan.may_sort: at least SORTED_MIN_PER_BIN points a bin below
+    KEEP_SORT_POINTS, whatever the grid from there on."""
+    import types
+
+    import torch
+
+    from spinifel_gb300 import _lib
+    from spinifel_gb300.nufft import NufftPlan
+
+    monkeypatch.setattr(_lib, "lib", lambda: types.SimpleNamespace(
+        spf_nufft_sort_count=lambda h: 0))
+    P = object.__new__(NufftPlan)
+    P._h = types.SimpleNamespace(value=None)
+    P.device = torch.device("cpu")
+    for padded in ((64, 64, 64), (332, 330, 330), (650, 650, 652)):
+        P.n_padded = padded
+        line = 5 * -(-padded[0] // 8) * -(-padded[1] // 8) * -(-padded[2] // 8)
+        big = P.KEEP_SORT_POINTS
+        assert P.may_sort(line - 1) == (line - 1 >= big)
+        assert P.may_sort(line) and P.may_sort(big)
