@@ -263,7 +263,8 @@ int spf_slice_t2_f64(spf_nufft64_plan plan, const double *d_quats, int64_t n_ori
                      void *stream);
 /* The same on a detector of n_panels x nx x ny pixels (n_pix in that order):
  * for kernel widths up to 13 the sums run over pairs of floats, accurate to
- * about 2^-46, from footprint boxes staged in shared memory. */
+ * about 2^-46, from footprint boxes staged in shared memory (in FP64 as above on
+ * detectors of panels so thin that this is quicker). */
 int spf_slice_t2_f64_det(spf_nufft64_plan plan, const double *d_quats, int64_t n_orient,
                          const double *d_ppr, int n_panels, int nx, int ny, double scale,
                          double *d_out, void *stream);

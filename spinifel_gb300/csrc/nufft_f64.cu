@@ -727,6 +727,18 @@ int spf_slice_t2_f64(spf_nufft64_plan P, const double *d_quats, int64_t n_orient
   return slice_f64(P, d_quats, n_orient, d_ppr, n_pix, scale, d_out, nullptr, as_stream(stream));
 }
 
+// Whether slices by pairs are the quicker ones.  A patch costs the same however few
+// of its 32 pixels a panel has; the FP64 kernel's unit is 32 consecutive pixels.
+// By width, a patch over a unit: 0.78-0.95 at W = 3, 0.62 at 4, 0.41 at 7, 0.33 at
+// 10, 0.30 at 13 (in FP64 always at W = 2: 1.02-1.2).  Pairs / FP64, us: 1 x 4096 x 1
+// pixels (8 patches a unit) 2,912 / 1,354 at W = 13 and 1,973 / 797 at 10;
+// 1 x 4096 x 3 (2.7) 1,760 / 2,306 at 13, 807 / 748 at 7; 16 x 17 x 19 (1.5)
+// 569 / 1,354 at 13, 196 / 216 at 4.
+static bool pairs_pay(int w, int64_t patches, int64_t n_pix) {
+  const int64_t units = (n_pix + PAIR_PIX - 1) / PAIR_PIX;
+  return (0.12 + 2.3 / w) * (double)patches <= 0.95 * (double)units;
+}
+
 int spf_slice_t2_f64_det(spf_nufft64_plan P, const double *d_quats, int64_t n_orient,
                          const double *d_ppr, int n_panels, int nx, int ny, double scale,
                          double *d_out, void *stream) {
@@ -737,7 +749,7 @@ int spf_slice_t2_f64_det(spf_nufft64_plan P, const double *d_quats, int64_t n_or
   const int64_t patches =
       (int64_t)n_panels * ((nx + PAIR_PX - 1) / PAIR_PX) * ((ny + PAIR_PY - 1) / PAIR_PY);
   const int64_t n_pix = (int64_t)n_panels * nx * ny;
-  if (!P->pair_pad || patches > 65535)
+  if (!P->pair_pad || patches > 65535 || !pairs_pay(P->w, patches, n_pix))
     return spf_slice_t2_f64(P, d_quats, n_orient, d_ppr, n_pix, scale, d_out, stream);
   SPF_REQUIRE(d_quats && d_ppr && d_out, "spf_slice_t2_f64_det: NULL pointer");
   SPF_REQUIRE(n_orient < (1LL << 31) && n_pix <= 65535LL * 128,

@@ -311,7 +311,8 @@ class NufftPlan64:
               out_bf16=None, det_shape: tuple | None = None):
         """FP64 slices [n_orient, n_pix] (real part) at the given orientations.
         With det_shape = (n_panels, nx, ny) the sums run over pairs of floats
-        (about 2^-46) where the plan's kernel is no wider than 13."""
+        (about 2^-46) where the plan's kernel is no wider than 13 and the
+        panels are not thin ones."""
         if out_bf16 is not None:
             raise ValueError("the FP64 plan writes no bf16 copy")
         quats = self._f64(quats)

@@ -768,3 +768,25 @@ def test_fp64_distances_where_the_tile_changed(n_data, n_ref):
     xi, ri = (x * 100).round(), (r * 100).round()
     got = matching.dist_f64(ri, xi).reshape(n_data, n_ref)
     assert torch.equal(got, ((xi[:, None, :] - ri[None, :, :]) ** 2).sum(2))
+
+
+@pytest.mark.parametrize("det", [(1, 1, 700), (1, 700, 1), (2, 300, 2), (5, 1, 7)])
+@pytest.mark.parametrize("eps", [1e-6, 1e-12])
+def test_fp64_slices_of_thin_panels(det, eps):
+    """Panels a pixel or two wide: the FP64 kernel's bits where it is the quicker
+    one, and never further from them than pairs may be (6e-14 of the largest)."""
+    from spinifel_gb300 import geom
+    from spinifel_gb300.nufft import NufftPlan64
+
+    rng = np.random.default_rng(41)
+    ppr = rng.standard_normal((3,) + det)
+    q = geom.uniform_quaternions(4, rng)
+    P = NufftPlan64(21, eps)
+    P.set_modes(torch.as_tensor(rng.random((21, 21, 21)), device="cuda"))
+    p = torch.as_tensor(ppr.reshape(3, -1), device="cuda")
+    flat, got = P.slice(q, p, 0.7), P.slice(q, p, 0.7, det_shape=det)
+    patches = det[0] * -(-det[1] // 4) * -(-det[2] // 8)
+    units = -(-p.shape[1] // 32)
+    if (0.12 + 2.3 / P.width) * patches > 0.95 * units:
+        assert torch.equal(flat, got)
+    assert float((flat - got).abs().max()) <= 6e-14 * float(flat.abs().max())
