@@ -73,8 +73,8 @@ int spf_selftest_bounded_wait(int64_t timeout_ms, int *d_result, void *stream);
  *                           block, codes 1..5; 6 and 7 are 16 x 16
  *                           patches of 4 x 8 and 8 x 4 warp blocks with a
  *                           per-CTA choice of the shared box's strides
- *                           against bank conflicts; default 0 = picked by
- *                           the pixels' spacing); every shape gives the
+ *                           against bank conflicts; default 0 = picked by width,
+ *                           pixels' spacing and panels); every shape gives the
  *                           same bits
  *   SPF_TUNE_SORT_ITEM    : points per work item of the bin-sorted passes
  *                           (read by spf_nufft_sort_orient /

@@ -31,7 +31,7 @@ from . import _lib
 HERE = os.path.dirname(os.path.abspath(__file__))
 # part of every cache key; changes when a tuned kernel or the meaning of a
 # choice does, so that choices timed against other kernels are not taken
-KERNELS = 2
+KERNELS = 3
 _lock = threading.Lock()
 
 
@@ -152,8 +152,8 @@ def tune_fp32(frames_f32, frames_sq, refs, group_sizes=(4, 8, 16), reps=1, force
 
 # code 0 is no shape but the kernel's own rule; the others hold for every
 # detector and grid of the process until the code is set back
-SLICE_SHAPES = {0: "by the pixels' spacing: 8x16 patch, 4x8 warps (with stride search from "
-                   "0.5 cells), or shape 6 from 2.2 cells", 1: "16x16 patch, 8x4 warps",
+SLICE_SHAPES = {0: "by width, spacing and panels: 8x16 or 16x16 patch, 4x8 warps, "
+                   "with or without stride search", 1: "16x16 patch, 8x4 warps",
                 2: "8x32 patch, 2x16 warps", 3: "8x32 patch, 4x8 warps",
                 4: "32x8 patch, 8x4 warps", 5: "32x8 patch, 16x2 warps",
                 6: "16x16 patch, 4x8 warps, stride search",

@@ -423,7 +423,8 @@ constexpr int SLICE_SMEM_FLOATS = 11264;  // 44 KB
 // + 0..3, sk = dk + 0..3) by the number of distinct banks its warps'
 // footprint starts hit (one warp-wide OR of bank bits per candidate) and
 // keeps the best one that fits in shared memory.
-constexpr int SLICE_SHAPE_8X16 = 8;  // 128 threads, picked by default_shape
+constexpr int SLICE_SHAPE_8X16 = 8;   // 128 threads (9: with the search)
+constexpr int SLICE_SHAPE_16X16 = 10;  // as 6 without the search; 8 to 10 are default_shape's
 struct PatchShape {
   int px, py, wx, wy, search;
 };
@@ -439,6 +440,7 @@ __host__ __device__ inline PatchShape slice_shape(int code) {
     case 7: return PatchShape{16, 16, 8, 4, 1};
     case SLICE_SHAPE_8X16: return PatchShape{8, 16, 4, 8, 0};
     case SLICE_SHAPE_8X16 + 1: return PatchShape{8, 16, 4, 8, 1};
+    case SLICE_SHAPE_16X16: return PatchShape{16, 16, 4, 8, 0};
     default: return PatchShape{16, 16, 4, 8, 1};  // 6
   }
 }
@@ -1639,25 +1641,43 @@ int spf_slice_t2(spf_nufft_plan P, const float *d_quats, int64_t n_orient, const
   return check_launch("k_slice_t2");
 }
 
-// Patch shape where none was tuned, by the spacing of the pixels in grid
-// cells (n / sqrt(n_pix) for a detector that spans the grid, as the panels of
+// Patch shape where none was tuned.
+// Panels that leave half of their 8 x 16 patches' threads without a pixel, or have
+// as many 16 x 16 patches: 8 x 16 without the search (1 x 4096 x 1 pixels 154 us, 203
+// with 16 x 16; 256 panels of 4 x 4: 66 and 126).
+// Else by the kernel's width and the spacing of the pixels in grid cells
+// (n / sqrt(n_pix), for a detector that spans the grid as the panels of
 // a flat detector do).  The patch decides whether its box fits in shared
-// memory; the stride search (16 reductions a warp) pays unless the footprints
-// of a warp all but coincide.  Times in us with 16 x 16 patches, 16 x 16 with
-// the search, 8 x 16 without and with it (grid, detector, orientations):
+// memory; the stride search (16 reductions a warp) pays where the W^3 taps
+// outweigh it, unless the footprints of a warp all but coincide.  Times in us
+// with 16 x 16 patches, 16 x 16 with the search, 8 x 16 without and with it, W = 7
+// (grid, detector, orientations):
 //   0.35 cells  90^3,  4 x 128 x 128,  100:   384   420   377   417
 //   0.63 cells 162^3,  4 x 128 x 128,  500:  2474  2061  2119  2001
 //   1.25 cells 320^3,  4 x 128 x 128,  200:  1622  1474  1469  1312
 //   1.41 cells  90^3,  4 x 32 x 32,   2000:  1308  1187   989   893
 //   1.72 cells 128^3,  3 x 50 x 37,    500:   362   315   313   284
 //   2.53 cells 162^3,  4 x 32 x 32,   1000:  1639  1629  3793  1779
-// (A detector with more 8 x 16 patches than a launch takes keeps 16 x 16.)
+// and over the best of the four, at other widths (points out to the grid's edge):
+//   W = 3  0.63 cells 1.00 1.16 1.01 1.16   1.25 1.00 1.11 1.26 1.32   2.53 1.00 1.15 2.01 2.07
+//   W = 4  0.63 cells 1.05 1.14 1.00 1.12   1.25 1.01 1.00 1.11 1.09   2.53 1.08 1.00 2.14 2.01
+//   W = 5  0.63 cells 1.11 1.14 1.00 1.04   1.25 1.51 1.29 1.56 1.00   2.53 1.17 1.00 2.41 1.12
+//   W = 6  0.63 cells 1.30 1.11 1.09 1.00   1.25 1.36 1.32 1.10 1.00   2.53 1.04 1.00 1.17 1.12
+// (A detector with more 8 x 16 patches than a launch takes has 16 x 16.)
 static int default_shape(const spf_nufft_plan_s *P, int n_panels, int nx, int ny) {
   const int64_t n_pix = (int64_t)n_panels * nx * ny;
-  if ((int64_t)n_panels * ((nx + 7) / 8) * ((ny + 15) / 16) > 65535) return 6;
+  const int64_t patches8 = (int64_t)n_panels * ((nx + 7) / 8) * ((ny + 15) / 16);
+  const int64_t patches16 = (int64_t)n_panels * ((nx + 15) / 16) * ((ny + 15) / 16);
   const int n = std::max(P->n[0], std::max(P->n[1], P->n[2]));
   const double cells = n / sqrt((double)n_pix);
-  return cells < 0.5 ? SLICE_SHAPE_8X16 : cells < 2.2 ? SLICE_SHAPE_8X16 + 1 : 6;
+  const int wide = cells >= 2.2 ? 6 : SLICE_SHAPE_16X16;  // 16 x 16
+  if (P->w <= 3 && patches8 > patches16 && 2 * n_pix >= patches8 * 128) return SLICE_SHAPE_16X16;
+  if (patches8 > 65535) return P->w <= 3 ? SLICE_SHAPE_16X16 : wide;
+  if (patches8 == patches16 || 2 * n_pix < patches8 * 128) return SLICE_SHAPE_8X16;
+  if (P->w == 4) return cells < 1.0 ? SLICE_SHAPE_8X16 : wide;
+  return cells < (P->w == 5 ? 1.0 : 0.5) ? SLICE_SHAPE_8X16
+         : cells < 2.2                   ? SLICE_SHAPE_8X16 + 1
+                                         : 6;
 }
 
 int spf_slice_t2_det(spf_nufft_plan P, const float *d_quats, int64_t n_orient, const float *d_ppr,

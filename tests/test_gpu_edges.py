@@ -790,3 +790,21 @@ def test_fp64_slices_of_thin_panels(det, eps):
     if (0.12 + 2.3 / P.width) * patches > 0.95 * units:
         assert torch.equal(flat, got)
     assert float((flat - got).abs().max()) <= 6e-14 * float(flat.abs().max())
+
+
+@pytest.mark.parametrize("eps", [1e-1, 1e-2, 1e-3, 1e-4, 1e-5, 1e-6, 1e-7])
+def test_slices_by_every_rule_of_the_patch_shape(eps):
+    """Detectors and grids on every side of the shape's rule: the bits of the
+    thread-per-point kernel, at every width."""
+    from spinifel_gb300 import geom
+    from spinifel_gb300.nufft import NufftPlan
+
+    rng = np.random.default_rng(43)
+    for M in (9, 41, 81):
+        P = NufftPlan(M, eps)
+        P.set_modes(torch.as_tensor(rng.random((M, M, M)), device="cuda"))
+        for det in ((1, 1, 300), (1, 300, 1), (7, 8, 16), (3, 9, 17), (2, 24, 40), (1, 64, 64),
+                    (1, 200, 200), (3, 2, 5), (1, 1, 1)):
+            ppr = torch.as_tensor(rng.standard_normal((3, int(np.prod(det)))), device="cuda")
+            q = torch.as_tensor(geom.uniform_quaternions(3, rng), device="cuda")
+            assert torch.equal(P.slice(q, ppr, 0.5, det_shape=det), P.slice(q, ppr, 0.5))
