@@ -84,7 +84,7 @@ int spf_selftest_bounded_wait(int64_t timeout_ms, int *d_result, void *stream);
  *                           given-up GEMM wait (SPF_ERR_TIMEOUT in its
  *                           error word, after the GEMM), the other bf16
  *                           GEMMs give up at each CTA's last tile, and the
- *                           re-rank of up to 13 frames an SM treat every odd
+ *                           re-rank of up to 10 frames an SM treat every odd
  *                           frame as one whose copies gave no sign, so that tests can
  *                           check the void answers, their completion and the
  *                           report through spf_device_error without a device

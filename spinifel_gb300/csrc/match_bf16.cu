@@ -939,21 +939,26 @@ __global__ void __launch_bounds__(RX_THREADS)
 }
 
 // The same distances, bit for bit, with one CTA per frame, for calls of up to
-// RF_RESIDENT frames an SM: warp 1 streams the frame's row and the rows of
+// RF_RESIDENT_VEC (or RF_RESIDENT) frames an SM: warp 1 streams the frame's row and the rows of
 // the candidates in the band through a ring (one bulk copy a row and chunk;
 // 4-byte asynchronous copies where rows are not 16-byte aligned), warp 0 runs
 // the chains, lane c that of candidate c.  A chain of n_pix dependent FMAs
 // cannot be shortened, so with few frames its latency is the time (131 us for
 // 65,536 pixels at four clocks an FMA); here the loads, the copies and the
 // barriers run beside it: 5 frames of 65,536 pixels take 175 us against
-// 496 us in k_rerank_exact.  Beyond one wave of CTAs k_rerank_exact is faster:
+// 496 us in k_rerank_exact.  With many frames k_rerank_exact is faster:
 // its CTAs are all resident, walk the rows in step and share them in L2
-// (957 us against 1,600 us for 4,096 frames, 50,000 references).
+// (957 us against 1,600 us for 4,096 frames, 50,000 references).  The line, us
+// for GEMM, merge and re-rank by this kernel and by that (references, pixels):
+// 1,300 frames 725 / 780 (1,000, 65,536), 185 / 194 (3,000, 8,192), 1,600 frames
+// 859 / 811, 213 / 207, 1,900 frames 1,075 / 869, 244 / 217.  Rows that are not
+// 16-byte aligned, which that kernel loads word by word: 1,900 frames 165 / 203
+// (3,000, 4,095), so there it stays for as many CTAs as are resident.
 constexpr int RF_THREADS = 64;
 constexpr int RF_MAX_STAGES = 16;
 constexpr int RF_RING_FEW = 11776;  // floats: five 256-pixel stages of all nine rows, 4 CTAs an SM
 constexpr int RF_RING_MANY = 4096;  // 13 CTAs an SM
-constexpr int RF_RESIDENT_FEW = 4, RF_RESIDENT = 13;
+constexpr int RF_RESIDENT_FEW = 4, RF_RESIDENT_VEC = 10, RF_RESIDENT = 13;
 
 template <int C>
 __device__ __forceinline__ bool rerank_chain(const float *ring, int slot, int nr, int stages,
@@ -1265,7 +1270,8 @@ static int launch_rerank(const float *cand_d, const int32_t *cand_i, const float
                          const float *ref_sq, int64_t n_ref, float ref_sq_max, int64_t n_pix,
                          int64_t ref_offset, float *work, int32_t *idx, float *dist,
                          int32_t *uncertified, int32_t *top8, unsigned int *err, cudaStream_t s) {
-  if (n_img <= (int64_t)RF_RESIDENT * sm_count()) {
+  const bool vec = n_pix % 4 == 0 && aligned(img, 16) && aligned(ref, 16);
+  if (n_img <= (int64_t)(vec ? RF_RESIDENT_VEC : RF_RESIDENT) * sm_count()) {
     const int ring = n_img <= (int64_t)RF_RESIDENT_FEW * sm_count() ? RF_RING_FEW : RF_RING_MANY;
     k_rerank_frame<<<(unsigned)n_img, RF_THREADS, ring * sizeof(float), s>>>(
         cand_d, cand_i, img, img_sq, n_img, ref, ref_sq, n_ref, ref_sq_max, n_pix, ref_offset,

@@ -808,3 +808,19 @@ def test_slices_by_every_rule_of_the_patch_shape(eps):
             ppr = torch.as_tensor(rng.standard_normal((3, int(np.prod(det)))), device="cuda")
             q = torch.as_tensor(geom.uniform_quaternions(3, rng), device="cuda")
             assert torch.equal(P.slice(q, ppr, 0.5, det_shape=det), P.slice(q, ppr, 0.5))
+
+
+@pytest.mark.parametrize("n_pix", [64, 65])
+@pytest.mark.parametrize("per_sm", [4, 10, 13])
+def test_rerank_at_the_lines_between_kernels(per_sm, n_pix):
+    """One frame fewer, as many and one more than the frames an SM at which
+    the re-rank changes kernels: the plain path's answer."""
+    from spinifel_gb300 import matching
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    fr, rs = _match_operands(per_sm * sms + 1, 300, n_pix, 50 + per_sm)
+    want_i, want_d = matching.argmin_fp32(fr.f32, rs.f32, images_sq=fr.sq, refs_sq=rs.sq)
+    for n in (per_sm * sms - 1, per_sm * sms, per_sm * sms + 1):
+        part = matching.FrameSet(fr.f32[:n], bf16=fr.bf16[:n], sq=fr.sq[:n], n4=fr.n4[:n])
+        idx, dist = matching.match_bf16(part, rs)
+        assert torch.equal(idx.to(want_i.dtype), want_i[:n]) and torch.equal(dist, want_d[:n])
