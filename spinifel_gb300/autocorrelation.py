@@ -33,10 +33,13 @@ def plan_for(M, eps=DEFAULT_EPS) -> NufftPlan:
     return p
 
 
-def _dtype(eps) -> torch.dtype:
-    """Device type of the plan for eps: converting to it at once gives what
-    converting through FP64 gives."""
-    return torch.float32 if float(eps) >= FP32_EPS_FLOOR else torch.float64
+def _dtype(eps, *arrs) -> torch.dtype:
+    """Device type to bring arrs to for a plan of eps: its own where they are on the
+    device (converting to it at once gives what converting through FP64 gives),
+    FP64 where they are not (the host converts slower than the copy and the device
+    take: 67 / 55 us for 70,000 values, 195 / 152 for 2.1e6)."""
+    on_device = all(_arrays.is_torch(a) and a.is_cuda for a in arrs)
+    return torch.float32 if on_device and float(eps) >= FP32_EPS_FLOOR else torch.float64
 
 
 def _numel(a) -> int:
@@ -70,11 +73,11 @@ def forward(ugrid, H_, K_, L_, support, use_recip_sym, N, eps=DEFAULT_EPS):
             assert np.all(np.isreal(ugrid))
     g = _arrays.to_dev(ugrid.real if _arrays.is_torch(ugrid) and torch.is_complex(ugrid)
                        else (np.real(ugrid) if not _arrays.is_torch(ugrid) else ugrid),
-                       _dtype(eps))
+                       _dtype(eps, ugrid))
     P = plan_for(g.shape, eps)
     P.set_modes(g, support, isign=-1, want_imag=True)
     x, y, z = (_arrays.to_dev(np.asarray(a).reshape(-1) if not _arrays.is_torch(a) else a,
-                              P.dtype) for a in (H_, K_, L_))
+                              _dtype(eps, a)) for a in (H_, K_, L_))
     re, im = P.interp(x, y, z, want_imag=True)
     out = torch.complex(re, im)
     assert out.numel() == N

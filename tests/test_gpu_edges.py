@@ -824,3 +824,24 @@ def test_rerank_at_the_lines_between_kernels(per_sm, n_pix):
         part = matching.FrameSet(fr.f32[:n], bf16=fr.bf16[:n], sq=fr.sq[:n], n4=fr.n4[:n])
         idx, dist = matching.match_bf16(part, rs)
         assert torch.equal(idx.to(want_i.dtype), want_i[:n]) and torch.equal(dist, want_d[:n])
+
+
+@pytest.mark.parametrize("eps", [1e-6, 1e-12])
+def test_forward_takes_every_kind_of_array(eps):
+    """numpy, host and device tensors of both types: the same values bit for bit where
+    the inputs are, single precision's where they are single."""
+    from spinifel_gb300 import autocorrelation as ac
+
+    rng = np.random.default_rng(61)
+    M, n = 15, 700
+    model = rng.random((M, M, M)).astype(np.float32)
+    pts = [rng.uniform(-3, 3, n).astype(np.float32) for _ in range(3)]
+    want = ac.forward(model, *pts, 1.0, True, n, eps=eps)
+    assert isinstance(want, np.ndarray)
+    for dt in (np.float32, np.float64):  # the same values in both types
+        a = [v.astype(dt) for v in (model, *pts)]
+        for dev in (None, "cpu", "cuda"):
+            b = a if dev is None else [torch.as_tensor(v, device=dev) for v in a]
+            got = ac.forward(*b, 1.0, True, n, eps=eps)
+            got = got if dev is None else got.cpu().numpy()
+            np.testing.assert_array_equal(got, want)
