@@ -45,12 +45,13 @@ __device__ __forceinline__ int wrap(int i, int n) {
   return i < 0 ? i + n : i;
 }
 
-// grid[k mod n] = f_k * support_k / (p1 p2 p3), zero elsewhere
+// grid[k mod n] = f_k * support_k / (p1 p2 p3), zero elsewhere; and *peak = 0
 template <class T>
 __global__ void k_modes_to_grid(const T *__restrict__ f, const T *__restrict__ sup, int m1, int m2,
                                 int m3, GridDims g, const T *__restrict__ ip1,
                                 const T *__restrict__ ip2, const T *__restrict__ ip3,
-                                T *__restrict__ grid) {
+                                T *__restrict__ grid, unsigned long long *__restrict__ peak) {
+  if (peak && blockIdx.x == 0 && threadIdx.x == 0 && threadIdx.y == 0) *peak = 0;
   const int64_t row = (int64_t)blockIdx.x * ROWS_PER_CTA + threadIdx.y;
   if (row >= (int64_t)g.n1 * g.n2) return;
   const int fa = (int)(row / g.n2), fb = (int)(row % g.n2);
@@ -75,14 +76,17 @@ __global__ void k_modes_to_grid(const T *__restrict__ f, const T *__restrict__ s
 }
 
 // re[i] = Re F[(i - off) mod n] for every padded cell, and where asked for
-// im = im_sign Im F or the pairs (re, im)
+// im = im_sign Im F or the pairs (re, im); for doubles, in *peak the bits of
+// max |re| (NaN above infinity above all values)
 template <class T>
 __global__ void k_spectrum_to_padded(const typename Complex<T>::type *__restrict__ half,
                                      GridDims g, T im_sign, T *__restrict__ re,
                                      T *__restrict__ im,
-                                     typename Complex<T>::type *__restrict__ cx) {
+                                     typename Complex<T>::type *__restrict__ cx,
+                                     unsigned long long *__restrict__ peak) {
   const int64_t row = (int64_t)blockIdx.x * ROWS_PER_CTA + threadIdx.y;
   if (row >= (int64_t)g.p1 * g.p2) return;
+  unsigned long long top = 0;
   const int nh = g.n3 / 2 + 1;
   const int a = wrap((int)(row / g.p2) - g.off1, g.n1), b = wrap((int)(row % g.p2) - g.off2, g.n2);
   const auto *h = half + ((int64_t)a * g.n2 + b) * nh;
@@ -95,6 +99,10 @@ __global__ void k_spectrum_to_padded(const typename Complex<T>::type *__restrict
     const bool direct = c < nh;
     const auto v = direct ? h[c] : hm[g.n3 - c];
     re[row * g.p3 + k] = v.x;
+    if constexpr (sizeof(T) == 8) {
+      const unsigned long long b = (unsigned long long)__double_as_longlong(v.x) & ~(1ULL << 63);
+      top = b > top ? b : top;
+    }
     const T y = direct ? im_sign * v.y : -im_sign * v.y;
     if (im) im[row * g.p3 + k] = y;
     if (cx) {
@@ -103,6 +111,16 @@ __global__ void k_spectrum_to_padded(const typename Complex<T>::type *__restrict
       q.y = y;
       cx[row * g.p3 + k] = q;
     }
+  }
+  if constexpr (sizeof(T) == 8) {
+    if (!peak) return;
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+      const unsigned long long u = __shfl_xor_sync(0xffffffffu, top, o);
+      top = u > top ? u : top;
+    }
+    // most rows are below what others have put there
+    if (threadIdx.x == 0 && top > *(volatile unsigned long long *)peak) atomicMax(peak, top);
   }
 }
 

@@ -1592,12 +1592,12 @@ int spf_nufft_t2_set_modes(spf_nufft_plan P, const float *d_modes, const float *
   const GridDims g = grid_dims(P);
   k_modes_to_grid<float><<<row_grid((int64_t)g.n1 * g.n2), row_block(), 0, s>>>(
       d_modes, d_support, P->m[0], P->m[1], P->m[2], g, P->inv_p[0], P->inv_p[1], P->inv_p[2],
-      P->fine);
+      P->fine, nullptr);
   SPF_TRY(check_launch("k_modes_to_grid"));
   SPF_TRY(fft_exec(P, s, "spf_nufft_t2_set_modes"));
   k_spectrum_to_padded<float><<<row_grid((int64_t)g.p1 * g.p2), row_block(), 0, s>>>(
       P->half, g, isign < 0 ? float(1) : float(-1), P->re_pad, nullptr,
-      P->cx_pad);
+      P->cx_pad, nullptr);
   return check_launch("k_spectrum_to_padded");
 }
 

@@ -276,24 +276,6 @@ __device__ __forceinline__ Pair es_pair(Pair f, int a, const PairKernel &k,
   return fast_two_sum(w.h, __fadd_rn(w.l, __fadd_rn(T.y, Tu.l)));
 }
 
-// bits of max |v| (NaN above infinity above all values)
-__global__ void __launch_bounds__(256)
-    k_peak(const double *__restrict__ v, int64_t n, unsigned long long *__restrict__ peak) {
-  unsigned long long m = 0;
-#pragma unroll 4
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v[i]) & ~(1ULL << 63);
-    m = b > m ? b : m;
-  }
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) {
-    const unsigned long long u = __shfl_xor_sync(0xffffffffu, m, o);
-    m = u > m ? u : m;
-  }
-  if ((threadIdx.x & 31) == 0) atomicMax(peak, m);
-}
-
 __global__ void k_to_pairs(const double *__restrict__ v, int64_t n,
                            const unsigned long long *__restrict__ peak,
                            float2 *__restrict__ out) {
@@ -547,9 +529,15 @@ static Pair pair_of(double v) {
 static int alloc_pairs(spf_nufft64_plan P) {
   const size_t npad = (size_t)P->np[0] * P->np[1] * P->np[2];
   const int n = (int)ceil(EXP_PER_UNIT * P->beta) + 2;
+  // exp(-j / 128) as a product of two (to 2^-52): an exponential for each of the
+  // 3,900 takes the host longer than the allocation
+  constexpr int step = 64;
+  double part[step], whole = 1.0;
+  for (int j = 0; j < step; ++j) part[j] = exp(-(double)j / EXP_PER_UNIT);
   std::vector<float2> t(n);
   for (int j = 0; j < n; ++j) {
-    const Pair p = pair_of(exp(-(double)j / EXP_PER_UNIT));
+    if (j % step == 0) whole = exp(-(double)j / EXP_PER_UNIT);
+    const Pair p = pair_of(whole * part[j % step]);
     t[j] = make_float2(p.h, p.l);
   }
   if (cudaMalloc(&P->pair_pad, (npad + n + 1) * sizeof(float2)) != cudaSuccess) {
@@ -657,9 +645,6 @@ int spf_nufft64_plan_info(spf_nufft64_plan P, int *n_fine, int *width, double *b
 // captured slicing reads the model set last)
 static int make_pairs(spf_nufft64_plan P, cudaStream_t s) {
   const int64_t npad = (int64_t)P->np[0] * P->np[1] * P->np[2];
-  SPF_TRY(check_cuda(cudaMemsetAsync(P->peak, 0, sizeof(*P->peak), s), "spf_nufft64_t2_set_modes"));
-  k_peak<<<grid_for(npad, 1024, (int64_t)sm_count() * 8), 256, 0, s>>>(P->re_pad, npad, P->peak);
-  SPF_TRY(check_launch("k_peak"));
   k_to_pairs<<<grid_for(npad, 256, (int64_t)sm_count() * 16), 256, 0, s>>>(P->re_pad, npad, P->peak,
                                                                           P->pair_pad);
   return check_launch("k_to_pairs");
@@ -677,12 +662,12 @@ int spf_nufft64_t2_set_modes(spf_nufft64_plan P, const double *d_modes, const do
   const GridDims g = grid_dims(P);
   k_modes_to_grid<double><<<row_grid((int64_t)g.n1 * g.n2), row_block(), 0, s>>>(
       d_modes, d_support, P->m[0], P->m[1], P->m[2], g, P->inv_p[0], P->inv_p[1], P->inv_p[2],
-      P->fine);
+      P->fine, P->peak);
   SPF_TRY(check_launch("k_modes_to_grid"));
   SPF_TRY(fft_exec(P, s, "spf_nufft64_t2_set_modes"));
   k_spectrum_to_padded<double><<<row_grid((int64_t)g.p1 * g.p2), row_block(), 0, s>>>(
       P->half, g, isign < 0 ? double(1) : double(-1), P->re_pad,
-      want_imag ? P->im_pad : nullptr, nullptr);
+      want_imag ? P->im_pad : nullptr, nullptr, P->peak);
   SPF_TRY(check_launch("k_spectrum_to_padded"));
   return P->pair_pad ? make_pairs(P, s) : SPF_OK;
 }
